@@ -595,8 +595,8 @@ def run_b200(args, rank, world, local):
         achieved = N * alg / (kms / kn / 1e3) / 1e9
         achieved_read = N * read / (kms / kn / 1e3) / 1e9
         peak, src = peaks()
-        kname = ("mech_kernel<finest, PCG, Gauss-point moduli, " +
-                 ("rows staged by TMA tensor copies" if TMA_STAGING else "rows staged by per-lane cp.async") +
+        kname = ("mech_tile_kernel<Gauss-point moduli, PCG, " +
+                 ("planes staged by TMA tensor copies" if TMA_STAGING else "planes staged by per-thread cp.async") +
                  "> (w = K(d) p, (p, w))")
         basis = "algorithmic: u 24 + bulK,G,d 24 + regime 2 + out 24 B per finest node"
         roofline = {"bound": "hbm", "kernel": kname,

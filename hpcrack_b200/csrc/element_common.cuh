@@ -1,0 +1,121 @@
+// Shared by the element-operator kernels (element_kernels.cu, mech_tile.cu): launch arguments, the
+// epilogue of one finished node, launch set-up.
+#pragma once
+
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include "device_common.cuh"
+#include "internal.h"
+
+namespace hpc {
+
+struct StripGeo {
+  int tx, ty, tz;            // strips per axis
+  int wy, cz;                // element rows (2..kWY) and output planes per strip
+  long long nstrips;
+};
+
+
+template <typename T>
+struct MechKT {
+  LevelGeo g;
+  LevelGeo gf;  // fine level (FAS)
+  StripGeo sg;
+  const T* fields[6];  // staged: u0,u1,u2 then K,G,d (finest) or Ke,Ge (coarse)
+  T* out;
+  const int8_t* choice;
+  double small_k;
+  T* fu;
+  int set_fnorm;
+  const T* invM;
+  const T* rf;
+  const T* gpm;  // finest level, precomputed Gauss-point moduli: K - 2G/3 at [g * n + e], G at [(8 + g) * n + e]
+  RedTarget red;
+  double* err;   // tensor-core kernel / TMA staging: set to 1 when a bounded wait ran out
+  alignas(64) CUtensorMap tmap;  // TMA staging: the staged vector as {px, ny, nz, 3}
+  alignas(64) CUtensorMap gmap;  // TMA staging: the Gauss-point moduli as {px, ny, nz, 16} (finest applies)
+};
+using MechK = MechKT<double>;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// What a kernel does with the finished operator row tot of node (x, ey, kk), by epilogue; own_p is the
+// applied vector at the node (EPI_PCG); pre_f and pre_m are f and (where k.invM is set) M^-1 at the node
+// (EPI_RESIDUAL).
+template <typename T, int EPI>
+__device__ __forceinline__ void node_epilogue(const MechKT<T>& k, int x, int ey, int kk, const T (&tot)[3],
+                                              const T (&own_p)[3], const T (&pre_f)[3], const T (&pre_m)[3],
+                                              double& red0, double& red1, double& red2) {
+  const long long n = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
+  const long long N = k.g.n;
+  if (EPI == EPI_PLAIN) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) k.out[n + m * N] = tot[m];
+  } else if (EPI == EPI_RESIDUAL) {
+    const BcFlags bc = bc_flags(k.g, x, ey, kk);
+    const bool fix[3] = {bc.c0, bc.c1, bc.c2};
+    // a slab's ghost planes keep the sums as they are (a select: ghost values may be anything)
+    const bool own = owned_plane(k.g, kk);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      T fv = pre_f[m];
+      if (k.set_fnorm && fix[m]) {
+        fv = tot[m];
+        k.fu[n + m * N] = fv;
+      }
+      if (k.red.slot[0] >= 0) {  // sums nobody reads are skipped
+        const double s0 = fma((double)fv, (double)fv, red0);
+        red0 = own ? s0 : red0;
+      }
+      const T rv = fix[m] ? T(0) : fv - tot[m];
+      k.out[n + m * N] = rv;
+      if (k.invM) {
+        const double s1 = fma((double)rv, (double)(rv * pre_m[m]), red1);
+        red1 = own ? s1 : red1;
+      }
+      if (k.red.slot[2] >= 0) {
+        const double s2 = fma((double)rv, (double)rv, red2);
+        red2 = own ? s2 : red2;
+      }
+    }
+  } else if (EPI == EPI_PCG) {  // w = K p, (p, w)
+    const bool own = owned_plane(k.g, kk);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      k.out[n + m * N] = tot[m];
+      const double s0 = fma((double)own_p[m], (double)tot[m], red0);
+      red0 = own ? s0 : red0;
+    }
+  } else if (EPI == EPI_FAS) {
+    // coarsen_f_standard_routine (multigrid_intergrid.cpp:124-342) fused with the coarse apply;
+    // a slab's lower ghost plane has no fine plane below it (its value comes from the neighbour)
+    const int fz = 2 * kk + k.g.zsh;
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+      k.out[n + m * N] =
+          tot[m] + (fz >= 0 ? full_weight(k.gf, k.rf + (long long)m * k.gf.n, 2 * x, 2 * ey, fz) : T(0));
+  } else if (EPI == EPI_REACTION) {
+    // Dirichlet_force_u (boundary_conditions.cpp:69-111)
+    const BcFlags bc = bc_flags(k.g, x, ey, kk);
+    if (bc.c0) k.out[n] = tot[0];
+    if (bc.c1) k.out[n + N] = tot[1];
+    if (bc.c2) k.out[n + 2 * N] = tot[2];
+  }
+}
+
+// Opt-in of a kernel's dynamic shared memory (max_smem) and its resident blocks per SM at `smem` bytes and
+// `threads` threads, looked up on first use so that later launches - also those inside a stream
+// capture - only enqueue work.
+int kernel_cfg(const void* kern, size_t max_smem, size_t smem, int threads, int* per_sm);
+int num_sms();
+// A level's vector (components n apart) or moduli array (ncomp planes n apart) as a TMA tensor
+// {px, ny, nz, ncomp}, x fastest, with the given box.
+template <typename T>
+int encode_tensor(const LevelGeo& g, const T* src, int ncomp, int bx, int by, int bz, CUtensorMap* map);
+// Tile kernels (mech_tile.cu): the mechanical operator with precomputed Gauss-point moduli (finest level,
+// k.gpm set) or element-constant moduli (coarse levels).
+template <typename T>
+int launch_mech_tile(hpc_ctx* c, MechKT<T>& k, bool finest, int epi);
+
+}  // namespace hpc

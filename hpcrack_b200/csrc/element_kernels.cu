@@ -22,6 +22,7 @@
 #include <mutex>
 
 #include "device_common.cuh"
+#include "element_common.cuh"
 #include "internal.h"
 
 namespace hpc {
@@ -33,12 +34,6 @@ constexpr int kWY = 8;
 constexpr int kOX = 30;      // output nodes per strip in x (lanes 1..30)
 constexpr int kRowW = 33;    // staged row width (32 lanes + the x+1 read of lane 31)
 constexpr int kRing = 4;     // staged node rows in flight / in use per warp
-
-struct StripGeo {
-  int tx, ty, tz;            // strips per axis
-  int wy, cz;                // element rows (2..kWY) and output planes per strip
-  long long nstrips;
-};
 
 inline StripGeo strip_geo(const LevelGeo& g, int wy, int cz, int ox = kOX) {
   StripGeo s;
@@ -122,10 +117,9 @@ struct Stream {
     cp_async_commit();
   }
   // Row s has landed for every lane of the warp (this lane's copies, then the warp barrier).
-  __device__ __forceinline__ bool wait(int) const {
+  __device__ __forceinline__ void wait() const {
     cp_async_wait2();
     __syncwarp();
-    return true;
   }
   __device__ __forceinline__ T at(int s, int f, int c, int col) const {
     return ring[(((s & (kRing - 1)) * NF + f) * 2 + c) * kRowW + col];
@@ -133,110 +127,8 @@ struct Stream {
 };
 
 // ------------------------------------------------------------------------------------------
-// TMA staging (cp.async.bulk.tensor): one elected lane per warp copies a whole staged row - the 3
-// vector components on the two planes kk, kk+1, x from xs to xs + BX - 1 - with one tensor copy into
-// the warp's ring slot, completion counted on the slot's mbarrier; every lane waits on the barrier's
-// phase.  The copy's x start must be a multiple of 16 bytes, so it starts at xs = the strip's first
-// column (x0 - 1) rounded down to 16 bytes, the box is BX wide (33 columns plus that offset, rounded
-// up to 16 bytes) and the lanes index from the offset.  Out-of-range coordinates (x < 0, x >= px,
-// y = -1 or ny, z = -1 or nz) read zeros, as the cp.async staging's zero fill does; columns nx .. px-1
-// are padding slots, zero in every vector.  Loads only, no multicast, this GPU's own memory.
-// ------------------------------------------------------------------------------------------
-template <typename T> struct TmaShape;
-template <> struct TmaShape<float> { static constexpr int BX = 36; };   // 144 B; offset <= 3
-template <> struct TmaShape<double> { static constexpr int BX = 34; };  // 272 B; offset <= 1
-template <typename T>
-constexpr int tma_slot_bytes() { return ((3 * 2 * TmaShape<T>::BX * (int)sizeof(T)) + 127) / 128 * 128; }
-constexpr int kTmaHead = 128;              // per warp: 4 mbarriers, padded to the slots' 128-B alignment
-constexpr unsigned kTmaWaitPolls = 1u << 24;  // far above any copy's latency; then the kernel reports
-template <typename T>
-__host__ __device__ constexpr size_t tma_warp_bytes(int wy) {
-  return (size_t)kTmaHead + (size_t)kRing * tma_slot_bytes<T>() + (size_t)(wy - 1) * 3 * 32 * sizeof(T);
-}
-
-// The copy's inner extent is a multiple of 16 bytes and covers 33 columns after any offset below 16
-// bytes; ring slots and every warp's share of shared memory stay on 128-byte boundaries.
-static_assert(TmaShape<float>::BX * 4 % 16 == 0 && TmaShape<float>::BX >= 33 + 3, "float box");
-static_assert(TmaShape<double>::BX * 8 % 16 == 0 && TmaShape<double>::BX >= 33 + 1, "double box");
-static_assert(tma_warp_bytes<float>(2) % 128 == 0 && tma_warp_bytes<float>(4) % 128 == 0 &&
-                  tma_warp_bytes<float>(8) % 128 == 0, "float warp share");
-static_assert(tma_warp_bytes<double>(2) % 128 == 0 && tma_warp_bytes<double>(4) % 128 == 0 &&
-                  tma_warp_bytes<double>(8) % 128 == 0, "double warp share");
-static_assert(kWY == 8, "the warp-share alignment above is checked for strip heights 2, 4 and 8");
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-template <typename T>
-struct TmaStream {
-  static constexpr int BX = TmaShape<T>::BX;
-  static constexpr int SLOT = tma_slot_bytes<T>() / (int)sizeof(T);  // elements per ring slot
-  T* ring;
-  uint64_t* bars;
-  const CUtensorMap* map;
-  int xs, off, y0, z0, nlayers, total, rows;
-  unsigned base;  // rows this warp staged before the strip: the slot and phase of row s are base + s's
-  double* err;
-
-  __device__ __forceinline__ void issue(int s, int lane) const {
-    if (lane != 0 || s >= total) return;
-    const int li = s / rows, r = s - li * rows;
-    const int kk = z0 - 1 + li, y = y0 - 1 + r;
-    const unsigned g = base + (unsigned)s;
-    const uint32_t bar = smem_u32(bars + (g & (kRing - 1)));
-    const uint32_t dst = smem_u32(ring + (size_t)(g & (kRing - 1)) * SLOT);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(3 * 2 * BX * (int)sizeof(T))
-                 : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-        "%5}], [%6];" ::"r"(dst),
-        "l"(map), "r"(xs), "r"(y), "r"(kk), "r"(0), "r"(bar)
-        : "memory");
-  }
-  // Waits for row s; a wait that runs out sets *err and returns false (the kernel then stops).
-  __device__ __forceinline__ bool wait(int s) const {
-    const unsigned g = base + (unsigned)s;
-    const uint32_t bar = smem_u32(bars + (g & (kRing - 1)));
-    const uint32_t parity = (g / kRing) & 1u;
-    for (unsigned i = 0; i < kTmaWaitPolls; ++i) {
-      uint32_t ok;
-      asm volatile(
-          "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}\n"
-          : "=r"(ok)
-          : "r"(bar), "r"(parity)
-          : "memory");
-      if (ok) return true;
-    }
-    if (err) *err = 1.0;
-    return false;
-  }
-  __device__ __forceinline__ T at(int s, int f, int c, int col) const {
-    return ring[(size_t)((base + (unsigned)s) & (kRing - 1)) * SLOT + (f * 2 + c) * BX + off + col];
-  }
-};
-
-// ------------------------------------------------------------------------------------------
 // mechanical
 // ------------------------------------------------------------------------------------------
-template <typename T>
-struct MechKT {
-  LevelGeo g;
-  LevelGeo gf;  // fine level (FAS)
-  StripGeo sg;
-  const T* fields[6];  // staged: u0,u1,u2 then K,G,d (finest) or Ke,Ge (coarse)
-  T* out;
-  const int8_t* choice;
-  double small_k;
-  T* fu;
-  int set_fnorm;
-  const T* invM;
-  const T* rf;
-  const T* gpm;  // finest level, precomputed Gauss-point moduli: K - 2G/3 at [g * n + e], G at [(8 + g) * n + e]
-  RedTarget red;
-  double* err;   // tensor-core kernel / TMA staging: set to 1 when a bounded wait ran out
-  alignas(64) CUtensorMap tmap;  // TMA staging: the staged vector as {px, ny, nz, 3} (finest applies)
-};
-using MechK = MechKT<double>;
 
 // d clamped to [0, 1] (K_G_d_g, material_gauss_point.cpp:51-54), decided on the bit pattern:
 // negative values (sign bit set) give 0, values above 1 give 1.
@@ -306,61 +198,21 @@ __device__ __forceinline__ void assemble_row(const MechKT<T>& k, const ST& st, i
       *zp = yp[1][m] + X[0][1][m];
     }
     if (kk >= z0 && lane >= 1 && lane <= 30 && x < k.g.nx && ey < k.g.ny) {
-      const long long n = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
-      const long long N = k.g.n;
-      if (EPI == EPI_PLAIN) {
+      T own_p[3] = {T(0), T(0), T(0)};
+      if (EPI == EPI_PCG) {
 #pragma unroll
-        for (int m = 0; m < 3; ++m) k.out[n + m * N] = tot[m];
-      } else if (EPI == EPI_RESIDUAL) {
-        const BcFlags bc = bc_flags(k.g, x, ey, kk);
-        const bool fix[3] = {bc.c0, bc.c1, bc.c2};
-        // a slab's ghost planes keep the sums as they are (a select: ghost values may be anything)
-        const bool own = owned_plane(k.g, kk);
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          T fv = k.fu[n + m * N];
-          if (k.set_fnorm && fix[m]) {
-            fv = tot[m];
-            k.fu[n + m * N] = fv;
-          }
-          if (k.red.slot[0] >= 0) {  // sums nobody reads are skipped
-            const double s0 = fma((double)fv, (double)fv, red0);
-            red0 = own ? s0 : red0;
-          }
-          const T rv = fix[m] ? T(0) : fv - tot[m];
-          k.out[n + m * N] = rv;
-          if (k.invM) {
-            const double s1 = fma((double)rv, (double)(rv * k.invM[n + m * N]), red1);
-            red1 = own ? s1 : red1;
-          }
-          if (k.red.slot[2] >= 0) {
-            const double s2 = fma((double)rv, (double)rv, red2);
-            red2 = own ? s2 : red2;
-          }
-        }
-      } else if (EPI == EPI_PCG) {  // w = K p, (p, w)
-        const bool own = owned_plane(k.g, kk);
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          k.out[n + m * N] = tot[m];
-          const double s0 = fma((double)st.at(si - 1, m, 0, lane), (double)tot[m], red0);
-          red0 = own ? s0 : red0;
-        }
-      } else if (EPI == EPI_FAS) {
-        // coarsen_f_standard_routine (multigrid_intergrid.cpp:124-342) fused with the coarse apply;
-        // a slab's lower ghost plane has no fine plane below it (its value comes from the neighbour)
-        const int fz = 2 * kk + k.g.zsh;
-#pragma unroll
-        for (int m = 0; m < 3; ++m)
-          k.out[n + m * N] =
-              tot[m] + (fz >= 0 ? full_weight(k.gf, k.rf + (long long)m * k.gf.n, 2 * x, 2 * ey, fz) : T(0));
-      } else if (EPI == EPI_REACTION) {
-        // Dirichlet_force_u (boundary_conditions.cpp:69-111)
-        const BcFlags bc = bc_flags(k.g, x, ey, kk);
-        if (bc.c0) k.out[n] = tot[0];
-        if (bc.c1) k.out[n + N] = tot[1];
-        if (bc.c2) k.out[n + 2 * N] = tot[2];
+        for (int m = 0; m < 3; ++m) own_p[m] = st.at(si - 1, m, 0, lane);
       }
+      T pre_f[3] = {T(0), T(0), T(0)}, pre_m[3] = {T(0), T(0), T(0)};
+      if (EPI == EPI_RESIDUAL) {
+        const long long n = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          pre_f[m] = k.fu[n + m * k.g.n];
+          if (k.invM) pre_m[m] = k.invM[n + m * k.g.n];
+        }
+      }
+      node_epilogue<T, EPI>(k, x, ey, kk, tot, own_p, pre_f, pre_m, red0, red1, red2);
     }
   }
 #pragma unroll
@@ -369,43 +221,24 @@ __device__ __forceinline__ void assemble_row(const MechKT<T>& k, const ST& st, i
     for (int m = 0; m < 3; ++m) yp[c][m] = X[1][c][m];
 }
 
-// T = double: the plain form; T = float: the precision form's V-cycle (reductions stay FP64).
-// GPM: the finest level's Gauss-point moduli come precomputed (gp_material_kernel) instead of being
-// interpolated from the staged nodal K, G, d in every apply.
-// TMA: the finest applies on precomputed moduli stage their rows with tensor copies (TmaStream)
-// instead of per-lane cp.async; the same values reach the same arithmetic, so the same bits.
-template <typename T, bool FINEST, int EPI, bool DIAG, bool ISO, bool GPM = false, bool TMA = false>
-__global__ void __launch_bounds__(kWarps * 32) mech_kernel(const __grid_constant__ MechKT<T> k) {
+// The finest level from its nodal moduli and phase field (calls outside a running solve), and the
+// diagonals of every level.
+template <bool FINEST, int EPI, bool DIAG, bool ISO>
+__global__ void __launch_bounds__(kWarps * 32) mech_kernel(const __grid_constant__ MechK k) {
+  using T = double;
   constexpr int NU = DIAG ? 0 : 3;
-  constexpr int NF = NU + (FINEST ? (GPM ? 0 : 3) : 2);
-  static_assert(!TMA || (FINEST && GPM && !DIAG), "TMA staging serves the finest applies on precomputed moduli");
+  constexpr int NF = NU + (FINEST ? 3 : 2);
   extern __shared__ __align__(128) unsigned char mech_smem[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  // per warp: [TMA: 4 mbarriers] the staging ring, then the z-carry of the strip's wy - 1 output rows
-  const size_t wbytes = TMA ? tma_warp_bytes<T>(k.sg.wy)
-                            : (size_t)(kRing * NF * 2 * kRowW + (k.sg.wy - 1) * 3 * 32) * sizeof(T);
-  // TMA: ring slots on 128-byte boundaries (the launch adds 128 bytes for this alignment)
-  unsigned char* base = TMA ? mech_smem + ((128u - (smem_u32(mech_smem) & 127u)) & 127u) : mech_smem;
-  unsigned char* wbase = base + (size_t)wib * wbytes;
-  T* ring = reinterpret_cast<T*>(wbase + (TMA ? kTmaHead : 0));
-  T* zc = ring + (TMA ? (size_t)kRing * TmaStream<T>::SLOT : (size_t)kRing * NF * 2 * kRowW);  // [row][comp][lane]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(wbase);
-  if constexpr (TMA) {
-    if (lane == 0) {
-#pragma unroll
-      for (int i = 0; i < kRing; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bars + i)) : "memory");
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    __syncwarp();
-  }
-  const SFt<T> s = make_sf<T>(k.g);
+  // per warp: the staging ring, then the z-carry of the strip's wy - 1 output rows
+  T* ring = reinterpret_cast<T*>(mech_smem) + (size_t)wib * (kRing * NF * 2 * kRowW + (k.sg.wy - 1) * 3 * 32);
+  T* zc = ring + (size_t)kRing * NF * 2 * kRowW;  // [row][comp][lane]
+  const SF s = make_sf(k.g);
   double red0 = 0.0, red1 = 0.0, red2 = 0.0;
   const long long nwarps_total = (long long)gridDim.x * kWarps;
   const T* fptr[NF];
 #pragma unroll
   for (int f = 0; f < NF; ++f) fptr[f] = k.fields[f];
-  unsigned staged = 0;  // rows this warp staged so far (TMA: slot and barrier phase bookkeeping)
 
   for (long long strip = (long long)blockIdx.x * kWarps + wib; strip < k.sg.nstrips; strip += nwarps_total) {
     const int sx = (int)(strip % k.sg.tx);
@@ -417,103 +250,83 @@ __global__ void __launch_bounds__(kWarps * 32) mech_kernel(const __grid_constant
     const int x = x0 - 1 + lane;
     const int zend = min(z0 + k.sg.cz - 1, k.g.nz - 1);
     const int nlayers = zend - z0 + 2;
-    // one strip, whichever staging: rows issued two ahead, each row waited for before use
-    auto run_strip = [&](auto& st) -> bool {
-      st.issue(0, lane);
-      st.issue(1, lane);
-      T yp[2][3];
-      for (int si = 0; si < st.total; ++si) {
-        st.issue(si + 2, lane);
-        if (!st.wait(si)) return false;
-        const int li = si / rows, r = si - li * rows;
-        const int kk = z0 - 1 + li;
-        if (r == 0) {
+    Stream<NF, T> st{ring, fptr, x, y0, z0, nlayers, nlayers * rows, rows, &k.g};
+    st.issue(0, lane);
+    st.issue(1, lane);
+    T yp[2][3];
+    for (int si = 0; si < st.total; ++si) {
+      st.issue(si + 2, lane);
+      st.wait();
+      const int li = si / rows, r = si - li * rows;
+      const int kk = z0 - 1 + li;
+      if (r == 0) {
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+        for (int c = 0; c < 2; ++c)
 #pragma unroll
-            for (int m = 0; m < 3; ++m) yp[c][m] = T(0);
-          __syncwarp();
-          continue;
-        }
-        const int rr = r - 1, ey = y0 - 1 + rr;
-        if (EPI == EPI_RESIDUAL && rr >= 1 && kk >= z0 && lane >= 1 && lane <= 30 && x < k.g.nx && ey < k.g.ny) {
-          // the epilogue reads f and M^-1 of this row's output node: start them towards L2 now, so
-          // their latency overlaps the element math instead of following it
-          const long long n = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
-#pragma unroll
-          for (int m = 0; m < 3; ++m) {
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(k.fu + n + m * k.g.n));
-            if (k.invM) asm volatile("prefetch.global.L2 [%0];" ::"l"(k.invM + n + m * k.g.n));
-          }
-        }
-        // ---- element (x, ey, kk) from stream rows si-1 (y = ey) and si (y = ey+1)
-        T f[3][8];
-        const bool valid = lane < 31 && x >= 0 && x <= k.g.nx - 2 && ey >= 0 && ey <= k.g.ny - 2 && kk >= 0 &&
-                           kk <= k.g.nz - 2;
-        if (valid) {
-          T Kw[8], Gw[8];
-          // ISO: the 1/h^2 of the two gradients goes into the Gauss weight (see sf_forward)
-          const T wg = ISO ? T(k.g.wg) * (s.ih[0] * s.ih[0]) : T(k.g.wg);
-          if (FINEST && GPM) {
-            const long long e = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              Kw[g] = k.gpm[(long long)g * k.g.n + e];
-              Gw[g] = k.gpm[(long long)(8 + g) * k.g.n + e];
-            }
-          } else if (FINEST) {
-            T Kn[8], Gn[8], dn[8];
-#pragma unroll
-            for (int n = 0; n < 8; ++n) {
-              const int a = n & 1, b = (n >> 1) & 1, c = n >> 2;
-              const int srow = b ? si : si - 1;
-              Kn[n] = st.at(srow, NU + 0, c, lane + a);
-              Gn[n] = st.at(srow, NU + 1, c, lane + a);
-              dn[n] = st.at(srow, NU + 2, c, lane + a);
-            }
-            const long long e = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
-            mech_moduli_finest(Kn, Gn, dn, k.choice[e], T(k.small_k), wg, s, Kw, Gw);
-          } else {
-            const T K = st.at(si - 1, NU + 0, 0, lane) * wg, G = st.at(si - 1, NU + 1, 0, lane) * wg;
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              Kw[g] = K;
-              Gw[g] = G;
-            }
-          }
-          if constexpr (DIAG) {
-            mech_element_diag(Kw, Gw, s, f);
-          } else {
-            T u[3][8];
-#pragma unroll
-            for (int n = 0; n < 8; ++n) {
-              const int a = n & 1, b = (n >> 1) & 1, c = n >> 2;
-              const int srow = b ? si : si - 1;
-#pragma unroll
-              for (int m = 0; m < 3; ++m) u[m][n] = st.at(srow, m, c, lane + a);
-            }
-            mech_element<ISO, T, FINEST && GPM>(u, Kw, Gw, s, f);
-          }
-        } else {
-#pragma unroll
-          for (int m = 0; m < 3; ++m)
-#pragma unroll
-            for (int n = 0; n < 8; ++n) f[m][n] = T(0);
-        }
-        assemble_row<T, EPI>(k, st, si, lane, x, ey, kk, z0, rr, f, yp, zc, red0, red1, red2);
+          for (int m = 0; m < 3; ++m) yp[c][m] = T(0);
         __syncwarp();
+        continue;
       }
-      return true;
-    };
-    if constexpr (TMA) {
-      constexpr int A = 16 / (int)sizeof(T);  // columns per 16 bytes: the copy's x start is a multiple
-      const int xs = x0 - 1 >= 0 ? (x0 - 1) / A * A : -A;
-      TmaStream<T> st{ring, bars, &k.tmap, xs, (x0 - 1) - xs, y0, z0, nlayers, nlayers * rows, rows, staged, k.err};
-      if (!run_strip(st)) break;
-      staged += (unsigned)st.total;
-    } else {
-      Stream<NF, T> st{ring, fptr, x, y0, z0, nlayers, nlayers * rows, rows, &k.g};
-      run_strip(st);
+      const int rr = r - 1, ey = y0 - 1 + rr;
+      if (EPI == EPI_RESIDUAL && rr >= 1 && kk >= z0 && lane >= 1 && lane <= 30 && x < k.g.nx && ey < k.g.ny) {
+        // the epilogue reads f and M^-1 of this row's output node: start them towards L2 now, so
+        // their latency overlaps the element math instead of following it
+        const long long n = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(k.fu + n + m * k.g.n));
+          if (k.invM) asm volatile("prefetch.global.L2 [%0];" ::"l"(k.invM + n + m * k.g.n));
+        }
+      }
+      // ---- element (x, ey, kk) from stream rows si-1 (y = ey) and si (y = ey+1)
+      T f[3][8];
+      const bool valid = lane < 31 && x >= 0 && x <= k.g.nx - 2 && ey >= 0 && ey <= k.g.ny - 2 && kk >= 0 &&
+                         kk <= k.g.nz - 2;
+      if (valid) {
+        T Kw[8], Gw[8];
+        // ISO: the 1/h^2 of the two gradients goes into the Gauss weight (see sf_forward)
+        const T wg = ISO ? T(k.g.wg) * (s.ih[0] * s.ih[0]) : T(k.g.wg);
+        if (FINEST) {
+          T Kn[8], Gn[8], dn[8];
+#pragma unroll
+          for (int n = 0; n < 8; ++n) {
+            const int a = n & 1, b = (n >> 1) & 1, c = n >> 2;
+            const int srow = b ? si : si - 1;
+            Kn[n] = st.at(srow, NU + 0, c, lane + a);
+            Gn[n] = st.at(srow, NU + 1, c, lane + a);
+            dn[n] = st.at(srow, NU + 2, c, lane + a);
+          }
+          const long long e = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
+          mech_moduli_finest(Kn, Gn, dn, k.choice[e], T(k.small_k), wg, s, Kw, Gw);
+        } else {
+          const T K = st.at(si - 1, NU + 0, 0, lane) * wg, G = st.at(si - 1, NU + 1, 0, lane) * wg;
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            Kw[g] = K;
+            Gw[g] = G;
+          }
+        }
+        if constexpr (DIAG) {
+          mech_element_diag(Kw, Gw, s, f);
+        } else {
+          T u[3][8];
+#pragma unroll
+          for (int n = 0; n < 8; ++n) {
+            const int a = n & 1, b = (n >> 1) & 1, c = n >> 2;
+            const int srow = b ? si : si - 1;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) u[m][n] = st.at(srow, m, c, lane + a);
+          }
+          mech_element<ISO>(u, Kw, Gw, s, f);
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+#pragma unroll
+          for (int n = 0; n < 8; ++n) f[m][n] = T(0);
+      }
+      assemble_row<T, EPI>(k, st, si, lane, x, ey, kk, z0, rr, f, yp, zc, red0, red1, red2);
+      __syncwarp();
     }
   }
   if (EPI == EPI_RESIDUAL || EPI == EPI_PCG) {
@@ -852,7 +665,7 @@ __global__ void __launch_bounds__(kWarps * 32) mech_tc_kernel(MechKT<float> k) {
 }
 
 static int g_num_sms = 0;
-static int num_sms() {
+int num_sms() {
   if (g_num_sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -903,13 +716,12 @@ static std::mutex g_cfg_mu;
 static KernelCfg g_cfg[512];
 static int g_ncfg = 0;
 
-template <class Kern>
-static int kernel_cfg(Kern kern, size_t max_smem, size_t smem, int* per_sm_out) {
+int kernel_cfg(const void* kern, size_t max_smem, size_t smem, int threads, int* per_sm_out) {
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(g_cfg_mu);
   for (int i = 0; i < g_ncfg; ++i)
-    if (g_cfg[i].fn == (const void*)kern && g_cfg[i].device == dev && g_cfg[i].smem == smem) {
+    if (g_cfg[i].fn == kern && g_cfg[i].device == dev && g_cfg[i].smem == smem) {
       *per_sm_out = g_cfg[i].per_sm;
       return HPC_OK;
     }
@@ -920,9 +732,9 @@ static int kernel_cfg(Kern kern, size_t max_smem, size_t smem, int* per_sm_out) 
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(smem)");
   }
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, smem);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
   if (e != cudaSuccess || per_sm <= 0) per_sm = 1;
-  if (g_ncfg < 512) g_cfg[g_ncfg++] = KernelCfg{(const void*)kern, dev, smem, per_sm};
+  if (g_ncfg < 512) g_cfg[g_ncfg++] = KernelCfg{kern, dev, smem, per_sm};
   *per_sm_out = per_sm;
   return HPC_OK;
 }
@@ -971,7 +783,7 @@ static int autotune_shape(hpc_ctx* c, Kern kern, Args a, const SmemPlan& plan, S
       a.sg = strip_geo(a.g, wy, cz, ox);
       const size_t smem = plan.bytes(wy);
       int per_sm = 1;
-      if ((rc = kernel_cfg(kern, plan.bytes(kWY), smem, &per_sm))) break;
+      if ((rc = kernel_cfg((const void*)kern, plan.bytes(kWY), smem, kWarps * 32, &per_sm))) break;
       const int grid = grid_for(a.sg, (long long)num_sms() * per_sm);
       if (grid <= 0 || (size_t)grid * 3 > c->partials_cap) continue;
       kern<<<grid, kWarps * 32, smem, c->stream>>>(a);
@@ -1029,7 +841,7 @@ static int launch_strips(hpc_ctx* c, Kern kern, Args a, const SmemPlan& plan, in
   }
   const size_t smem = plan.bytes(a.sg.wy);
   int per_sm = 1;
-  if ((rc = kernel_cfg(kern, plan.bytes(kWY), smem, &per_sm))) return rc;
+  if ((rc = kernel_cfg((const void*)kern, plan.bytes(kWY), smem, kWarps * 32, &per_sm))) return rc;
   const int grid = grid_for(a.sg, (long long)num_sms() * per_sm);
   if (grid <= 0) return HPC_OK;
   if ((size_t)grid * 3 > c->partials_cap) return cuda_fail(cudaErrorInvalidValue, "partials buffer");
@@ -1073,20 +885,27 @@ static EncodeTiled tensor_map_encoder() {
   return fn;
 }
 template <typename T>
-static int encode_rows(const LevelGeo& g, const T* src, CUtensorMap* map) {
+int encode_tensor(const LevelGeo& g, const T* src, int ncomp, int bx, int by, int bz, CUtensorMap* map) {
   EncodeTiled enc = tensor_map_encoder();
   if (!enc) {
     set_error("TMA staging: cuTensorMapEncodeTiled unavailable");
     return HPC_ERR_CUDA;
   }
   const cuuint64_t es = sizeof(T);
-  const cuuint64_t dims[4] = {(cuuint64_t)g.px, (cuuint64_t)g.ny, (cuuint64_t)g.nz, 3};
+  const cuuint64_t dims[4] = {(cuuint64_t)g.px, (cuuint64_t)g.ny, (cuuint64_t)g.nz, (cuuint64_t)ncomp};
   const cuuint64_t strides[3] = {(cuuint64_t)g.px * es, (cuuint64_t)g.plane * es, (cuuint64_t)g.n * es};
-  const cuuint32_t box[4] = {(cuuint32_t)TmaShape<T>::BX, 1, 2, 3};
+  const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz, (cuuint32_t)ncomp};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = enc(map, sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-                         const_cast<T*>(src), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return enc(map, sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+                           const_cast<T*>(src), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {  // a host thread's first call: the runtime binds its context
+    HPC_CUDA(cudaFree(nullptr));
+    r = encode();
+  }
   if (r != CUDA_SUCCESS) {
     set_error("TMA staging: cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
     return HPC_ERR_CUDA;
@@ -1094,29 +913,18 @@ static int encode_rows(const LevelGeo& g, const T* src, CUtensorMap* map) {
   return HPC_OK;
 }
 
-template <bool F, int E, bool D, typename T = double>
-static int run_mech(hpc_ctx* c, const MechKT<T>& k, bool tma = false) {
-  const int cls = (F && E == EPI_PCG && !D) ? (sizeof(T) == 8 ? HPC_KC_MECH_PCG_FINEST : HPC_KC_MECH32_PCG_FINEST)
-                                             : HPC_KC_NONE;
-  if constexpr (F && !D) {
-    if (k.gpm && tma) {  // precomputed Gauss-point moduli, rows staged by tensor copies
-      const SmemPlan smem{128, (kTmaHead + (size_t)kRing * tma_slot_bytes<T>()) / sizeof(T), 3 * 32, sizeof(T)};
-      if (iso(k.g)) return launch_strips(c, mech_kernel<T, F, E, D, true, true, true>, k, smem, cls);
-      return launch_strips(c, mech_kernel<T, F, E, D, false, true, true>, k, smem, cls);
-    }
-    if (k.gpm) {  // precomputed Gauss-point moduli: only u is staged
-      constexpr int NF = 3;
-      const SmemPlan smem{0, (size_t)kRing * NF * 2 * kRowW, 3 * 32, sizeof(T)};
-      if (iso(k.g)) return launch_strips(c, mech_kernel<T, F, E, D, true, true>, k, smem, cls);
-      return launch_strips(c, mech_kernel<T, F, E, D, false, true>, k, smem, cls);
-    }
-  }
+template int encode_tensor<double>(const LevelGeo&, const double*, int, int, int, int, CUtensorMap*);
+template int encode_tensor<float>(const LevelGeo&, const float*, int, int, int, int, CUtensorMap*);
+
+template <bool F, int E, bool D>
+static int run_mech(hpc_ctx* c, const MechK& k) {
+  const int cls = (E == EPI_PCG && !D) ? HPC_KC_MECH_PCG_FINEST : HPC_KC_NONE;
   constexpr int NF = (D ? 0 : 3) + (F ? 3 : 2);
-  const SmemPlan smem{0, (size_t)kRing * NF * 2 * kRowW, 3 * 32, sizeof(T)};
+  const SmemPlan smem{0, (size_t)kRing * NF * 2 * kRowW, 3 * 32, sizeof(double)};
   if constexpr (!D) {
-    if (iso(k.g)) return launch_strips(c, mech_kernel<T, F, E, D, true>, k, smem, cls);
+    if (iso(k.g)) return launch_strips(c, mech_kernel<F, E, D, true>, k, smem, cls);
   }
-  return launch_strips(c, mech_kernel<T, F, E, D, false>, k, smem, cls);
+  return launch_strips(c, mech_kernel<F, E, D, false>, k, smem, cls);
 }
 
 static void mech_fields(hpc_ctx* c, int level, bool finest, bool diag, const double* src, MechK& k) {
@@ -1154,20 +962,12 @@ int launch_mech(hpc_ctx* c, const MechCall& m) {
   k.gpm = (m.finest && c->gpm_active) ? c->F[m.level].gpm : nullptr;
   k.red = make_red(c, m.s_out0, m.s_out1, m.s_out2);
   k.err = c->scal + S_ERR;
-  const bool f = m.finest;
-  const bool tma = f && k.gpm && c->tma_stage;
-  if (tma) {
-    const int rc = encode_rows<double>(k.g, k.fields[0], &k.tmap);
-    if (rc) return rc;
-  }
+  if (!m.finest || k.gpm) return launch_mech_tile(c, k, m.finest, m.epi);
   switch (m.epi) {
-    case EPI_PLAIN: return f ? run_mech<true, EPI_PLAIN, false>(c, k, tma) : run_mech<false, EPI_PLAIN, false>(c, k);
-    case EPI_RESIDUAL:
-      return f ? run_mech<true, EPI_RESIDUAL, false>(c, k, tma) : run_mech<false, EPI_RESIDUAL, false>(c, k);
-    case EPI_PCG: return f ? run_mech<true, EPI_PCG, false>(c, k, tma) : run_mech<false, EPI_PCG, false>(c, k);
-    case EPI_FAS: return run_mech<false, EPI_FAS, false>(c, k);
-    case EPI_REACTION:
-      return f ? run_mech<true, EPI_REACTION, false>(c, k, tma) : run_mech<false, EPI_REACTION, false>(c, k);
+    case EPI_PLAIN: return run_mech<true, EPI_PLAIN, false>(c, k);
+    case EPI_RESIDUAL: return run_mech<true, EPI_RESIDUAL, false>(c, k);
+    case EPI_PCG: return run_mech<true, EPI_PCG, false>(c, k);
+    case EPI_REACTION: return run_mech<true, EPI_REACTION, false>(c, k);
   }
   return HPC_ERR_ARG;
 }
@@ -1233,20 +1033,8 @@ int launch_mech_f32(hpc_ctx* c, const MechCall32& m) {
       case EPI_FAS: return run_mech_tc<false, EPI_FAS>(c, k);
     }
   }
-  const bool tma = fin && k.gpm && c->tma_stage;
-  if (tma) {
-    const int rc = encode_rows<float>(g, k.fields[0], &k.tmap);
-    if (rc) return rc;
-  }
-  switch (m.epi) {
-    case EPI_PLAIN:
-      return fin ? run_mech<true, EPI_PLAIN, false>(c, k, tma) : run_mech<false, EPI_PLAIN, false>(c, k);
-    case EPI_RESIDUAL:
-      return fin ? run_mech<true, EPI_RESIDUAL, false>(c, k, tma) : run_mech<false, EPI_RESIDUAL, false>(c, k);
-    case EPI_PCG: return fin ? run_mech<true, EPI_PCG, false>(c, k, tma) : run_mech<false, EPI_PCG, false>(c, k);
-    case EPI_FAS: return run_mech<false, EPI_FAS, false>(c, k);
-  }
-  return HPC_ERR_ARG;
+  if (fin && !k.gpm) return HPC_ERR_ARG;  // the V-cycle runs on precomputed moduli
+  return launch_mech_tile(c, k, fin, m.epi);
 }
 
 // Gauss-point moduli of the finest level, computed once per mechanical solve (the material is

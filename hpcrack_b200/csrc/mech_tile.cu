@@ -1,0 +1,464 @@
+// Mechanical operator on column tiles: the finest level with the Gauss-point moduli of the running
+// solve, the coarse levels with element-constant moduli, FP64 and FP32, with the fused epilogues of
+// element_common.cuh.
+//
+// A block owns a tile of kTX x TY element columns (one thread each) and marches it up z over a chunk of
+// output planes; it finishes the (kTX - 1) x (TY - 1) inner node columns.  Marching lets a thread keep,
+// per node plane, what both element layers that touch the plane need:
+//   * forward: the in-plane part of the gradients (the x- and y-derivatives interpolated to the 2x2
+//     in-plane Gauss coordinates, and the interpolated values) is formed once per plane, not once per
+//     element, from 4 nodes per component;
+//   * adjoint: the stresses of the layers below and above a plane are added in that in-plane form, and
+//     taken back to the 4 nodes once per plane.
+// That is about 365 floating-point operations per element against 600 for element-by-element sum
+// factorisation, and half the node assembly.  x-neighbours are combined with a shuffle inside a row of
+// 16 lanes, y-neighbours through a shared-memory row exchange, one block barrier per layer.
+// Node planes and moduli arrive up to three layers ahead in shared-memory stages (tensor copies by one
+// thread, completion on the stage's mbarrier, or per-thread cp.async); the carried parts stay in
+// registers, two layers per loop turn so that they swap roles instead of being moved.
+//
+// What bounds it: FP64, the FP64 pipe (66 % of its cycles on 193^3; two warps per scheduler cannot hide
+// all dependent latencies); FP32, instruction issue (80 % of the slots).  Per launch on B200, with the
+// element-by-element strip kernel it replaced in brackets: 257^3 FP64 656 us (1043), FP32 401 us (759);
+// 129^3 109 (196), 68 (151); 65^3 28 (63), 21 (53); 33^3 16 (25), 15 (23).  At 176 (88) bytes a node the
+// 257^3 applies move 4.6 (3.7) TB/s.
+// Every node is written once, by the tile that owns it, with the same arithmetic wherever tile and
+// chunk boundaries fall: no atomics, deterministic, independent of the chunk height except for the
+// order of the reductions.
+#include <algorithm>
+
+#include "element_common.cuh"
+
+namespace hpc {
+namespace {
+
+constexpr int kTX = 16;  // element columns of a tile in x: a half-warp, 128 B (64 B) of FP64 (FP32) per row
+constexpr unsigned kTileWaitPolls = 1u << 24;  // far above any copy's latency; then the kernel reports
+
+// Columns staged per row: the 17 nodes of a tile plus the offset to the copy's 16-byte aligned start.
+template <typename T> struct TileRow;
+template <> struct TileRow<double> { static constexpr int BX = 18; };
+template <> struct TileRow<float> { static constexpr int BX = 20; };
+
+// Shared memory of a block: [0, 128) the stages' mbarriers; the stages' node planes and (finest) moduli
+// layers; the y exchange.
+template <typename T, bool GPM, int TY, int NS>
+struct TileSmem {
+  static constexpr int BX = TileRow<T>::BX, NT = kTX * TY, XP = 20;  // XP: exchange row pitch (bank spread)
+  static constexpr size_t up(size_t b) { return (b + 127) / 128 * 128; }
+  static constexpr size_t node = up(sizeof(T) * 3 * (TY + 1) * BX), mod = GPM ? up(sizeof(T) * 16 * TY * BX) : 0;
+  static constexpr size_t o_node = 128, o_mod = o_node + NS * node, o_exch = o_mod + NS * mod;
+  static constexpr size_t total = o_exch + sizeof(T) * 2 * 3 * TY * XP;
+  static constexpr size_t bytes = total + 128;  // + alignment of the dynamic base
+};
+
+// What a thread carries from one element layer to the next: of the node plane between them the in-plane
+// forward parts (ex, dy, iy; see plane_forward), the lower layer's adjoint parts (aex, ady, and its
+// stresses sz acting through d/dz), and the thread's own node value.
+template <typename T>
+struct PlaneState {
+  T ex[3][2], dy[3][2], iy[3][4], aex[3][2], ady[3][2], sz[3][4], own[3];
+};
+
+// In-plane part of one node plane, per component: ex[p] = d/dx at in-plane Gauss row p, dy[q] = d/dy at
+// Gauss column q, iy[q + 2p] = value.  v[a + 2b] = node (a, b).
+template <typename T>
+__device__ __forceinline__ void plane_forward(const T (&v)[4], const T (&t)[2], T (&ex)[2], T (&dy)[2], T (&iy)[4]) {
+  const T d0 = v[1] - v[0], d1 = v[3] - v[2], dd = d1 - d0;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const T i0 = fma(t[q], d0, v[0]), i1 = fma(t[q], d1, v[2]);
+    dy[q] = i1 - i0;
+    iy[q] = fma(t[0], dy[q], i0);
+    iy[q + 2] = fma(t[1], dy[q], i0);
+    ex[q] = fma(t[q], dd, d0);
+  }
+}
+// Exact transpose of plane_forward.
+template <typename T>
+__device__ __forceinline__ void plane_adjoint(const T (&ex)[2], const T (&dy)[2], const T (&iy)[4], const T (&t)[2],
+                                              T (&f)[4]) {
+  T d1 = fma(t[1], ex[1], t[0] * ex[0]);
+  T d0 = ex[0] + ex[1] - d1;
+  T i0[2], i1[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    i1[q] = fma(t[1], iy[q + 2], fma(t[0], iy[q], dy[q]));
+    i0[q] = iy[q] + iy[q + 2] - i1[q];
+  }
+  d0 = fma(t[1], i0[1], fma(t[0], i0[0], d0));
+  d1 = fma(t[1], i1[1], fma(t[0], i1[0], d1));
+  f[1] = d0;
+  f[0] = i0[0] + i0[1] - d0;
+  f[3] = d1;
+  f[2] = i1[0] + i1[1] - d1;
+}
+
+template <typename T, bool GPM, int EPI, bool ISO, bool TMA, int TY, int MINB, int NS>
+__global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_constant__ MechKT<T> k) {
+  using S = TileSmem<T, GPM, TY, NS>;
+  constexpr int BX = S::BX, NT = S::NT, NY = TY + 1;
+  extern __shared__ __align__(128) unsigned char tile_smem[];
+  unsigned char* base = tile_smem + ((128u - (smem_u32(tile_smem) & 127u)) & 127u);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base);
+  T* exch = reinterpret_cast<T*>(base + S::o_exch);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & (kTX - 1);
+  // the two half-warps of a warp work 4 rows apart: with the staged row pitch that spreads an FP32
+  // warp over all 32 banks
+  const int row = (warp & 3) + 4 * (lane >> 4) + 8 * (warp >> 2);
+  constexpr int A16 = 16 / (int)sizeof(T);  // columns per 16 bytes: a tensor copy's x start is a multiple
+  const SFt<T> s = make_sf<T>(k.g);
+  const T wg = ISO ? T(k.g.wg) * (s.ih[0] * s.ih[0]) : T(k.g.wg);
+  double red0 = 0.0, red1 = 0.0, red2 = 0.0;
+  int bad = 0;
+
+  if constexpr (TMA) {
+    if (tid == 0) {
+#pragma unroll
+      for (int i = 0; i < NS; ++i)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bars + i)) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+  }
+  // tiles fastest: the blocks resident together work the same planes of neighbouring tiles, so that the
+  // cache lines and DRAM pages a tile's rows share with its neighbours are fetched once
+  const int tiles = k.sg.tx * k.sg.ty, chunks = (int)gridDim.x / tiles;
+  const int tile = (int)(blockIdx.x % (unsigned)tiles), chunk = (int)(blockIdx.x / (unsigned)tiles);
+  const int z0 = (int)((long long)k.g.nz * chunk / chunks), zend = (int)((long long)k.g.nz * (chunk + 1) / chunks) - 1;
+  const int x0 = (tile % k.sg.tx) * (kTX - 1), y0 = (tile / k.sg.tx) * (TY - 1);
+  const int x = x0 - 1 + tx, y = y0 - 1 + row;
+  const int nl = zend - z0 + 2;  // element layers z0 - 1 .. zend; plane j of the stream is z0 - 1 + j
+  const int xs = x0 - 1 >= 0 ? (x0 - 1) / A16 * A16 : -A16;
+  const int off = (x0 - 1) - xs;
+  const bool xy_elem = x >= 0 && x <= k.g.nx - 2 && y >= 0 && y <= k.g.ny - 2;
+  const bool out_node = tx >= 1 && row >= 1 && x < k.g.nx && y < k.g.ny;
+
+  auto node_slot = [&](int j) {
+    return reinterpret_cast<T*>(base + S::o_node + (size_t)((unsigned)j % NS) * S::node);
+  };
+  auto mod_slot = [&](int j) {
+    return reinterpret_cast<T*>(base + S::o_mod + (size_t)((unsigned)j % NS) * S::mod);
+  };
+  // Stage j: node plane j and (finest) the moduli of element layer j - 1, the one below the plane.
+  auto issue = [&](int j) {
+    if (j <= nl) {
+      const int kk = z0 - 1 + j;
+      if constexpr (TMA) {
+        if (tid == 0) {
+          const uint32_t bar = smem_u32(bars + (unsigned)j % NS);
+          const bool mods = GPM && j >= 1;
+          const int bytes = (int)sizeof(T) * BX * (3 * NY + (mods ? 16 * TY : 0));
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+          asm volatile(
+              "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+              "%4, %5}], [%6];" ::"r"(smem_u32(node_slot(j))),
+              "l"(&k.tmap), "r"(xs), "r"(y0 - 1), "r"(kk), "r"(0), "r"(bar)
+              : "memory");
+          if (mods)
+            asm volatile(
+                "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+                "%3, %4, %5}], [%6];" ::"r"(smem_u32(mod_slot(j))),
+                "l"(&k.gmap), "r"(xs), "r"(y0 - 1), "r"(kk - 1), "r"(0), "r"(bar)
+                : "memory");
+        }
+      } else {
+        // the nodes of a row one column apart, zeros outside the grid
+        T* dst = node_slot(j);
+        for (int q = tid; q < 3 * NY * 17; q += NT) {
+          const int c = q % 17, r = q / 17, ry = r % NY, m = r / NY;
+          const int gx = x0 - 1 + c, gy = y0 - 1 + ry;
+          const bool ok = gx >= 0 && gx < k.g.nx && gy >= 0 && gy < k.g.ny && kk >= 0 && kk < k.g.nz;
+          const T* src = k.fields[m] + (ok ? (long long)gx + (long long)gy * k.g.px + (long long)kk * k.g.plane : 0);
+          const unsigned d = smem_u32(dst + (m * NY + ry) * BX + off + c);
+          asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(sizeof(T)),
+                       "r"(ok ? (int)sizeof(T) : 0)
+                       : "memory");
+        }
+        if (GPM && j >= 1) {
+          T* md = mod_slot(j) + row * BX + off + tx;
+          const bool ok = xy_elem && kk >= 1 && kk - 1 <= k.g.nz - 2;
+          const T* src = k.gpm + (ok ? (long long)x + (long long)y * k.g.px + (long long)(kk - 1) * k.g.plane : 0);
+#pragma unroll
+          for (int g = 0; g < 16; ++g) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(smem_u32(md + g * TY * BX)),
+                         "l"(src + (long long)g * k.g.n), "n"(sizeof(T)), "r"(ok ? (int)sizeof(T) : 0)
+                         : "memory");
+          }
+        }
+      }
+    }
+    if constexpr (!TMA) asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  // Stage j has landed, for every thread: this thread's wait; without tensor copies the others' too.  A
+  // wait that runs out returns false: the block then stops and reports.
+  auto wait = [&](int j) -> bool {
+    if constexpr (TMA) {
+            const uint32_t bar = smem_u32(bars + (unsigned)j % NS), parity = ((unsigned)j / NS) & 1u;
+      for (unsigned i = 0; i < kTileWaitPolls; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, "
+            "p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+      }
+      return false;
+    } else {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(NS - 1) : "memory");
+      __syncthreads();
+      return true;
+    }
+  };
+  // coarse levels: the element's moduli one layer ahead in registers
+  T lam_n = T(0), G_n = T(0);
+  auto coarse_mod = [&](int kk) {
+    lam_n = G_n = T(0);
+    if (!GPM && xy_elem && kk >= 0 && kk <= k.g.nz - 2) {
+      const long long e = (long long)x + (long long)y * k.g.px + (long long)kk * k.g.plane;
+      const T K = k.fields[3][e] * wg;
+      G_n = k.fields[4][e] * wg;
+      lam_n = fma(T(-2.0 / 3.0), G_n, K);
+    }
+  };
+
+  // One element layer li: state a of the node plane below it -> state b of the plane above; the plane
+  // below is finished.  False when a wait ran out.
+  auto layer = [&](int li, const PlaneState<T>& a, PlaneState<T>& b) -> bool {
+    const int kk = z0 - 1 + li;
+    const T lam_c = lam_n, G_c = G_n;
+    if (!GPM) coarse_mod(kk + 1);
+    // the residual's f and M^-1 of this plane's node: in flight under the arithmetic
+    T pre_f[3], pre_m[3];
+    if (EPI == EPI_RESIDUAL && out_node && kk >= z0) {
+      const long long n = (long long)x + (long long)y * k.g.px + (long long)kk * k.g.plane;
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        pre_f[m] = k.fu[n + m * k.g.n];
+        pre_m[m] = k.invM ? k.invM[n + m * k.g.n] : T(0);
+      }
+    }
+    if (!wait(li + 1)) bad = 1;
+    // ---- upper node plane: in-plane parts; d/dz between the planes
+    T gz[3][4];
+    {
+      const T* nd = node_slot(li + 1) + row * BX + off + tx;
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        const T v[4] = {nd[m * NY * BX], nd[m * NY * BX + 1], nd[m * NY * BX + BX], nd[m * NY * BX + BX + 1]};
+        plane_forward(v, s.t, b.ex[m], b.dy[m], b.iy[m]);
+        b.own[m] = v[0];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          gz[m][q] = b.iy[m][q] - a.iy[m][q];
+          if (!ISO) gz[m][q] *= s.ih[2];
+        }
+      }
+    }
+    // ---- stresses of the layer by Gauss level r; lo: the lower plane's adjoint with the layer below
+    T lo_ex[3][2], lo_dy[3][2];
+    const T* mod = mod_slot(li + 1) + row * BX + off + tx;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      T gx[3][2], gy[3][2], sx[3][2], sy[3][2];
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          gx[m][q] = fma(s.t[r], b.ex[m][q] - a.ex[m][q], a.ex[m][q]);
+          gy[m][q] = fma(s.t[r], b.dy[m][q] - a.dy[m][q], a.dy[m][q]);
+          if (!ISO) {
+            gx[m][q] *= s.ih[0];
+            gy[m][q] *= s.ih[1];
+          }
+        }
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int i = q + 2 * p;
+          const T lam = GPM ? mod[(i + 4 * r) * TY * BX] : lam_c, G = GPM ? mod[(8 + i + 4 * r) * TY * BX] : G_c;
+          const T exx = gx[0][p], eyy = gy[1][q], ezz = gz[2][i];
+          const T lt = lam * (exx + eyy + ezz), G2 = G + G;
+          const T sxy = G * (gx[1][p] + gy[0][q]), sxz = G * (gx[2][p] + gz[0][i]), syz = G * (gy[2][q] + gz[1][i]);
+          const T sxx = fma(G2, exx, lt), syy = fma(G2, eyy, lt), szz = fma(G2, ezz, lt);
+          sx[0][p] = q ? sx[0][p] + sxx : sxx;
+          sx[1][p] = q ? sx[1][p] + sxy : sxy;
+          sx[2][p] = q ? sx[2][p] + sxz : sxz;
+          sy[0][q] = p ? sy[0][q] + sxy : sxy;
+          sy[1][q] = p ? sy[1][q] + syy : syy;
+          sy[2][q] = p ? sy[2][q] + syz : syz;
+          b.sz[0][i] = r ? b.sz[0][i] + sxz : sxz;
+          b.sz[1][i] = r ? b.sz[1][i] + syz : syz;
+          b.sz[2][i] = r ? b.sz[2][i] + szz : szz;
+        }
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (!ISO) {
+            sx[m][q] *= s.ih[0];
+            sy[m][q] *= s.ih[1];
+          }
+          // 1 - t[r] = t[1 - r]
+          lo_ex[m][q] = fma(s.t[1 - r], sx[m][q], r ? lo_ex[m][q] : a.aex[m][q]);
+          lo_dy[m][q] = fma(s.t[1 - r], sy[m][q], r ? lo_dy[m][q] : a.ady[m][q]);
+          b.aex[m][q] = r ? fma(s.t[1], sx[m][q], b.aex[m][q]) : s.t[0] * sx[m][q];
+          b.ady[m][q] = r ? fma(s.t[1], sy[m][q], b.ady[m][q]) : s.t[0] * sy[m][q];
+        }
+    }
+    // ---- lower plane finished: back to its nodes, x-neighbours by shuffle, y-neighbours by exchange
+    T X0[3];
+    T* ex_w = exch + (size_t)(li & 1) * 3 * TY * S::XP + row * S::XP + tx;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      T iy[4], f[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (!ISO) b.sz[m][q] *= s.ih[2];
+        iy[q] = a.sz[m][q] - b.sz[m][q];
+      }
+      plane_adjoint(lo_ex[m], lo_dy[m], iy, s.t, f);
+      X0[m] = f[0] + __shfl_up_sync(kFull, f[1], 1, kTX);
+      ex_w[m * TY * S::XP] = f[2] + __shfl_up_sync(kFull, f[3], 1, kTX);
+    }
+    bad = __syncthreads_or(bad);
+    if (bad) return false;
+    issue(li + 1 + NS);  // into the stage every thread has just read
+    if (kk >= z0 && out_node) {
+      T tot[3];
+#pragma unroll
+      for (int m = 0; m < 3; ++m) tot[m] = X0[m] + ex_w[m * TY * S::XP - S::XP];
+      node_epilogue<T, EPI>(k, x, y, kk, tot, a.own, pre_f, pre_m, red0, red1, red2);
+    }
+    return true;
+  };
+
+#pragma unroll
+  for (int j = 0; j < NS; ++j) issue(j);
+  coarse_mod(z0 - 1);
+  PlaneState<T> a, b;
+  if (!wait(0)) bad = 1;
+  {
+    const T* nd = node_slot(0) + row * BX + off + tx;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const T v[4] = {nd[m * NY * BX], nd[m * NY * BX + 1], nd[m * NY * BX + BX], nd[m * NY * BX + BX + 1]};
+      plane_forward(v, s.t, a.ex[m], a.dy[m], a.iy[m]);
+      a.own[m] = v[0];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a.sz[m][q] = T(0);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) a.aex[m][q] = a.ady[m][q] = T(0);
+    }
+  }
+  bad = __syncthreads_or(bad);
+  if (!bad) issue(NS);
+  // two layers per turn: the two states swap roles instead of being copied
+  for (int li = 0; !bad;) {
+    if (!layer(li, a, b) || ++li == nl) break;
+    if (!layer(li, b, a) || ++li == nl) break;
+  }
+  if constexpr (!TMA) asm volatile("cp.async.wait_all;\n" ::: "memory");
+  if (TMA && bad && tid == 0 && k.err) *k.err = 1.0;
+  if (EPI == EPI_RESIDUAL || EPI == EPI_PCG) {
+    double v[3] = {red0, red1, red2};
+    grid_reduce<3>(v, k.red);
+  }
+}
+
+// Tile height, resident blocks the registers are budgeted for, and staged layers.  FP64: 8 rows, 2 blocks of
+// 128 threads (a layer's state and arithmetic take 230-250 registers); 16 rows in one block leave nothing
+// to run across the layer barrier (257^3 apply 822 us against 737 us), a third block needs the carried
+// state in shared memory, whose traffic then binds (815 us).  FP32: 16 rows, 2 blocks of 256 threads (125
+// registers); with 8 rows the tiles overlap more (410 against 401 us).  Two stages instead of three cost
+// FP64 7 % (703 against 656 us): a layer's arithmetic is too short to cover the copies.
+template <typename T> struct TileShape;
+template <> struct TileShape<double> { static constexpr int TY = 8, MINB = 2, NS = 3; };
+template <> struct TileShape<float> { static constexpr int TY = 16, MINB = 1, NS = 3; };
+
+// Tiles of a level and the z chunks they are marched in: a chunk of cz planes costs its block cz + 1 layers
+// and a pipeline start of about two layers' time, and blocks run in waves of `slots`; the number of
+// chunks that minimises waves x (cz + 3) wins.
+StripGeo tile_geo(const LevelGeo& g, int ty, long long slots, long long cap) {
+  StripGeo s;
+  s.wy = ty;
+  s.tx = (g.nx + kTX - 2) / (kTX - 1);
+  s.ty = (g.ny + ty - 2) / (ty - 1);
+  const long long tiles = (long long)s.tx * s.ty;
+  long long best = -1;
+  for (int n = 1; n <= g.nz && (n == 1 || tiles * n <= cap); ++n) {
+    const int cz = (g.nz + n - 1) / n;
+    const long long cost = ((tiles * n + slots - 1) / slots) * (cz + 3);
+    if (best < 0 || cost < best) {
+      best = cost;
+      s.cz = cz;
+      s.tz = n;
+    }
+  }
+  s.nstrips = tiles * s.tz;
+  return s;
+}
+
+template <typename T, bool GPM, int EPI, bool ISO, bool TMA>
+int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
+  constexpr int TY = TileShape<T>::TY, NS = TileShape<T>::NS;
+  using S = TileSmem<T, GPM, TY, NS>;
+  auto kern = mech_tile_kernel<T, GPM, EPI, ISO, TMA, TY, TileShape<T>::MINB, NS>;
+  int per_sm = 1, rc;
+  if ((rc = kernel_cfg((const void*)kern, S::bytes, S::bytes, kTX * TY, &per_sm))) return rc;
+  k.sg = tile_geo(k.g, TY, (long long)num_sms() * per_sm, (long long)c->partials_cap / 3);
+  if ((size_t)k.sg.nstrips * 3 > c->partials_cap) return cuda_fail(cudaErrorInvalidValue, "partials buffer");
+  if constexpr (TMA) {
+    if ((rc = encode_tensor<T>(k.g, k.fields[0], 3, S::BX, TY + 1, 1, &k.tmap))) return rc;
+    if (GPM && (rc = encode_tensor<T>(k.g, k.gpm, 16, S::BX, TY, 1, &k.gmap))) return rc;
+  }
+  timing_begin(c, cls);
+  kern<<<(unsigned)k.sg.nstrips, kTX * TY, S::bytes, c->stream>>>(k);
+  timing_end(c, cls);
+  HPC_CHECK_LAUNCH(c);
+  return HPC_OK;
+}
+
+template <typename T, bool GPM, int EPI>
+int run_tile_e(hpc_ctx* c, MechKT<T>& k, int cls) {
+  const bool iso = k.g.hx == k.g.hy && k.g.hy == k.g.hz;
+  if (c->tma_stage) return iso ? run_tile<T, GPM, EPI, true, true>(c, k, cls) : run_tile<T, GPM, EPI, false, true>(c, k, cls);
+  return iso ? run_tile<T, GPM, EPI, true, false>(c, k, cls) : run_tile<T, GPM, EPI, false, false>(c, k, cls);
+}
+
+}  // namespace
+
+template <typename T>
+int launch_mech_tile(hpc_ctx* c, MechKT<T>& k, bool finest, int epi) {
+  const int pcg = sizeof(T) == 8 ? HPC_KC_MECH_PCG_FINEST : HPC_KC_MECH32_PCG_FINEST;
+  if (finest) {
+    switch (epi) {
+      case EPI_RESIDUAL: return run_tile_e<T, true, EPI_RESIDUAL>(c, k, HPC_KC_NONE);
+      case EPI_PCG: return run_tile_e<T, true, EPI_PCG>(c, k, pcg);
+      case EPI_REACTION:
+        if constexpr (sizeof(T) == 8) return run_tile_e<T, true, EPI_REACTION>(c, k, HPC_KC_NONE);
+        break;
+      case EPI_PLAIN: return run_tile_e<T, true, EPI_PLAIN>(c, k, HPC_KC_NONE);
+    }
+    return HPC_ERR_ARG;
+  }
+  switch (epi) {
+    case EPI_RESIDUAL: return run_tile_e<T, false, EPI_RESIDUAL>(c, k, HPC_KC_NONE);
+    case EPI_PCG: return run_tile_e<T, false, EPI_PCG>(c, k, HPC_KC_NONE);
+    case EPI_FAS: return run_tile_e<T, false, EPI_FAS>(c, k, HPC_KC_NONE);
+    case EPI_PLAIN: return run_tile_e<T, false, EPI_PLAIN>(c, k, HPC_KC_NONE);
+    case EPI_REACTION:
+      if constexpr (sizeof(T) == 8) return run_tile_e<T, false, EPI_REACTION>(c, k, HPC_KC_NONE);
+      break;
+  }
+  return HPC_ERR_ARG;
+}
+template int launch_mech_tile<double>(hpc_ctx*, MechKT<double>&, bool, int);
+template int launch_mech_tile<float>(hpc_ctx*, MechKT<float>&, bool, int);
+
+}  // namespace hpc
