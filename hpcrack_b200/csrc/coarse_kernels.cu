@@ -1,14 +1,32 @@
-// The coarsest level's smoother in one thread block: pcg_u (mechanical_pcg.cpp:223-330) with all
-// of its iterations - Dirichlet values, residual, direction, K p, dots, updates - in one launch,
-// the level's vectors and element forces held in shared memory.  The V-cycle calls the coarsest
-// solve once per cycle with 50 iterations (mechanical_multigrid.cpp:29-32); on a 9^3 level the
-// multi-kernel smoother spends its time in launch and grid-synchronisation latency (three
-// dependent kernels per iteration), which this kernel replaces by block barriers.
+// Smoothers of small levels in one thread-block cluster: pcg_u (mechanical_pcg.cpp:223-330) with all of
+// its iterations - Dirichlet values, residual, direction, K p, dots, updates - in one launch, the
+// level's vectors in the cluster's shared memory.  The V-cycle calls the coarsest solve once per cycle
+// with 50 iterations (mechanical_multigrid.cpp:29-32) and the next levels' smoothers with a few; as
+// separate kernels an iteration costs three dependent launches and their reduction tails.
 //
-// Element forces are computed element-parallel into a shared buffer and gathered per node in a
-// fixed order (no atomics): results are deterministic; their rounding differs from the strip
-// kernels' only in the order of the same sums.
+// The level is cut into slabs of node planes along its longest axis, one slab per block of the cluster.
+// A block computes every element layer that touches its planes (the layers between two slabs are
+// computed by both), so an iteration exchanges only two things: the dot-product partials, written by
+// every warp to every block, and the preconditioned residual of the slabs' boundary planes, from which
+// a neighbour forms its ghost copy of the direction.  They travel as asynchronous stores into the
+// receiver's shared memory that its mbarrier counts, two exchanges per iteration: (p, w), and (r, M^-1 r)
+// with the boundary planes.  A buffer is written again only after every warp has read it: a block sends
+// the next (p, w) when it has every warp's (r, M^-1 r), which a warp sends after reading its (p, w).
+//
+// Element forces are computed element-parallel into shared memory and gathered per node in a fixed order
+// (layer below, layer above): no atomics, the sums are the same for every number of blocks; the
+// partials are added in rank and warp order.  The rounding differs from the
+// tile kernels' only in the order of the same sums.
+//
+// What bounds it: the serial chain of an iteration (about 2.4 us on 9^3: a third the element arithmetic and
+// gather, a third the two sums with their quotients, the rest the direction, the updates and the
+// exchanges).  50 iterations on 9^3: 121 us, against 388 us in one thread block, and 194 us with cluster
+// barriers and release fences instead of counted stores; 4 iterations on 17^3 take 33 us against about
+// 90 us in separate kernels.  Increments: 33^3 FAS 6.3 -> 5.1 ms, 65^3 precision form (3) 98 -> 74 ms.
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <mutex>
 
 #include "device_common.cuh"
 #include "internal.h"
@@ -16,216 +34,507 @@
 namespace hpc {
 namespace {
 
-constexpr int kCoarseThreads = 512;
+constexpr int kBlocks = 16;  // cluster size (non-portable; hpc_create asks for it)
+constexpr size_t kMaxSmem = 220 * 1024;
 
-struct CoarseArgs {
-  LevelGeo g;
-  double* u;
-  const double* fu;
-  double* ru;
-  const double* invM;
-  const double* Ke;
-  const double* Ge;
-  double Ut;
-  int nb;
-  double* scal;
-  int s_rnorm;
+// How a level is laid over the cluster.
+struct ClusterPlan {
+  int axis;            // planes are cut along this axis (0 x, 1 y, 2 z)
+  int planes, n1, n2;  // extent along it; the other two axes, n1 the lower-numbered one
+  int active;          // blocks that hold planes
+  int lp;              // element layers a block computes at most
+  int threads, slots;  // threads a block; own nodes and elements a thread at most
+  size_t smem;
 };
 
-// Sum over the block in a fixed order (warp trees, then the warps' sums in warp order).
-__device__ double block_sum(double v, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  v = warp_sum(v);
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (warp == 0) {
-    t = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
-    t = warp_sum(t);
-    if (lane == 0) red[32] = t;
+// Block shapes, smallest first: a level takes the first that holds a block's share.  Own nodes and elements
+// are unrolled over `slots` (the nodes' vectors live in registers): a coarsest level that needs one slot
+// does not run through the code of more, which a few iterations would mostly spend fetching.
+constexpr int kShapes[][2] = {{128, 1}, {256, 2}, {512, 2}};
+
+// The level's longest axis is cut; false where a block's share exceeds the register slots or shared memory.
+template <typename T>
+bool cluster_plan(const LevelGeo& g, ClusterPlan* p) {
+  const int n[3] = {g.nx, g.ny, g.nz};
+  if (n[0] < 2 || n[1] < 2 || n[2] < 2) return false;
+  p->axis = 2;
+  for (int a = 1; a >= 0; --a)
+    if (n[a] > n[p->axis]) p->axis = a;
+  p->planes = n[p->axis];
+  p->n1 = p->axis == 0 ? n[1] : n[0];
+  p->n2 = p->axis == 2 ? n[1] : n[2];
+  p->active = std::min(kBlocks, p->planes);
+  const size_t PN = (size_t)p->n1 * p->n2, EN = (size_t)(p->n1 - 1) * (p->n2 - 1);
+  const size_t np = (size_t)(p->planes + p->active - 1) / p->active;
+  p->lp = (int)np + 1;
+  const size_t vals = 2 * 3 * PN + 3 * (np + 2) * PN + (2 + 24) * (np + 1) * EN;
+  for (const auto& sh : kShapes) {
+    p->threads = sh[0];
+    p->slots = sh[1];
+    p->smem = sizeof(double) * 3 * kBlocks * (sh[0] / 32) + sizeof(T) * vals + 32;
+    const size_t most = (size_t)sh[0] * sh[1];
+    if (np * PN <= most && (np + 1) * EN <= most) return p->smem <= kMaxSmem;
   }
-  __syncthreads();
-  return red[32];
+  return false;
 }
 
-__global__ void __launch_bounds__(kCoarseThreads, 1) coarse_pcg_kernel(CoarseArgs a) {
-  extern __shared__ __align__(16) double csm[];
-  const LevelGeo& g = a.g;
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int N = nx * ny * nz, ex = nx - 1, ey = ny - 1, ez = nz - 1, E = ex * ey * ez;
-  double* su = csm;          // 3N
-  double* sr = su + 3 * N;   // 3N
-  double* sp = sr + 3 * N;   // 3N
-  double* sw = sp + 3 * N;   // 3N
-  double* sm = sw + 3 * N;   // 3N inverse diagonal
-  double* sK = sm + 3 * N;   // E element moduli (times the Gauss weight, 1/h^2 folded when isotropic)
-  double* sG = sK + E;       // E
-  double* sf = sG + E;       // 24 E element forces [m*8+n][e]
-  double* red = sf + 24 * E; // 33
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const bool iso = g.hx == g.hy && g.hy == g.hz;
-  const SF s = make_sf(g);
-  const double wg = iso ? g.wg * (s.ih[0] * s.ih[0]) : g.wg;
+// u, fu, ru in IO; the arithmetic and the material in T.
+template <typename T, typename IO>
+struct ClusterArgs {
+  LevelGeo g;
+  ClusterPlan p;
+  IO* u;
+  const IO* fu;
+  IO* ru;  // may be null
+  const T* invM;
+  const T* Ke;
+  const T* Ge;
+  T Ut;
+  int nb;
+  double* scal;
+  int s_rnorm;  // -1: not wanted
+  double* err;  // set to 1 when a bounded wait ran out
+};
 
-  // ---- load the level (dense layout in shared memory) and set the Dirichlet values (Dirichlet_BD)
-  for (int q = tid; q < N; q += nt) {
-    const int i = q % nx, j = (q / nx) % ny, k = q / (nx * ny);
-    const long long n = nidx(g, i, j, k);
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t remote(uint32_t addr, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// A value into another block's shared memory, counted by the mbarrier beside it (no fence, no cluster
+// barrier: the receiver waits for the bytes).
+__device__ __forceinline__ void put(uint32_t addr, uint32_t bar, double v) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(addr), "d"(v),
+               "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void put(uint32_t addr, uint32_t bar, float v) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(addr), "f"(v),
+               "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void expect(uint32_t bar, int bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+constexpr unsigned kClusterPolls = 1u << 22;  // far above any exchange's latency; then the kernel reports
+// The phase of `bar` with this parity has completed; false when the wait ran out.
+__device__ __forceinline__ bool arrived(uint32_t bar, uint32_t parity) {
+  for (unsigned i = 0; i < kClusterPolls; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, "
+        "1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename T, typename IO, bool ISO, int kThreads, int kSlots>
+__global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_constant__ ClusterArgs<T, IO> A) {
+  constexpr int kWarpsC = kThreads / 32;
+  extern __shared__ __align__(16) unsigned char csm[];
+  const LevelGeo& g = A.g;
+  const ClusterPlan& P = A.p;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)blockIdx.x;
+  const int PN = P.n1 * P.n2, E1 = P.n1 - 1, EN = E1 * (P.n2 - 1);
+  // own planes [a, b), element layers [la, lb); local plane 0 of the direction is plane a - 1
+  const bool active = rank < P.active;
+  const int a = active ? (int)((long long)P.planes * rank / P.active) : 0;
+  const int b = active ? (int)((long long)P.planes * (rank + 1) / P.active) : 0;
+  const int np = b - a, la = max(a - 1, 0), lb = active ? min(b, P.planes - 1) : la;
+  const int NO = np * PN, NE = (lb - la) * EN;     // own nodes, elements computed
+  // mbarriers of the two exchanges of an iteration, then what they bring
+  const uint32_t barA = smem_addr(csm), barB = barA + 8;
+  double* partA = reinterpret_cast<double*>(csm + 16);  // (p, w) partials of every warp of the cluster
+  double* partB = partA + kBlocks * kWarpsC;       // (r, M^-1 r)
+  double* partN = partB + kBlocks * kWarpsC;       // |r|^2 of the first residual
+  // M^-1 r of planes a - 1 and b, from the neighbours (ahead of what depends on a block's own np: every
+  // block has it at the same address)
+  T* zh = reinterpret_cast<T*>(partN + kBlocks * kWarpsC);
+  const int SP = (np + 2) * PN;
+  T* sp = zh + 2 * 3 * PN;  // direction, component stride SP
+  T* sK = sp + 3 * SP;      // element moduli lam and G (times the Gauss weight; over h^2 when isotropic)
+  T* sG = sK + P.lp * EN;
+  T* sf = sG + P.lp * EN;   // element forces [m*8+n][element]
+  const int FS = P.lp * EN;
+  const SFt<T> s = make_sf<T>(g);
+  const T wg = ISO ? T(g.wg) * (s.ih[0] * s.ih[0]) : T(g.wg);
+  // local offsets of a step in x, y, z (nodes)
+  const int sx = P.axis == 0 ? PN : 1, sy = P.axis == 0 ? 1 : (P.axis == 1 ? PN : P.n1), sz = P.axis == 2 ? PN : P.n1;
+  auto coords = [&](int plane, int i1, int i2, int& i, int& j, int& k) {
+    if (P.axis == 0) {
+      i = plane, j = i1, k = i2;
+    } else if (P.axis == 1) {
+      i = i1, j = plane, k = i2;
+    } else {
+      i = i1, j = i2, k = plane;
+    }
+  };
+  auto node = [&](int pl, int in) {
+    int i, j, k;
+    coords(pl, in % P.n1, in / P.n1, i, j, k);
+    return nidx(g, i, j, k);
+  };
+  auto node_fix = [&](int pl, int in, bool& top) -> unsigned {
+    int i, j, k;
+    coords(pl, in % P.n1, in / P.n1, i, j, k);
     const BcFlags bc = bc_flags(g, i, j, k);
-    const bool fix[3] = {bc.c0, bc.c1, bc.c2};
+    top = bc.top;
+    return (bc.c0 ? 1u : 0u) | (bc.c1 ? 2u : 0u) | (bc.c2 ? 4u : 0u);
+  };
+
+  // ---- load: the direction buffer takes u with its Dirichlet values (Dirichlet_BD), ghost planes included
+  for (int q = tid; q < SP; q += kThreads) {
+    const int pl = a - 1 + q / PN, in = q % PN;
+    const bool inside = active && pl >= 0 && pl < P.planes;
+    bool top = false;
+    const unsigned fx = inside ? node_fix(pl, in, top) : 0u;
+    const long long n = inside ? node(pl, in) : 0;
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      double uv = a.u[n + m * g.n];
-      if (fix[m]) uv = (m == 2 && bc.top) ? a.Ut : 0.0;
-      su[m * N + q] = uv;
-      sm[m * N + q] = a.invM[n + m * g.n];
-      sp[m * N + q] = 0.0;
+      T uv = inside ? (T)A.u[n + m * g.n] : T(0);
+      if ((fx >> m) & 1u) uv = (m == 2 && top) ? A.Ut : T(0);
+      sp[m * SP + q] = uv;
     }
   }
-  for (int e = tid; e < E; e += nt) {
-    const int i = e % ex, j = (e / ex) % ey, k = e / (ex * ey);
-    const long long n = nidx(g, i, j, k);
-    sK[e] = a.Ke[n] * wg;
-    sG[e] = a.Ge[n] * wg;
+  // elements q = tid + t kThreads: where element q's corner 0 sits in the direction buffer
+  int corner0[kSlots];
+#pragma unroll
+  for (int t = 0; t < kSlots; ++t) {
+    const int q = tid + t * kThreads;
+    corner0[t] = 0;
+    if (q < NE) {
+      const int l = la + q / EN, e = q % EN;
+      int i, j, k;
+      coords(l, e % E1, e / E1, i, j, k);
+      const long long n = nidx(g, i, j, k);
+      const T G = A.Ge[n] * wg;
+      sK[q] = ISO ? fma(T(-2.0 / 3.0), G, A.Ke[n] * wg) : A.Ke[n] * wg;
+      sG[q] = G;
+      corner0[t] = (l - (a - 1)) * PN + (e / E1) * P.n1 + e % E1;
+    }
   }
-  __syncthreads();
+  // own nodes q = tid + t kThreads: vectors in registers; the Dirichlet rows (bits 0-2), which corners of
+  // the node have an element (bits 8 + d + 2 d1 + 4 d2, d along the axis), and its corner-0 element's slot
+  T u[kSlots][3], r[kSlots][3], mi[kSlots][3], w[kSlots][3];
+  unsigned info[kSlots];
+  int eslot[kSlots];
+#pragma unroll
+  for (int t = 0; t < kSlots; ++t) {
+    const int q = tid + t * kThreads;
+    info[t] = 0;
+    eslot[t] = 0;
+    if (q < NO) {
+      const int pl = a + q / PN, in = q % PN, i1 = in % P.n1, i2 = in / P.n1;
+      const long long n = node(pl, in);
+      bool top;
+      info[t] = node_fix(pl, in, top);
+      eslot[t] = (pl - la) * EN + i2 * E1 + i1;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const int d = c & 1, d1 = (c >> 1) & 1, d2 = c >> 2;
+        if (pl - d >= 0 && pl - d < P.planes - 1 && i1 - d1 >= 0 && i1 - d1 < E1 && i2 - d2 >= 0 && i2 - d2 < P.n2 - 1)
+          info[t] |= 256u << c;
+      }
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        u[t][m] = (T)A.u[n + m * g.n];
+        if ((info[t] >> m) & 1u) u[t][m] = (m == 2 && top) ? A.Ut : T(0);
+        mi[t][m] = A.invM[n + m * g.n];
+      }
+    }
+  }
+  // element corner (d along the axis, d1, d2) -> corner number in x, y, z
+  const int cd = P.axis == 0 ? 1 : (P.axis == 1 ? 2 : 4), c1 = P.axis == 0 ? 2 : 1, c2 = P.axis == 2 ? 2 : 4;
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barA) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barB) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  cluster_sync();  // every block of the cluster has started and its barriers exist: it may be written to
+  // bytes an exchange brings to this block: a partial of every warp; with (r, M^-1 r) also the ghost planes
+  constexpr int kPartBytes = kBlocks * kWarpsC * (int)sizeof(double);
+  const int zbytes = active ? ((rank > 0) + (rank + 1 < P.active)) * 3 * PN * (int)sizeof(T) : 0;
+  bool ok = true;
+  uint32_t phA = 0, phB = 0;
+  auto receive = [&](uint32_t bar, uint32_t& phase) {  // after a wait that ran out none is tried again
+    if (ok && !arrived(bar, phase)) ok = false;
+    phase ^= 1u;
+  };
 
-  // element forces of the field v into sf, then gathered per node into out (fixed order)
-  auto apply = [&](const double* v, double* out) {
-    for (int e = tid; e < E; e += nt) {
-      const int i = e % ex, j = (e / ex) % ey, k = e / (ex * ey);
-      double uu[3][8], Kw[8], Gw[8], f[3][8];
+  // K v of the own nodes into w, v in the direction buffer
+  auto apply = [&]() {
+#pragma unroll
+    for (int t = 0; t < kSlots; ++t) {
+      const int q = tid + t * kThreads;
+      if (q >= NE) break;
+      const T* v = sp + corner0[t];
+      T f[3][8];
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
-        const int q = (i + (n & 1)) + (j + ((n >> 1) & 1)) * nx + (k + (n >> 2)) * nx * ny;
+        const int o = (n & 1) * sx + ((n >> 1) & 1) * sy + (n >> 2) * sz;
 #pragma unroll
-        for (int m = 0; m < 3; ++m) uu[m][n] = v[m * N + q];
-        Kw[n] = sK[e];
-        Gw[n] = sG[e];
+        for (int m = 0; m < 3; ++m) f[m][n] = v[m * SP + o];
       }
-      if (iso)
-        mech_element<true>(uu, Kw, Gw, s, f);
-      else
+      if constexpr (ISO) {
+        mech_element_const(f, sK[q], sG[q]);
+      } else {
+        T uu[3][8], Kw[8], Gw[8];
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+          Kw[n] = sK[q];
+          Gw[n] = sG[q];
+#pragma unroll
+          for (int m = 0; m < 3; ++m) uu[m][n] = f[m][n];
+        }
         mech_element<false>(uu, Kw, Gw, s, f);
+      }
 #pragma unroll
       for (int m = 0; m < 3; ++m)
 #pragma unroll
-        for (int n = 0; n < 8; ++n) sf[(m * 8 + n) * E + e] = f[m][n];
+        for (int n = 0; n < 8; ++n) sf[(m * 8 + n) * FS + q] = f[m][n];
     }
     __syncthreads();
-    for (int q = tid; q < N; q += nt) {
-      const int i = q % nx, j = (q / nx) % ny, k = q / (nx * ny);
-      double acc[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {  // the element whose corner n is this node
-        const int a0 = n & 1, b0 = (n >> 1) & 1, c0 = n >> 2;
-        const int ei = i - a0, ej = j - b0, ek = k - c0;
-        if (ei < 0 || ej < 0 || ek < 0 || ei >= ex || ej >= ey || ek >= ez) continue;
-        const int e = ei + ej * ex + ek * ex * ey;
+    for (int t = 0; t < kSlots; ++t) {
+      if (tid + t * kThreads >= NO) continue;
+      T acc[3] = {T(0), T(0), T(0)};
 #pragma unroll
-        for (int m = 0; m < 3; ++m) acc[m] += sf[(m * 8 + n) * E + e];
-      }
+      for (int d = 1; d >= 0; --d)
 #pragma unroll
-      for (int m = 0; m < 3; ++m) out[m * N + q] = acc[m];
+        for (int c = 0; c < 4; ++c) {
+          const int d1 = c & 1, d2 = c >> 1;
+          if (info[t] & (256u << (d + 2 * d1 + 4 * d2))) {
+            const T* fe = sf + (d * cd + d1 * c1 + d2 * c2) * FS + eslot[t] - (d * EN + d2 * E1 + d1);
+#pragma unroll
+            for (int m = 0; m < 3; ++m) acc[m] += fe[m * 8 * FS];
+          }
+        }
+#pragma unroll
+      for (int m = 0; m < 3; ++m) w[t][m] = acc[m];
     }
-    __syncthreads();
+  };
+  // this warp's partial to every block of the cluster
+  auto share = [&](double* part, uint32_t bar, double v) {
+    v = warp_sum(v);
+    if (lane < kBlocks) put(remote(smem_addr(part + rank * kWarpsC + warp), lane), remote(bar, lane), v);
+  };
+  // the cluster's sum, the same bits in every thread (rank and warp order, then the shuffle tree)
+  auto total = [&](const double* part) {
+    double v = 0.0;
+#pragma unroll
+    for (int q = 0; q < kBlocks * kWarpsC / 32; ++q) v += part[q * 32 + lane];
+    return warp_sum(v);
+  };
+  // M^-1 r of an own node on a boundary plane to the neighbour's ghost copy
+  auto share_z = [&](int q, int m, T z) {
+    if (q < PN && rank > 0) put(remote(smem_addr(zh + (3 + m) * PN + q), rank - 1), remote(barB, rank - 1), z);
+    if (q >= NO - PN && rank + 1 < P.active)
+      put(remote(smem_addr(zh + m * PN + q - (NO - PN)), rank + 1), remote(barB, rank + 1), z);
   };
 
-  // ---- Initial residual r = f - K u, zero on Dirichlet rows; rz = (r, M^-1 r)
-  apply(su, sw);
+  // ---- initial residual r = f - K u, zero on Dirichlet rows
+  if (tid == 0) expect(barB, 2 * kPartBytes + zbytes);
+  apply();
   double rz = 0.0, rn = 0.0;
-  for (int q = tid; q < N; q += nt) {
-    const int i = q % nx, j = (q / nx) % ny, k = q / (nx * ny);
-    const long long n = nidx(g, i, j, k);
-    const BcFlags bc = bc_flags(g, i, j, k);
-    const bool fix[3] = {bc.c0, bc.c1, bc.c2};
+#pragma unroll
+  for (int t = 0; t < kSlots; ++t) {
+    const int q = tid + t * kThreads;
+    if (q >= NO) continue;
+    const long long n = node(a + q / PN, q % PN);
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      const double rv = fix[m] ? 0.0 : a.fu[n + m * g.n] - sw[m * N + q];
-      sr[m * N + q] = rv;
-      rz = fma(rv, rv * sm[m * N + q], rz);
-      rn = fma(rv, rv, rn);
+      const T rv = (info[t] >> m) & 1u ? T(0) : (T)A.fu[n + m * g.n] - w[t][m], z = rv * mi[t][m];
+      r[t][m] = rv;
+      rz = fma((double)rv, (double)z, rz);
+      rn = fma((double)rv, (double)rv, rn);
+      share_z(q, m, z);
     }
   }
-  rz = block_sum(rz, red);
-  rn = block_sum(rn, red);
-  if (tid == 0 && a.s_rnorm >= 0) a.scal[a.s_rnorm] = rn;
+  share(partB, barB, rz);
+  share(partN, barB, rn);
+  receive(barB, phB);
+  rz = total(partB);
+  if (rank == 0 && warp == 0 && A.s_rnorm >= 0) {
+    rn = total(partN);
+    if (lane == 0) A.scal[A.s_rnorm] = rn;
+  }
 
   double rz_prev = 1.0;
-  for (int it = 0; it < a.nb; ++it) {
-    const double beta = it == 0 ? 0.0 : rz / rz_prev;
-    for (int q = tid; q < 3 * N; q += nt) {
-      const double z = sr[q] * sm[q];
-      sp[q] = it == 0 ? z : fma(beta, sp[q], z);
-    }
-    __syncthreads();
-    apply(sp, sw);
-    double pw = 0.0;
-    for (int q = tid; q < 3 * N; q += nt) pw = fma(sp[q], sw[q], pw);
-    pw = block_sum(pw, red);
-    const double alpha = rz / pw;
-    double rz_new = 0.0;
-    for (int q = tid; q < N; q += nt) {
-      const int i = q % nx, j = (q / nx) % ny, k = q / (nx * ny);
-      const BcFlags bc = bc_flags(g, i, j, k);
-      const bool fix[3] = {bc.c0, bc.c1, bc.c2};
+  for (int it = 0; it < A.nb; ++it) {
+    // direction p = M^-1 r + beta p; on the ghost planes from the neighbours' M^-1 r (planes outside the
+    // level stay zero)
+    const T beta = it == 0 ? T(0) : (T)(rz / rz_prev);
+#pragma unroll
+    for (int t = 0; t < kSlots; ++t) {
+      const int q = tid + t * kThreads;
+      if (q >= NO) continue;
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
-        const int o = m * N + q;
-        su[o] = fma(sp[o], alpha, su[o]);
-        const double rv = fix[m] ? 0.0 : fma(-sw[o], alpha, sr[o]);
-        sr[o] = rv;
-        rz_new = fma(rv, rv * sm[o], rz_new);
+        const T z = r[t][m] * mi[t][m];
+        T* p = sp + m * SP + PN + q;
+        *p = it == 0 ? z : fma(beta, *p, z);
       }
     }
-    rz_prev = rz;
-    rz = block_sum(rz_new, red);
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      if (side ? b >= P.planes : a == 0) continue;
+      for (int in = tid; in < PN; in += kThreads)
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          T* p = sp + m * SP + (side ? SP - PN : 0) + in;
+          const T z = zh[(side * 3 + m) * PN + in];
+          *p = it == 0 ? z : fma(beta, *p, z);
+        }
+    }
+    if (tid == 0) expect(barA, kPartBytes);
+    __syncthreads();
+    apply();
+    double pw = 0.0;
+#pragma unroll
+    for (int t = 0; t < kSlots; ++t) {
+      const int q = tid + t * kThreads;
+      if (q >= NO) continue;
+#pragma unroll
+      for (int m = 0; m < 3; ++m) pw = fma((double)sp[m * SP + PN + q], (double)w[t][m], pw);
+    }
+    share(partA, barA, pw);
+    const bool more = it + 1 < A.nb;
+    if (more && tid == 0) expect(barB, kPartBytes + zbytes);
+    receive(barA, phA);
+    const T alpha = (T)(rz / total(partA));
+    double rz_new = 0.0;
+#pragma unroll
+    for (int t = 0; t < kSlots; ++t) {
+      const int q = tid + t * kThreads;
+      if (q >= NO) continue;
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        u[t][m] = fma(sp[m * SP + PN + q], alpha, u[t][m]);
+        const T rv = (info[t] >> m) & 1u ? T(0) : fma(-w[t][m], alpha, r[t][m]), z = rv * mi[t][m];
+        r[t][m] = rv;
+        rz_new = fma((double)rv, (double)z, rz_new);
+        if (more) share_z(q, m, z);
+      }
+    }
+    if (more) {
+      share(partB, barB, rz_new);
+      receive(barB, phB);
+      rz_prev = rz;
+      rz = total(partB);
+    }
   }
 
   // ---- write u and the last residual back
-  for (int q = tid; q < N; q += nt) {
-    const int i = q % nx, j = (q / nx) % ny, k = q / (nx * ny);
-    const long long n = nidx(g, i, j, k);
+#pragma unroll
+  for (int t = 0; t < kSlots; ++t) {
+    const int q = tid + t * kThreads;
+    if (q >= NO) continue;
+    const long long n = node(a + q / PN, q % PN);
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      a.u[n + m * g.n] = su[m * N + q];
-      a.ru[n + m * g.n] = sr[m * N + q];
+      A.u[n + m * g.n] = (IO)u[t][m];
+      if (A.ru) A.ru[n + m * g.n] = (IO)r[t][m];
     }
   }
+  if (!ok && lane == 0) *A.err = 1.0;
+  cluster_sync();  // no block ends while another may still write to it
 }
 
-size_t coarse_smem_bytes(const LevelGeo& g) {
-  const size_t N = (size_t)g.nx * g.ny * g.nz, E = (size_t)(g.nx - 1) * (g.ny - 1) * (g.nz - 1);
-  return sizeof(double) * (15 * N + 26 * E + 33);
+template <typename T, typename IO>
+using ClusterKernel = void (*)(const ClusterArgs<T, IO>);
+template <typename T, typename IO, bool ISO>
+ClusterKernel<T, IO> shape_kernel(int threads) {
+  if (threads == 128) return cluster_pcg_kernel<T, IO, ISO, 128, 1>;
+  if (threads == 256) return cluster_pcg_kernel<T, IO, ISO, 256, 2>;
+  return cluster_pcg_kernel<T, IO, ISO, 512, 2>;
 }
 
-}  // namespace
-
-bool coarse_pcg_fits(hpc_ctx* c, int level) {
-  if (level == c->maxlevel) return false;  // the finest level's material is nodal, not element-constant
-  return coarse_pcg_fits_geo(c->L[level]);
-}
-bool coarse_pcg_fits_geo(const LevelGeo& g) { return coarse_smem_bytes(g) <= 220 * 1024; }
-
-// Shared-memory opt-in of the kernel on the current device (called by hpc_create).
-int coarse_pcg_prepare() {
-  HPC_CUDA(cudaFuncSetAttribute(coarse_pcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-  return HPC_OK;
-}
-
-int launch_coarse_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
-                         const double* Ke, const double* Ge, double Ut, int nb) {
-  const size_t smem = coarse_smem_bytes(g);
-  CoarseArgs a{g, u, fu, ru, invM, Ke, Ge, Ut, nb, c->scal, S_RNORM};
-  coarse_pcg_kernel<<<1, kCoarseThreads, smem, c->stream>>>(a);
+template <typename T, typename IO>
+int launch_cluster(hpc_ctx* c, const ClusterArgs<T, IO>& a) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kBlocks);
+  cfg.blockDim = dim3(a.p.threads);
+  cfg.dynamicSmemBytes = a.p.smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kBlocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const bool iso = a.g.hx == a.g.hy && a.g.hy == a.g.hz;
+  HPC_CUDA(cudaLaunchKernelEx(&cfg, iso ? shape_kernel<T, IO, true>(a.p.threads) : shape_kernel<T, IO, false>(a.p.threads),
+                              a));
   HPC_CHECK_LAUNCH(c);
   return HPC_OK;
 }
 
-int launch_coarse_pcg(hpc_ctx* c, int level, double Ut, int nb) {
+template <typename T, typename IO>
+int prepare() {
+  for (const auto& sh : kShapes)
+    for (ClusterKernel<T, IO> k : {shape_kernel<T, IO, true>(sh[0]), shape_kernel<T, IO, false>(sh[0])}) {
+      HPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+      HPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
+  return HPC_OK;
+}
+
+}  // namespace
+
+bool cluster_pcg_fits_geo(const LevelGeo& g) {
+  ClusterPlan p;
+  return cluster_plan<double>(g, &p);
+}
+bool cluster_pcg_fits(hpc_ctx* c, int level) {
+  if (level == c->maxlevel) return false;  // the finest level's material is nodal, not element-constant
+  return cluster_pcg_fits_geo(c->L[level]);
+}
+
+// Attributes of the kernels, set once per device (called by hpc_create).
+int cluster_pcg_prepare(int device) {
+  static std::mutex mu;
+  static bool done[64] = {};
+  std::lock_guard<std::mutex> lock(mu);
+  if (device >= 0 && device < 64 && done[device]) return HPC_OK;
+  int rc;
+  if ((rc = prepare<double, double>()) || (rc = prepare<double, float>()) || (rc = prepare<float, float>())) return rc;
+  if (device >= 0 && device < 64) done[device] = true;
+  return HPC_OK;
+}
+
+int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
+                          const double* Ke, const double* Ge, double Ut, int nb) {
+  ClusterArgs<double, double> a{g, {}, u, fu, ru, invM, Ke, Ge, Ut, nb, c->scal, S_RNORM, c->scal + S_ERR};
+  if (!cluster_plan<double>(g, &a.p)) return HPC_ERR_ARG;
+  return launch_cluster(c, a);
+}
+
+int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb) {
   const LevelFields& F = c->F[level];
-  return launch_coarse_pcg_on(c, c->L[level], F.u, F.fu, F.ru, F.preMu, F.Ke, F.Ge, Ut, nb);
+  return launch_cluster_pcg_on(c, c->L[level], F.u, F.fu, F.ru, F.preMu, F.Ke, F.Ge, Ut, nb);
+}
+
+int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb) {
+  const LevelF32& F = c->F32[level];
+  ClusterArgs<float, float> a{c->L[level], {}, F.u, F.fu, F.ru, F.invM, F.Ke, F.Ge, 0.f, nb, c->scal, -1, c->scal + S_ERR};
+  if (!cluster_plan<float>(a.g, &a.p)) return HPC_ERR_ARG;
+  return launch_cluster(c, a);
+}
+
+int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb) {
+  const LevelFields& F = c->F[level];
+  const LevelF32& G = c->F32[level];
+  ClusterArgs<double, float> a{c->L[level], {}, G.u, G.fu, nullptr, F.preMu, F.Ke, F.Ge, 0.0, nb, c->scal, S_RNORM, c->scal + S_ERR};
+  if (!cluster_plan<double>(a.g, &a.p)) return HPC_ERR_ARG;
+  return launch_cluster(c, a);
 }
 
 }  // namespace hpc

@@ -279,10 +279,10 @@ int pf_diags(hpc_ctx* c, int top, double lc) {
 // pcg_u (mechanical_pcg.cpp:223-330) with preMu of level l already built.  Device scalars only.
 static int pcg_u_dev(hpc_ctx* c, int l, double small_k, double Ut, int nb, int t) {
   if (nb > kMaxRelax) return arg_fail("nb_relax too large");
-  if (c->fused_coarsest && l == 0) {
-    const int mode = slab_coarsest_mode(c);
-    if (mode == 1) return slab_coarsest(c, Ut, nb);
-    if (mode == 0 && coarse_pcg_fits(c, l)) return launch_coarse_pcg(c, l, Ut, nb);
+  if (c->fused_coarsest) {
+    const int mode = slab_coarsest_mode(c);  // a split gathers its coarsest level only
+    if (mode == 1 && l == 0) return slab_coarsest(c, Ut, nb);
+    if (mode == 0 && cluster_pcg_fits(c, l)) return launch_cluster_pcg(c, l, Ut, nb);
   }
   LevelFields& F = c->F[l];
   int rc;
@@ -534,17 +534,26 @@ int gp_material(hpc_ctx* c, double small_k) {
   return HPC_OK;
 }
 
-// Kernels whose bounded waits ran out (tensor-core applies, TMA staging) report it in S_ERR.
+// Kernels whose bounded waits ran out (tensor-core applies, TMA staging, cluster exchanges) report it in
+// S_ERR.
+static int wait_error(hpc_ctx* c, double err) {
+  if (err == 0.0) return HPC_OK;
+  write_scalar(c, S_ERR, 0.0);
+  set_error("a bounded wait in a kernel (tensor copy, MMA completion or cluster exchange) ran out");
+  return HPC_ERR_CUDA;
+}
 int check_wait_error(hpc_ctx* c) {
   double err = 0.0;
-  int rc;
-  if ((rc = read_scalars(c, S_ERR, 1, &err))) return rc;
-  if (err != 0.0) {
-    write_scalar(c, S_ERR, 0.0);
-    set_error("a bounded wait in a kernel (tensor copy or MMA completion) ran out");
-    return HPC_ERR_CUDA;
-  }
-  return HPC_OK;
+  const int rc = read_scalars(c, S_ERR, 1, &err);
+  return rc ? rc : wait_error(c, err);
+}
+// The end of a smoother or cycle call: one scalar, and whether a wait ran out.
+static int read_result(hpc_ctx* c, int slot, double* out) {
+  double s[S_ERR + 1];
+  const int rc = read_scalars(c, 0, S_ERR + 1, s);
+  if (rc) return rc;
+  *out = s[slot];
+  return wait_error(c, s[S_ERR]);
 }
 
 // u_entire (mechanical_displacement.cpp:25-115).
@@ -592,7 +601,7 @@ static int u_entire_dev(hpc_ctx* c, const hpc_mg& mg, double small_k, double Ut,
     }
     if (rel <= mech_tol) break;
   }
-  if (c->tma_stage && (rc = check_wait_error(c))) return rc;
+  if ((rc = check_wait_error(c))) return rc;
   c->f_norm = f_norm;
   // externe_force_nodal (mechanical_right_hnd.cpp:18-38)
   if ((rc = launch_bc(c, L, c->F[L].u, nullptr, 0, Ut))) return rc;
@@ -663,6 +672,8 @@ int f32_material(hpc_ctx* c) {
 // residual is f itself and needs no operator apply.
 static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, bool u_zero = false) {
   if (nb > kMaxRelax) return arg_fail("nb_relax too large");
+  if (c->fused_coarsest && slab_coarsest_mode(c) == 0 && !c->tc_apply && cluster_pcg_fits(c, l))
+    return launch_cluster_pcg_f32(c, l, nb);
   LevelF32& F = c->F32[l];
   int rc;
   MechCall32 m{};
@@ -704,6 +715,8 @@ static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, bool u_zero = fals
 static int coarsest64(hpc_ctx* c, const hpc_mg& mg, double small_k) {
   const long long n3 = 3 * c->L[0].n;
   int rc;
+  if (c->fused_coarsest && slab_coarsest_mode(c) == 0 && cluster_pcg_fits(c, 0))
+    return launch_cluster_pcg_mixed(c, 0, mg.nu0);
   if ((rc = launch_to_f64(c, c->F32[0].u, c->F[0].u, n3))) return rc;
   if ((rc = launch_to_f64(c, c->F32[0].fu, c->F[0].fu, n3))) return rc;
   if ((rc = pcg_u_dev(c, 0, small_k, 0.0, mg.nu0, 1))) return rc;
@@ -903,7 +916,7 @@ static int u_entire_fcg_dev(hpc_ctx* c, const hpc_mg& mg, double small_k, double
     }
     rel = f_norm != 0 ? rn / f_norm : 1.0;
   }
-  if (((mixed && c->tc_apply) || c->tma_stage) && (rc = check_wait_error(c))) return rc;
+  if ((rc = check_wait_error(c))) return rc;
   c->f_norm = f_norm;
   // u = x, fu restored; externe_force_nodal (mechanical_right_hnd.cpp:18-38)
   HPC_CUDA(cudaMemcpyAsync(F.u, c->fcg.x, vbytes, cudaMemcpyDeviceToDevice, c->stream));
@@ -1155,7 +1168,7 @@ static int create_ctx(hpc_ctx** out, const hpc_geometry* geo, int device, int nr
   shape_table(N);
   int rc = upload_shape_table(N);
   if (rc) return fail(rc);
-  if ((rc = coarse_pcg_prepare())) return fail(rc);
+  if ((rc = cluster_pcg_prepare(device))) return fail(rc);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "create sync"));
   *out = c;
   return HPC_OK;
@@ -1541,8 +1554,7 @@ int hpc_pcg_u(hpc_ctx* c, int level, double small_k, double Ut, int nb_relax, in
   if (nb_relax > 0 && (rc = check_zero_diags(c, 0, "PreM_u"))) return rc;
   if ((rc = launch_invert(c, level, 3, c->F[level].preMu))) return rc;
   if ((rc = pcg_u_dev(c, level, small_k, Ut, nb_relax, t))) return rc;
-  if ((rc = read_scalars(c, S_FNORM, 1, f_norm))) return rc;
-  return HPC_OK;
+  return read_result(c, S_FNORM, f_norm);
 }
 
 int hpc_initial_residual_d(hpc_ctx* c, int level, double lc, double* r_norm) {
@@ -1584,7 +1596,7 @@ int hpc_cycle_u(hpc_ctx* c, int level, const hpc_mg* mg, double small_k, double 
   if ((rc = mech_diags(c, level, small_k))) return rc;
   long long it = 0;
   if ((rc = cycle_u_dev(c, level, *mg, small_k, Ut, t, &it))) return rc;
-  return read_scalars(c, S_FNORM, 1, f_norm);
+  return read_result(c, S_FNORM, f_norm);
 }
 
 int hpc_cycle_d(hpc_ctx* c, int level, const hpc_mg* mg, double lc, int t, double* fd_norm) {
@@ -1693,7 +1705,7 @@ int step_end_finish(hpc_ctx* c, const hpc_step_params* p, int mcy, long long mit
   if ((rc = read_scalars(c, S_RES0, 4, r3))) return rc;
   if (r3[3] != 0.0) {
     write_scalar(c, S_ERR, 0.0);
-    set_error("a bounded wait in a kernel (tensor copy or MMA completion) ran out");
+    set_error("a bounded wait in a kernel (tensor copy, MMA completion or cluster exchange) ran out");
     return HPC_ERR_CUDA;
   }
   const double FeW = r3[2] * p->voxel_size;

@@ -126,7 +126,7 @@ struct hpc_ctx {
   int use_graphs;
   int autotune;  // measure strip shapes on first use (hpc_set_autotune)
   int tc_apply;        // precision form: element contraction on the tensor cores (hpc_set_tensor_apply)
-  int fused_coarsest;  // coarse-level pcg_u in one block when the level fits (hpc_set_fused_coarsest)
+  int fused_coarsest;  // coarse-level pcg_u in one cluster when the level fits (hpc_set_fused_coarsest)
   int gpm_active;      // finest applies read F[maxlevel].gpm (set while a mechanical solve runs)
   int tma_stage;       // finest applies stage rows with tensor copies (hpc_set_tma_staging)
   // z-slab rank of a specimen split over ranks (hpc_create_slab); null for a whole specimen.  A
@@ -210,10 +210,10 @@ bool slab_levels(const hpc_geometry& g, int nr, int r, SlabLevel* out);
 int slab_attach(hpc_ctx* c, int nr, int r);  // a new context becomes rank r of nr
 void slab_release(hpc_ctx* c);
 // The coarsest level's pcg_u of a slab of several ranks, solved redundantly: every rank gathers the
-// whole coarsest level (its owned planes from every rank) and runs the one-block solver on it, then
+// whole coarsest level (its owned planes from every rank) and runs the one-cluster solver on it, then
 // keeps its own planes.  One exchange per visit instead of three collective steps per iteration.
 // 0: the context holds the whole coarsest level (no split, or one rank); 1: a split whose whole
-// coarsest level fits the one-block solver (slab_coarsest); 2: a split whose does not (per-iteration
+// coarsest level fits the one-cluster solver (slab_coarsest); 2: a split whose does not (per-iteration
 // kernels with their collective steps).
 int slab_coarsest_mode(hpc_ctx* c);
 int slab_coarsest(hpc_ctx* c, double Ut, int nb);
@@ -355,13 +355,16 @@ int launch_choice_level(hpc_ctx* c, int level, double small_k, bool do_choice, b
 int launch_crack(hpc_ctx* c, int level, const uint8_t* fx, const uint8_t* fy, const uint8_t* fz, double Hc);
 int launch_zero_count(hpc_ctx* c, int level, int ncomp, const double* v, int slot);
 int upload_shape_table(const double* N64);
-// Whole coarse-level pcg_u in one thread block (coarse_kernels.cu), for levels small enough
-bool coarse_pcg_fits(hpc_ctx* c, int level);
-int coarse_pcg_prepare();
-int launch_coarse_pcg(hpc_ctx* c, int level, double Ut, int nb);
-bool coarse_pcg_fits_geo(const LevelGeo& g);
-int launch_coarse_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
-                         const double* Ke, const double* Ge, double Ut, int nb);
+// Whole pcg_u of a small coarse level in one thread-block cluster (coarse_kernels.cu): FP64, FP32 mirror
+// (homogeneous Dirichlet values), and the FP32 mirror's u and fu with FP64 arithmetic and material.
+bool cluster_pcg_fits(hpc_ctx* c, int level);
+bool cluster_pcg_fits_geo(const LevelGeo& g);
+int cluster_pcg_prepare(int device);
+int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb);
+int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
+                          const double* Ke, const double* Ge, double Ut, int nb);
+int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb);
+int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb);
 int tuned_shapes(int* out5, int cap);  // measured strip shapes: {nx, ny, nz, wy, cz} per entry
 
 

@@ -357,7 +357,7 @@ int slab_coarsest_mode(hpc_ctx* c) {
   if (!c->slab || c->slab->nr == 1) return 0;
   LevelGeo g = c->L[0];
   g.nz = c->geo.element_nb[2] + 1;
-  return c->maxlevel > 0 && coarse_pcg_fits_geo(g) ? 1 : 2;
+  return c->maxlevel > 0 && cluster_pcg_fits_geo(g) ? 1 : 2;
 }
 
 int slab_coarsest(hpc_ctx* c, double Ut, int nb) {
@@ -401,7 +401,7 @@ int slab_coarsest(hpc_ctx* c, double Ut, int nb) {
   int rc = s->group ? local_gather(c, src, dst, nc, 5, co.g) : s->comm ? nccl_gather(c, src, dst, nc, 5, co.g) : no_transport();
   if (rc) return rc;
   // the same inputs on every rank, a deterministic solver: the same whole-level solution everywhere
-  if ((rc = launch_coarse_pcg_on(c, co.g, co.u, co.fu, co.ru, co.invM, co.Ke, co.Ge, Ut, nb))) return rc;
+  if ((rc = launch_cluster_pcg_on(c, co.g, co.u, co.fu, co.ru, co.invM, co.Ke, co.Ge, Ut, nb))) return rc;
   for (int m = 0; m < 3; ++m) {  // this rank's planes, ghost planes included
     HPC_CUDA(cudaMemcpyAsync(F.u + m * L.n, co.u + m * co.g.n + L.zb * L.plane, sizeof(double) * L.n,
                              cudaMemcpyDeviceToDevice, c->stream));

@@ -34,9 +34,8 @@ PRECISION_NU0_LARGE_COARSEST = 20
 
 
 def coarsest_in_one_block(maxlevel: int, element_nb) -> bool:
-    """Whether the library solves the coarsest level in one thread block (the rule of
-    coarse_pcg_fits in coarse_kernels.cu: 15 N + 26 E + 33 doubles of shared memory, at most 220 KiB,
-    and a coarsest level below the finest)."""
+    """Whether the coarsest level is small enough (15 N + 26 E + 33 doubles, at most 220 KiB: about 10^3
+    nodes, and below the finest level) for the precision form's longer coarsest solve."""
     e = [int(v) for v in element_nb]
     n_nodes = (e[0] + 1) * (e[1] + 1) * (e[2] + 1)
     n_elem = e[0] * e[1] * e[2]
@@ -235,7 +234,7 @@ class Hierarchy:
         self._c("hpc_set_tensor_apply", int(bool(on)))
 
     def set_fused_coarsest(self, on: bool):
-        """Coarsest-level pcg_u in one thread block (default) or as per-iteration kernels."""
+        """pcg_u of small coarse levels in one thread-block cluster (default) or as per-iteration kernels."""
         self._c("hpc_set_fused_coarsest", int(bool(on)))
 
     def set_tma_staging(self, on: bool = True):

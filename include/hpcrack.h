@@ -132,10 +132,10 @@ int hpc_set_choice_quirk(hpc_ctx* ctx, int reproduce);
 int hpc_set_autotune(hpc_ctx* ctx, int on);
 /* The measured shapes so far: up to cap entries {nx, ny, nz, element rows, planes}. */
 int hpc_tuned_shapes(int* out5, int cap, int* count);
-/* No counterpart in the reference: 1 (default) runs pcg_u on the coarsest level (mechanical_pcg.cpp:
- * 223-330 as called by mechanical_multigrid.cpp:29-32) in one thread block when the level fits in
- * shared memory (up to about 10^3 nodes); 0 uses the per-iteration kernels.  The two differ only in
- * the order of the same sums. */
+/* No counterpart in the reference: 1 (default) runs pcg_u on small coarse levels (mechanical_pcg.cpp:
+ * 223-330 as called by mechanical_multigrid.cpp:29-32 and 36-50) in one thread-block cluster when a
+ * level fits its shared memory (up to about 17^3 nodes); 0 uses the per-iteration kernels.  The two
+ * differ only in the order of the same sums. */
 int hpc_set_fused_coarsest(hpc_ctx* ctx, int on);
 /* No counterpart in the reference: 1 runs the element operator of the precision form's FP32 V-cycle
  * (mech_solver HPC_MECH_MIXED) on the tensor cores - strains and element forces as two TF32 GEMMs
@@ -369,7 +369,7 @@ int hpc_dmax_noalloc(const double* d, const double* d_old, long long n, double* 
  * mech_solver of hpc_step (hpc_batch_step returns HPC_ERR_ARG; the precision form's element
  * contraction stays on the CUDA cores), without strip autotuning; the coarse parts of its cycles replay as CUDA graphs
  * over NCCL (the NCCL calls captured inside), not over the in-process transport.  Its coarsest level is gathered on
- * every rank and solved redundantly by the one-block solver when the whole level fits it (one
+ * every rank and solved redundantly by the one-cluster solver when the whole level fits it (one
  * exchange per visit instead of three collective steps per iteration; hpc_set_fused_coarsest(ctx, 0)
  * selects the reference's distributed smoother there).
  * Out of scope: x and y splits. */
