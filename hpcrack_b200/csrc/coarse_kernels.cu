@@ -52,8 +52,12 @@ struct ClusterPlan {
 // does not run through the code of more, which a few iterations would mostly spend fetching.
 constexpr int kShapes[][2] = {{128, 1}, {256, 2}, {512, 2}};
 
+// Components of the field, and coefficients an element keeps: lam and G, or the phase field's mass and
+// gradient weights at its 8 Gauss points.
+template <bool PF> struct FieldShape { static constexpr int NC = PF ? 1 : 3, NM = PF ? 16 : 2; };
+
 // The level's longest axis is cut; false where a block's share exceeds the register slots or shared memory.
-template <typename T>
+template <typename T, bool PF>
 bool cluster_plan(const LevelGeo& g, ClusterPlan* p) {
   const int n[3] = {g.nx, g.ny, g.nz};
   if (n[0] < 2 || n[1] < 2 || n[2] < 2) return false;
@@ -67,11 +71,12 @@ bool cluster_plan(const LevelGeo& g, ClusterPlan* p) {
   const size_t PN = (size_t)p->n1 * p->n2, EN = (size_t)(p->n1 - 1) * (p->n2 - 1);
   const size_t np = (size_t)(p->planes + p->active - 1) / p->active;
   p->lp = (int)np + 1;
-  const size_t vals = 2 * 3 * PN + 3 * (np + 2) * PN + (2 + 24) * (np + 1) * EN;
+  constexpr int NC = FieldShape<PF>::NC, NM = FieldShape<PF>::NM;
+  const size_t vals = 2 * NC * PN + NC * (np + 2) * PN + (NM + 8 * NC) * (np + 1) * EN;
   for (const auto& sh : kShapes) {
     p->threads = sh[0];
     p->slots = sh[1];
-    p->smem = sizeof(double) * 3 * kBlocks * (sh[0] / 32) + sizeof(T) * vals + 32;
+    p->smem = sizeof(double) * 4 * kBlocks * (sh[0] / 32) + sizeof(T) * vals + 32;
     const size_t most = (size_t)sh[0] * sh[1];
     if (np * PN <= most && (np + 1) * EN <= most) return p->smem <= kMaxSmem;
   }
@@ -87,12 +92,12 @@ struct ClusterArgs {
   const IO* fu;
   IO* ru;  // may be null
   const T* invM;
-  const T* Ke;
+  const T* Ke;  // element moduli; phase field: nodal gc and element H
   const T* Ge;
-  T Ut;
+  T Ut;  // top value of u_z; phase field: the length scale lc
   int nb;
   double* scal;
-  int s_rnorm;  // -1: not wanted
+  int s_rnorm, s_fnorm;  // |r|^2 of the first residual, |f|^2 (phase field); -1: not wanted
   double* err;  // set to 1 when a bounded wait ran out
 };
 
@@ -136,9 +141,9 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <typename T, typename IO, bool ISO, int kThreads, int kSlots>
+template <typename T, typename IO, bool PF, bool ISO, int kThreads, int kSlots>
 __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_constant__ ClusterArgs<T, IO> A) {
-  constexpr int kWarpsC = kThreads / 32;
+  constexpr int kWarpsC = kThreads / 32, NC = FieldShape<PF>::NC, NM = FieldShape<PF>::NM;
   extern __shared__ __align__(16) unsigned char csm[];
   const LevelGeo& g = A.g;
   const ClusterPlan& P = A.p;
@@ -154,15 +159,14 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
   const uint32_t barA = smem_addr(csm), barB = barA + 8;
   double* partA = reinterpret_cast<double*>(csm + 16);  // (p, w) partials of every warp of the cluster
   double* partB = partA + kBlocks * kWarpsC;       // (r, M^-1 r)
-  double* partN = partB + kBlocks * kWarpsC;       // |r|^2 of the first residual
+  double* partN = partB + kBlocks * kWarpsC;       // |r|^2 of the first residual, then |f|^2
   // M^-1 r of planes a - 1 and b, from the neighbours (ahead of what depends on a block's own np: every
   // block has it at the same address)
-  T* zh = reinterpret_cast<T*>(partN + kBlocks * kWarpsC);
+  T* zh = reinterpret_cast<T*>(partN + 2 * kBlocks * kWarpsC);
   const int SP = (np + 2) * PN;
-  T* sp = zh + 2 * 3 * PN;  // direction, component stride SP
-  T* sK = sp + 3 * SP;      // element moduli lam and G (times the Gauss weight; over h^2 when isotropic)
-  T* sG = sK + P.lp * EN;
-  T* sf = sG + P.lp * EN;   // element forces [m*8+n][element]
+  T* sp = zh + 2 * NC * PN;  // direction, component stride SP
+  T* sc = sp + NC * SP;         // element coefficients [i][element]
+  T* sf = sc + NM * P.lp * EN;  // element forces [m*8+n][element]
   const int FS = P.lp * EN;
   const SFt<T> s = make_sf<T>(g);
   const T wg = ISO ? T(g.wg) * (s.ih[0] * s.ih[0]) : T(g.wg);
@@ -195,10 +199,10 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
     const int pl = a - 1 + q / PN, in = q % PN;
     const bool inside = active && pl >= 0 && pl < P.planes;
     bool top = false;
-    const unsigned fx = inside ? node_fix(pl, in, top) : 0u;
+    const unsigned fx = !PF && inside ? node_fix(pl, in, top) : 0u;
     const long long n = inside ? node(pl, in) : 0;
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
+    for (int m = 0; m < NC; ++m) {
       T uv = inside ? (T)A.u[n + m * g.n] : T(0);
       if ((fx >> m) & 1u) uv = (m == 2 && top) ? A.Ut : T(0);
       sp[m * SP + q] = uv;
@@ -215,15 +219,28 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
       int i, j, k;
       coords(l, e % E1, e / E1, i, j, k);
       const long long n = nidx(g, i, j, k);
-      const T G = A.Ge[n] * wg;
-      sK[q] = ISO ? fma(T(-2.0 / 3.0), G, A.Ke[n] * wg) : A.Ke[n] * wg;
-      sG[q] = G;
+      if constexpr (PF) {
+        double gcn[8], gcg[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) gcn[c] = A.Ke[nidx(g, i + (c & 1), j + ((c >> 1) & 1), k + (c >> 2))];
+        gp_material(gcn, s, gcg);
+        const double H2 = 2.0 * A.Ge[n], inv_lc = 1.0 / A.Ut;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          sc[c * FS + q] = g.wg * fma(gcg[c], inv_lc, H2);
+          sc[(8 + c) * FS + q] = wg * (gcg[c] * A.Ut);
+        }
+      } else {
+        const T G = A.Ge[n] * wg;
+        sc[q] = ISO ? fma(T(-2.0 / 3.0), G, A.Ke[n] * wg) : A.Ke[n] * wg;
+        sc[FS + q] = G;
+      }
       corner0[t] = (l - (a - 1)) * PN + (e / E1) * P.n1 + e % E1;
     }
   }
   // own nodes q = tid + t kThreads: vectors in registers; the Dirichlet rows (bits 0-2), which corners of
   // the node have an element (bits 8 + d + 2 d1 + 4 d2, d along the axis), and its corner-0 element's slot
-  T u[kSlots][3], r[kSlots][3], mi[kSlots][3], w[kSlots][3];
+  T u[kSlots][NC], r[kSlots][NC], mi[kSlots][NC], w[kSlots][NC];
   unsigned info[kSlots];
   int eslot[kSlots];
 #pragma unroll
@@ -234,8 +251,8 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
     if (q < NO) {
       const int pl = a + q / PN, in = q % PN, i1 = in % P.n1, i2 = in / P.n1;
       const long long n = node(pl, in);
-      bool top;
-      info[t] = node_fix(pl, in, top);
+      bool top = false;
+      info[t] = PF ? 0u : node_fix(pl, in, top);
       eslot[t] = (pl - la) * EN + i2 * E1 + i1;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -244,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
           info[t] |= 256u << c;
       }
 #pragma unroll
-      for (int m = 0; m < 3; ++m) {
+      for (int m = 0; m < NC; ++m) {
         u[t][m] = (T)A.u[n + m * g.n];
         if ((info[t] >> m) & 1u) u[t][m] = (m == 2 && top) ? A.Ut : T(0);
         mi[t][m] = A.invM[n + m * g.n];
@@ -261,7 +278,7 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
   cluster_sync();  // every block of the cluster has started and its barriers exist: it may be written to
   // bytes an exchange brings to this block: a partial of every warp; with (r, M^-1 r) also the ghost planes
   constexpr int kPartBytes = kBlocks * kWarpsC * (int)sizeof(double);
-  const int zbytes = active ? ((rank > 0) + (rank + 1 < P.active)) * 3 * PN * (int)sizeof(T) : 0;
+  const int zbytes = active ? ((rank > 0) + (rank + 1 < P.active)) * NC * PN * (int)sizeof(T) : 0;
   bool ok = true;
   uint32_t phA = 0, phB = 0;
   auto receive = [&](uint32_t bar, uint32_t& phase) {  // after a wait that ran out none is tried again
@@ -276,28 +293,37 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
       const int q = tid + t * kThreads;
       if (q >= NE) break;
       const T* v = sp + corner0[t];
-      T f[3][8];
+      T f[NC][8];
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
         const int o = (n & 1) * sx + ((n >> 1) & 1) * sy + (n >> 2) * sz;
 #pragma unroll
-        for (int m = 0; m < 3; ++m) f[m][n] = v[m * SP + o];
+        for (int m = 0; m < NC; ++m) f[m][n] = v[m * SP + o];
       }
-      if constexpr (ISO) {
-        mech_element_const(f, sK[q], sG[q]);
+      if constexpr (PF) {
+        double xv[8], aw[8], bw[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          xv[c] = f[0][c];
+          aw[c] = sc[c * FS + q];
+          bw[c] = sc[(8 + c) * FS + q];
+        }
+        pf_element<ISO>(xv, aw, bw, s, f[0]);
+      } else if constexpr (ISO) {
+        mech_element_const(f, sc[q], sc[FS + q]);
       } else {
         T uu[3][8], Kw[8], Gw[8];
 #pragma unroll
         for (int n = 0; n < 8; ++n) {
-          Kw[n] = sK[q];
-          Gw[n] = sG[q];
+          Kw[n] = sc[q];
+          Gw[n] = sc[FS + q];
 #pragma unroll
           for (int m = 0; m < 3; ++m) uu[m][n] = f[m][n];
         }
         mech_element<false>(uu, Kw, Gw, s, f);
       }
 #pragma unroll
-      for (int m = 0; m < 3; ++m)
+      for (int m = 0; m < NC; ++m)
 #pragma unroll
         for (int n = 0; n < 8; ++n) sf[(m * 8 + n) * FS + q] = f[m][n];
     }
@@ -305,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
 #pragma unroll
     for (int t = 0; t < kSlots; ++t) {
       if (tid + t * kThreads >= NO) continue;
-      T acc[3] = {T(0), T(0), T(0)};
+      T acc[NC] = {};
 #pragma unroll
       for (int d = 1; d >= 0; --d)
 #pragma unroll
@@ -314,11 +340,11 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
           if (info[t] & (256u << (d + 2 * d1 + 4 * d2))) {
             const T* fe = sf + (d * cd + d1 * c1 + d2 * c2) * FS + eslot[t] - (d * EN + d2 * E1 + d1);
 #pragma unroll
-            for (int m = 0; m < 3; ++m) acc[m] += fe[m * 8 * FS];
+            for (int m = 0; m < NC; ++m) acc[m] += fe[m * 8 * FS];
           }
         }
 #pragma unroll
-      for (int m = 0; m < 3; ++m) w[t][m] = acc[m];
+      for (int m = 0; m < NC; ++m) w[t][m] = acc[m];
     }
   };
   // this warp's partial to every block of the cluster
@@ -335,23 +361,25 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
   };
   // M^-1 r of an own node on a boundary plane to the neighbour's ghost copy
   auto share_z = [&](int q, int m, T z) {
-    if (q < PN && rank > 0) put(remote(smem_addr(zh + (3 + m) * PN + q), rank - 1), remote(barB, rank - 1), z);
+    if (q < PN && rank > 0) put(remote(smem_addr(zh + (NC + m) * PN + q), rank - 1), remote(barB, rank - 1), z);
     if (q >= NO - PN && rank + 1 < P.active)
       put(remote(smem_addr(zh + m * PN + q - (NO - PN)), rank + 1), remote(barB, rank + 1), z);
   };
 
   // ---- initial residual r = f - K u, zero on Dirichlet rows
-  if (tid == 0) expect(barB, 2 * kPartBytes + zbytes);
+  if (tid == 0) expect(barB, (PF ? 3 : 2) * kPartBytes + zbytes);
   apply();
-  double rz = 0.0, rn = 0.0;
+  double rz = 0.0, rn = 0.0, ff = 0.0;
 #pragma unroll
   for (int t = 0; t < kSlots; ++t) {
     const int q = tid + t * kThreads;
     if (q >= NO) continue;
     const long long n = node(a + q / PN, q % PN);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      const T rv = (info[t] >> m) & 1u ? T(0) : (T)A.fu[n + m * g.n] - w[t][m], z = rv * mi[t][m];
+    for (int m = 0; m < NC; ++m) {
+      const T fv = (T)A.fu[n + m * g.n];
+      const T rv = (info[t] >> m) & 1u ? T(0) : fv - w[t][m], z = rv * mi[t][m];
+      if (PF) ff = fma((double)fv, (double)fv, ff);
       r[t][m] = rv;
       rz = fma((double)rv, (double)z, rz);
       rn = fma((double)rv, (double)rv, rn);
@@ -360,11 +388,16 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
   }
   share(partB, barB, rz);
   share(partN, barB, rn);
+  if (PF) share(partN + kBlocks * kWarpsC, barB, ff);
   receive(barB, phB);
   rz = total(partB);
   if (rank == 0 && warp == 0 && A.s_rnorm >= 0) {
     rn = total(partN);
     if (lane == 0) A.scal[A.s_rnorm] = rn;
+    if (PF) {
+      ff = total(partN + kBlocks * kWarpsC);
+      if (lane == 0) A.scal[A.s_fnorm] = ff;
+    }
   }
 
   double rz_prev = 1.0;
@@ -377,7 +410,7 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
       const int q = tid + t * kThreads;
       if (q >= NO) continue;
 #pragma unroll
-      for (int m = 0; m < 3; ++m) {
+      for (int m = 0; m < NC; ++m) {
         const T z = r[t][m] * mi[t][m];
         T* p = sp + m * SP + PN + q;
         *p = it == 0 ? z : fma(beta, *p, z);
@@ -388,9 +421,9 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
       if (side ? b >= P.planes : a == 0) continue;
       for (int in = tid; in < PN; in += kThreads)
 #pragma unroll
-        for (int m = 0; m < 3; ++m) {
+        for (int m = 0; m < NC; ++m) {
           T* p = sp + m * SP + (side ? SP - PN : 0) + in;
-          const T z = zh[(side * 3 + m) * PN + in];
+          const T z = zh[(side * NC + m) * PN + in];
           *p = it == 0 ? z : fma(beta, *p, z);
         }
     }
@@ -403,7 +436,7 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
       const int q = tid + t * kThreads;
       if (q >= NO) continue;
 #pragma unroll
-      for (int m = 0; m < 3; ++m) pw = fma((double)sp[m * SP + PN + q], (double)w[t][m], pw);
+      for (int m = 0; m < NC; ++m) pw = fma((double)sp[m * SP + PN + q], (double)w[t][m], pw);
     }
     share(partA, barA, pw);
     const bool more = it + 1 < A.nb;
@@ -416,7 +449,7 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
       const int q = tid + t * kThreads;
       if (q >= NO) continue;
 #pragma unroll
-      for (int m = 0; m < 3; ++m) {
+      for (int m = 0; m < NC; ++m) {
         u[t][m] = fma(sp[m * SP + PN + q], alpha, u[t][m]);
         const T rv = (info[t] >> m) & 1u ? T(0) : fma(-w[t][m], alpha, r[t][m]), z = rv * mi[t][m];
         r[t][m] = rv;
@@ -439,7 +472,7 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
     if (q >= NO) continue;
     const long long n = node(a + q / PN, q % PN);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
+    for (int m = 0; m < NC; ++m) {
       A.u[n + m * g.n] = (IO)u[t][m];
       if (A.ru) A.ru[n + m * g.n] = (IO)r[t][m];
     }
@@ -450,15 +483,16 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
 
 template <typename T, typename IO>
 using ClusterKernel = void (*)(const ClusterArgs<T, IO>);
-template <typename T, typename IO, bool ISO>
+template <typename T, typename IO, bool PF, bool ISO>
 ClusterKernel<T, IO> shape_kernel(int threads) {
-  if (threads == 128) return cluster_pcg_kernel<T, IO, ISO, 128, 1>;
-  if (threads == 256) return cluster_pcg_kernel<T, IO, ISO, 256, 2>;
-  return cluster_pcg_kernel<T, IO, ISO, 512, 2>;
+  if (threads == 128) return cluster_pcg_kernel<T, IO, PF, ISO, 128, 1>;
+  if (threads == 256) return cluster_pcg_kernel<T, IO, PF, ISO, 256, 2>;
+  return cluster_pcg_kernel<T, IO, PF, ISO, 512, 2>;
 }
 
-template <typename T, typename IO>
-int launch_cluster(hpc_ctx* c, const ClusterArgs<T, IO>& a) {
+template <bool PF, typename T, typename IO>
+int launch_cluster(hpc_ctx* c, ClusterArgs<T, IO>& a) {
+  if (!cluster_plan<T, PF>(a.g, &a.p)) return HPC_ERR_ARG;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(kBlocks);
   cfg.blockDim = dim3(a.p.threads);
@@ -471,16 +505,16 @@ int launch_cluster(hpc_ctx* c, const ClusterArgs<T, IO>& a) {
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   const bool iso = a.g.hx == a.g.hy && a.g.hy == a.g.hz;
-  HPC_CUDA(cudaLaunchKernelEx(&cfg, iso ? shape_kernel<T, IO, true>(a.p.threads) : shape_kernel<T, IO, false>(a.p.threads),
-                              a));
+  HPC_CUDA(cudaLaunchKernelEx(
+      &cfg, iso ? shape_kernel<T, IO, PF, true>(a.p.threads) : shape_kernel<T, IO, PF, false>(a.p.threads), a));
   HPC_CHECK_LAUNCH(c);
   return HPC_OK;
 }
 
-template <typename T, typename IO>
+template <typename T, typename IO, bool PF>
 int prepare() {
   for (const auto& sh : kShapes)
-    for (ClusterKernel<T, IO> k : {shape_kernel<T, IO, true>(sh[0]), shape_kernel<T, IO, false>(sh[0])}) {
+    for (ClusterKernel<T, IO> k : {shape_kernel<T, IO, PF, true>(sh[0]), shape_kernel<T, IO, PF, false>(sh[0])}) {
       HPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
       HPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     }
@@ -491,7 +525,7 @@ int prepare() {
 
 bool cluster_pcg_fits_geo(const LevelGeo& g) {
   ClusterPlan p;
-  return cluster_plan<double>(g, &p);
+  return cluster_plan<double, false>(g, &p);
 }
 bool cluster_pcg_fits(hpc_ctx* c, int level) {
   if (level == c->maxlevel) return false;  // the finest level's material is nodal, not element-constant
@@ -505,16 +539,17 @@ int cluster_pcg_prepare(int device) {
   std::lock_guard<std::mutex> lock(mu);
   if (device >= 0 && device < 64 && done[device]) return HPC_OK;
   int rc;
-  if ((rc = prepare<double, double>()) || (rc = prepare<double, float>()) || (rc = prepare<float, float>())) return rc;
+  if ((rc = prepare<double, double, false>()) || (rc = prepare<double, float, false>()) ||
+      (rc = prepare<float, float, false>()) || (rc = prepare<double, double, true>()))
+    return rc;
   if (device >= 0 && device < 64) done[device] = true;
   return HPC_OK;
 }
 
 int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
                           const double* Ke, const double* Ge, double Ut, int nb) {
-  ClusterArgs<double, double> a{g, {}, u, fu, ru, invM, Ke, Ge, Ut, nb, c->scal, S_RNORM, c->scal + S_ERR};
-  if (!cluster_plan<double>(g, &a.p)) return HPC_ERR_ARG;
-  return launch_cluster(c, a);
+  ClusterArgs<double, double> a{g, {}, u, fu, ru, invM, Ke, Ge, Ut, nb, c->scal, S_RNORM, -1, c->scal + S_ERR};
+  return launch_cluster<false>(c, a);
 }
 
 int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb) {
@@ -524,17 +559,28 @@ int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb) {
 
 int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb) {
   const LevelF32& F = c->F32[level];
-  ClusterArgs<float, float> a{c->L[level], {}, F.u, F.fu, F.ru, F.invM, F.Ke, F.Ge, 0.f, nb, c->scal, -1, c->scal + S_ERR};
-  if (!cluster_plan<float>(a.g, &a.p)) return HPC_ERR_ARG;
-  return launch_cluster(c, a);
+  ClusterArgs<float, float> a{c->L[level], {}, F.u, F.fu, F.ru, F.invM, F.Ke, F.Ge, 0.f, nb, c->scal, -1, -1, c->scal + S_ERR};
+  return launch_cluster<false>(c, a);
 }
 
 int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb) {
   const LevelFields& F = c->F[level];
   const LevelF32& G = c->F32[level];
-  ClusterArgs<double, float> a{c->L[level], {}, G.u, G.fu, nullptr, F.preMu, F.Ke, F.Ge, 0.0, nb, c->scal, S_RNORM, c->scal + S_ERR};
-  if (!cluster_plan<double>(a.g, &a.p)) return HPC_ERR_ARG;
-  return launch_cluster(c, a);
+  ClusterArgs<double, float> a{c->L[level], {}, G.u, G.fu, nullptr, F.preMu, F.Ke, F.Ge, 0.0, nb, c->scal, S_RNORM, -1, c->scal + S_ERR};
+  return launch_cluster<false>(c, a);
+}
+
+bool cluster_pcg_d_fits(hpc_ctx* c, int level) {
+  ClusterPlan p;
+  return cluster_plan<double, true>(c->L[level], &p);
+}
+
+// pcg_d (phase_field_pcg.cpp:133-214) of a small level.
+int launch_cluster_pcg_d(hpc_ctx* c, int level, double lc, int nb) {
+  const LevelFields& F = c->F[level];
+  ClusterArgs<double, double> a{c->L[level], {}, F.d, F.fd, F.R, F.preMd, F.gc, F.H, lc, nb, c->scal, S_RNORM, S_FDNORM,
+                                c->scal + S_ERR};
+  return launch_cluster<true>(c, a);
 }
 
 }  // namespace hpc

@@ -113,6 +113,10 @@ int num_sms();
 // {px, ny, nz, ncomp}, x fastest, with the given box.
 template <typename T>
 int encode_tensor(const LevelGeo& g, const T* src, int ncomp, int bx, int by, int bz, CUtensorMap* map);
+constexpr int kTileX = 16;  // element columns of a tile in x
+// Tiles of a level, `ty` element rows high, and their z chunks (tz) for `slots` resident blocks; at most cap
+// blocks where one chunk allows it.
+StripGeo tile_geo(const LevelGeo& g, int ty, long long slots, long long cap);
 // Tile kernels (mech_tile.cu): the mechanical operator with precomputed Gauss-point moduli (finest level,
 // k.gpm set) or element-constant moduli (coarse levels).
 template <typename T>

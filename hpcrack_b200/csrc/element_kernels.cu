@@ -1083,30 +1083,24 @@ int launch_gp_material(hpc_ctx* c, double small_k) {
 // phase field
 // ------------------------------------------------------------------------------------------
 struct PfK {
-  LevelGeo g, gf;
+  LevelGeo g;
   StripGeo sg;
-  const double* fields[3];  // staged: x, gc, H (H is element data, read on the lower plane)
+  const double* fields[2];  // staged: gc, H (H is element data, read on the lower plane)
   double* out;
   double lc;
-  const double* fd;
-  const double* invM;
-  const double* rf;
-  RedTarget red;
 };
 
-template <int EPI, bool DIAG, bool ISO>
-__global__ void __launch_bounds__(kWarps * 32) pf_kernel(PfK k) {
-  constexpr int NF = 3;
+// diag A_d on the strips (the applies are in pf_tile.cu).
+__global__ void __launch_bounds__(kWarps * 32) pf_diag_kernel(PfK k) {
+  constexpr int NF = 2;
   extern __shared__ double smem[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   double* ring = smem + (size_t)wib * (kRing * NF * 2 * kRowW + (k.sg.wy - 1) * 32);
   double* zc = ring + kRing * NF * 2 * kRowW;  // [row][lane]
   const SF s = make_sf(k.g);
-  double red0 = 0.0, red1 = 0.0, red2 = 0.0;
   const long long nwarps_total = (long long)gridDim.x * kWarps;
-  // ISO: only the gradient term carries 1/h^2 (see sf_forward); the mass term keeps wg
-  const double wg = k.g.wg, wgb = ISO ? k.g.wg * (s.ih[0] * s.ih[0]) : k.g.wg, inv_lc = 1.0 / k.lc;
-  const double* fptr[NF] = {k.fields[0], k.fields[1], k.fields[2]};
+  const double wg = k.g.wg, inv_lc = 1.0 / k.lc;
+  const double* fptr[NF] = {k.fields[0], k.fields[1]};
 
   for (long long strip = (long long)blockIdx.x * kWarps + wib; strip < k.sg.nstrips; strip += nwarps_total) {
     const int sx = (int)(strip % k.sg.tx);
@@ -1124,8 +1118,7 @@ __global__ void __launch_bounds__(kWarps * 32) pf_kernel(PfK k) {
     double yp[2] = {0.0, 0.0};
     for (int si = 0; si < st.total; ++si) {
       st.issue(si + 2, lane);
-      cp_async_wait2();
-      __syncwarp();
+      st.wait();
       const int li = si / rows, r = si - li * rows;
       const int kk = z0 - 1 + li;
       if (r == 0) {
@@ -1142,26 +1135,16 @@ __global__ void __launch_bounds__(kWarps * 32) pf_kernel(PfK k) {
 #pragma unroll
         for (int n = 0; n < 8; ++n) {
           const int a = n & 1, b = (n >> 1) & 1, c = n >> 2;
-          gcn[n] = st.at(b ? si : si - 1, 1, c, lane + a);
+          gcn[n] = st.at(b ? si : si - 1, 0, c, lane + a);
         }
         gp_material(gcn, s, gcg);
-        const double H2 = 2.0 * st.at(si - 1, 2, 0, lane);
+        const double H2 = 2.0 * st.at(si - 1, 1, 0, lane);
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
           aw[g] = wg * fma(gcg[g], inv_lc, H2);
-          bw[g] = wgb * (gcg[g] * k.lc);
+          bw[g] = wg * (gcg[g] * k.lc);
         }
-        if (DIAG) {
-          pf_element_diag(aw, bw, s, f);
-        } else {
-          double xv[8];
-#pragma unroll
-          for (int n = 0; n < 8; ++n) {
-            const int a = n & 1, b = (n >> 1) & 1, c = n >> 2;
-            xv[n] = st.at(b ? si : si - 1, 0, c, lane + a);
-          }
-          pf_element<ISO>(xv, aw, bw, s, f);
-        }
+        pf_element_diag(aw, bw, s, f);
       } else {
 #pragma unroll
         for (int n = 0; n < 8; ++n) f[n] = 0.0;
@@ -1178,87 +1161,25 @@ __global__ void __launch_bounds__(kWarps * 32) pf_kernel(PfK k) {
         double* zp = zc + (rr - 1) * 32 + lane;
         const double tot = *zp + yp[0] + X[0][0];
         *zp = yp[1] + X[0][1];
-        if (kk >= z0 && lane >= 1 && lane <= 30 && x < k.g.nx && ey < k.g.ny) {
-          const long long n = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
-          if (EPI == EPI_PLAIN) {
-            k.out[n] = tot;
-          } else if (EPI == EPI_RESIDUAL) {
-            const double fv = k.fd[n];
-            const double rv = fv - tot;
-            k.out[n] = rv;
-            const bool own = owned_plane(k.g, kk);
-            const double s0 = fma(fv, fv, red0), s1 = fma(rv, rv, red1);
-            red0 = own ? s0 : red0;
-            red1 = own ? s1 : red1;
-            if (k.invM) {
-              const double s2 = fma(rv, rv * k.invM[n], red2);
-              red2 = own ? s2 : red2;
-            }
-          } else if (EPI == EPI_PCG) {
-            k.out[n] = tot;
-            const double s0 = fma(st.at(si - 1, 0, 0, lane), tot, red0);
-            red0 = owned_plane(k.g, kk) ? s0 : red0;
-          } else if (EPI == EPI_FAS) {
-            const int fz = 2 * kk + k.g.zsh;
-            k.out[n] = tot + (fz >= 0 ? full_weight(k.gf, k.rf, 2 * x, 2 * ey, fz) : 0.0);
-          }
-        }
+        if (kk >= z0 && lane >= 1 && lane <= 30 && x < k.g.nx && ey < k.g.ny)
+          k.out[(long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane] = tot;
       }
       yp[0] = X[1][0];
       yp[1] = X[1][1];
       __syncwarp();
     }
   }
-  if (EPI == EPI_RESIDUAL || EPI == EPI_PCG) {
-    double v[3] = {red0, red1, red2};
-    grid_reduce<3>(v, k.red);
-  }
-}
-
-template <int E, bool D>
-static int run_pf(hpc_ctx* c, const PfK& k, bool finest) {
-  const SmemPlan smem{0, (size_t)kRing * 3 * 2 * kRowW, 32, sizeof(double)};
-  const int cls = (finest && E == EPI_PCG && !D) ? HPC_KC_PF_PCG_FINEST : HPC_KC_NONE;
-  if constexpr (!D) {
-    if (iso(k.g)) return launch_strips(c, pf_kernel<E, D, true>, k, smem, cls);
-  }
-  return launch_strips(c, pf_kernel<E, D, false>, k, smem, cls);
-}
-
-int launch_pf(hpc_ctx* c, const PfCall& p) {
-  if (p.epi == EPI_FAS) HPC_SLAB_HALO(c, p.fine_level, p.rf, 1, sizeof(double));  // SendRecv(rf), :356
-  PfK k{};
-  k.g = c->L[p.level];
-  if (p.epi == EPI_FAS) k.gf = c->L[p.fine_level];
-  k.fields[0] = p.src;
-  k.fields[1] = c->F[p.level].gc;
-  k.fields[2] = c->F[p.level].H;
-  k.out = p.out;
-  k.lc = p.lc;
-  k.fd = p.fd;
-  k.invM = p.invM;
-  k.rf = p.rf;
-  k.red = make_red(c, p.s_out0, p.s_out1, p.s_out2);
-  const bool fin = p.level == c->maxlevel;
-  switch (p.epi) {
-    case EPI_PLAIN: return run_pf<EPI_PLAIN, false>(c, k, fin);
-    case EPI_RESIDUAL: return run_pf<EPI_RESIDUAL, false>(c, k, fin);
-    case EPI_PCG: return run_pf<EPI_PCG, false>(c, k, fin);
-    case EPI_FAS: return run_pf<EPI_FAS, false>(c, k, fin);
-  }
-  return HPC_ERR_ARG;
 }
 
 int launch_pf_diag(hpc_ctx* c, int level, double lc, double* out) {
   PfK k{};
   k.g = c->L[level];
-  k.fields[0] = c->F[level].d;
-  k.fields[1] = c->F[level].gc;
-  k.fields[2] = c->F[level].H;
+  k.fields[0] = c->F[level].gc;
+  k.fields[1] = c->F[level].H;
   k.out = out;
   k.lc = lc;
-  k.red = make_red(c, -1, -1, -1);
-  return run_pf<EPI_PLAIN, true>(c, k, false);
+  const SmemPlan smem{0, (size_t)kRing * 2 * 2 * kRowW, 32, sizeof(double)};
+  return launch_strips(c, pf_diag_kernel, k, smem, HPC_KC_NONE);
 }
 
 }  // namespace hpc

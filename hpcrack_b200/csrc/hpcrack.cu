@@ -321,6 +321,7 @@ static int pcg_u_dev(hpc_ctx* c, int l, double small_k, double Ut, int nb, int t
 // pcg_d (phase_field_pcg.cpp:133-214) with preMd built; fd_norm rewritten (S_FDNORM).
 static int pcg_d_dev(hpc_ctx* c, int l, double lc, int nb) {
   if (nb > kMaxRelax) return arg_fail("nb_relax too large");
+  if (c->fused_coarsest && slab_coarsest_mode(c) == 0 && cluster_pcg_d_fits(c, l)) return launch_cluster_pcg_d(c, l, lc, nb);
   LevelFields& F = c->F[l];
   int rc;
   PfCall m{};
@@ -1586,7 +1587,7 @@ int hpc_pcg_d(hpc_ctx* c, int level, double lc, int nb_relax, int t, double* fd_
   if (nb_relax > 0 && (rc = check_zero_diags(c, 0, "Precondition_M"))) return rc;
   if ((rc = launch_invert(c, level, 1, c->F[level].preMd))) return rc;
   if ((rc = pcg_d_dev(c, level, lc, nb_relax))) return rc;
-  return read_scalars(c, S_FDNORM, 1, fd_norm);
+  return read_result(c, S_FDNORM, fd_norm);
 }
 
 int hpc_cycle_u(hpc_ctx* c, int level, const hpc_mg* mg, double small_k, double Ut, int t, double* f_norm) {
@@ -1607,7 +1608,7 @@ int hpc_cycle_d(hpc_ctx* c, int level, const hpc_mg* mg, double lc, int t, doubl
   if ((rc = pf_diags(c, level, lc))) return rc;
   long long it = 0;
   if ((rc = cycle_d_dev(c, level, *mg, lc, &it))) return rc;
-  return read_scalars(c, S_FDNORM, 1, fd_norm);
+  return read_result(c, S_FDNORM, fd_norm);
 }
 
 int hpc_u_entire(hpc_ctx* c, const hpc_mg* mg, double small_k, double Ut, int t, double* f_norm, double mech_tol,
@@ -1648,7 +1649,7 @@ int hpc_phase_field(hpc_ctx* c, const hpc_mg* mg, double lc, int t, double* fd_n
   int cy = 0;
   long long it = 0;
   int rc = phase_field_dev(c, *mg, lc, pf_tol, &cy, &it);
-  if (rc) return rc;
+  if (rc || (rc = check_wait_error(c))) return rc;
   *fd_norm = c->fd_norm;
   if (cycles) *cycles = cy;
   if (iters) *iters = (int)it;

@@ -365,6 +365,9 @@ int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double
                           const double* Ke, const double* Ge, double Ut, int nb);
 int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb);
 int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb);
+// The same for pcg_d, any level that fits.
+bool cluster_pcg_d_fits(hpc_ctx* c, int level);
+int launch_cluster_pcg_d(hpc_ctx* c, int level, double lc, int nb);
 int tuned_shapes(int* out5, int cap);  // measured strip shapes: {nx, ny, nz, wy, cz} per entry
 
 

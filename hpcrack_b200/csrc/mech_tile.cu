@@ -30,9 +30,33 @@
 #include "element_common.cuh"
 
 namespace hpc {
+
+// Tiles of a level and the z chunks they are marched in: a chunk of cz planes costs its block cz + 1 layers
+// and a pipeline start of about two layers' time, and blocks run in waves of `slots`; the number of
+// chunks that minimises waves x (cz + 3) wins.
+StripGeo tile_geo(const LevelGeo& g, int ty, long long slots, long long cap) {
+  StripGeo s;
+  s.wy = ty;
+  s.tx = (g.nx + kTileX - 2) / (kTileX - 1);
+  s.ty = (g.ny + ty - 2) / (ty - 1);
+  const long long tiles = (long long)s.tx * s.ty;
+  long long best = -1;
+  for (int n = 1; n <= g.nz && (n == 1 || tiles * n <= cap); ++n) {
+    const int cz = (g.nz + n - 1) / n;
+    const long long cost = ((tiles * n + slots - 1) / slots) * (cz + 3);
+    if (best < 0 || cost < best) {
+      best = cost;
+      s.cz = cz;
+      s.tz = n;
+    }
+  }
+  s.nstrips = tiles * s.tz;
+  return s;
+}
+
 namespace {
 
-constexpr int kTX = 16;  // element columns of a tile in x: a half-warp, 128 B (64 B) of FP64 (FP32) per row
+constexpr int kTX = kTileX;  // element columns of a tile in x: a half-warp, 128 B (64 B) of FP64 (FP32) per row
 constexpr unsigned kTileWaitPolls = 1u << 24;  // far above any copy's latency; then the kernel reports
 
 // Columns staged per row: the 17 nodes of a tile plus the offset to the copy's 16-byte aligned start.
@@ -380,29 +404,6 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
 template <typename T> struct TileShape;
 template <> struct TileShape<double> { static constexpr int TY = 8, MINB = 2, NS = 3; };
 template <> struct TileShape<float> { static constexpr int TY = 16, MINB = 1, NS = 3; };
-
-// Tiles of a level and the z chunks they are marched in: a chunk of cz planes costs its block cz + 1 layers
-// and a pipeline start of about two layers' time, and blocks run in waves of `slots`; the number of
-// chunks that minimises waves x (cz + 3) wins.
-StripGeo tile_geo(const LevelGeo& g, int ty, long long slots, long long cap) {
-  StripGeo s;
-  s.wy = ty;
-  s.tx = (g.nx + kTX - 2) / (kTX - 1);
-  s.ty = (g.ny + ty - 2) / (ty - 1);
-  const long long tiles = (long long)s.tx * s.ty;
-  long long best = -1;
-  for (int n = 1; n <= g.nz && (n == 1 || tiles * n <= cap); ++n) {
-    const int cz = (g.nz + n - 1) / n;
-    const long long cost = ((tiles * n + slots - 1) / slots) * (cz + 3);
-    if (best < 0 || cost < best) {
-      best = cost;
-      s.cz = cz;
-      s.tz = n;
-    }
-  }
-  s.nstrips = tiles * s.tz;
-  return s;
-}
 
 template <typename T, bool GPM, int EPI, bool ISO, bool TMA>
 int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {

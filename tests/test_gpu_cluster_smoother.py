@@ -1,4 +1,4 @@
-"""The one-cluster smoother of small coarse levels against the C oracle's pcg_u (GPU).
+"""The one-cluster smoothers of small levels against the C oracle's pcg_u and pcg_d (GPU).
 
 Levels cut along each axis, with fewer planes than blocks, one and several planes a block, a block whose
 share is larger than its neighbours', each block shape (1 to 1024 elements a block), and a spacing that
@@ -10,7 +10,7 @@ import pytest
 
 from oracle.bindings import COracle
 from hpcrack_b200.solver import Hierarchy, RU, U
-from cases import load_random, rel
+from cases import D, R, load_random, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -35,6 +35,12 @@ def test_cluster_smoother(enb, roi):
         for impl in (gpu, orc):
             impl.pcg_u(0, 1e-5, Ut, nb, 1, 1.0)
         for f in (U, RU):
+            assert rel(gpu.get(f, 0), orc.get(f, 0)) < 1e-10, (nb, f)
+        for impl in (gpu, orc):
+            impl.fd_h(0)
+        fd = [impl.pcg_d(0, 2.0, nb, 1, 1.0)[1] for impl in (gpu, orc)]
+        assert abs(fd[0] - fd[1]) <= 1e-12 * fd[1]
+        for f in (D, R):
             assert rel(gpu.get(f, 0), orc.get(f, 0)) < 1e-10, (nb, f)
     gpu.close()
     orc.close()

@@ -1,6 +1,6 @@
-"""The tile kernels of the mechanical operator against the C oracle (GPU) where tiles end.
+"""The tile kernels of the mechanical and phase-field operators against the C oracle (GPU) where tiles end.
 
-A tile finishes 15 node columns in x and 7 (FP64) or 15 (FP32) in y: levels whose extents are a tile,
+A tile finishes 15 node columns in x and 7 (mechanical FP64) or 15 in y: levels whose extents are a tile,
 one node less and one node more, levels smaller than a tile, and a spacing that differs per axis.
 Coarse levels run through Internal_Force (element-constant moduli); the finest level's kernel on
 precomputed Gauss-point moduli runs inside a mechanical solve, here one V-cycle of u_entire with its
@@ -12,7 +12,7 @@ import pytest
 
 from oracle.bindings import COracle
 from hpcrack_b200.solver import Hierarchy
-from cases import FU, RU, U, load_random, rel
+from cases import D, FD, FU, R, RU, U, load_random, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -38,6 +38,16 @@ def test_tile_apply(geom, tma):
         for impl in (gpu, orc):
             impl.internal_force(l, U, RU, 1e-5)
         assert rel(gpu.get(RU, l), orc.get(RU, l)) < 1e-12, l
+    for l in range(ml + 1):
+        for impl in (gpu, orc):
+            impl.fld(l, D, R, 2.0)
+        assert rel(gpu.get(R, l), orc.get(R, l)) < 1e-12, l
+        for impl in (gpu, orc):
+            impl.fd_h(l)
+    for impl in (gpu, orc):
+        impl.phase_field((3, 2, 1, 1, 1), 2.0, 1, 1.0, pf_tol=1e-30)
+    for f in (D, R, FD):
+        assert rel(gpu.get(f, ml), orc.get(f, ml)) < 1e-10, f
     for t in (0, 1):
         for impl in (gpu, orc):
             impl.u_entire((3, 2, 1, 1, 1), 1e-5, 1.0, t, 1.0, mech_tol=1e-30)
