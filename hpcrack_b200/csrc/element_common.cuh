@@ -33,6 +33,13 @@ struct MechKT {
   const T* gpm;  // finest level, precomputed Gauss-point moduli: K - 2G/3 at [g * n + e], G at [(8 + g) * n + e]
   RedTarget red;
   double* err;   // tensor-core kernel / TMA staging: set to 1 when a bounded wait ran out
+  // PCG direction formed while the planes are staged (mech_tile.cu): p = r M^-1 + beta p_old, beta =
+  // red.scal[s_rz] / red.scal[s_rz_prev] (p = r M^-1 if dir_first), written to p_new; fields[0..2] hold p_old
+  const T* dir_r;
+  const T* dir_m;
+  T* p_new;
+  int dir_first, s_rz, s_rz_prev;
+  alignas(64) CUtensorMap rmap, mmap;  // dir_r, dir_m as {px, ny, nz, 3}
   alignas(64) CUtensorMap tmap;  // TMA staging: the staged vector as {px, ny, nz, 3}
   alignas(64) CUtensorMap gmap;  // TMA staging: the Gauss-point moduli as {px, ny, nz, 16} (finest applies)
 };
@@ -120,6 +127,6 @@ StripGeo tile_geo(const LevelGeo& g, int ty, long long slots, long long cap);
 // Tile kernels (mech_tile.cu): the mechanical operator with precomputed Gauss-point moduli (finest level,
 // k.gpm set) or element-constant moduli (coarse levels).
 template <typename T>
-int launch_mech_tile(hpc_ctx* c, MechKT<T>& k, bool finest, int epi);
+int launch_mech_tile(hpc_ctx* c, MechKT<T>& k, bool finest, int epi);  // EPI_PCG with k.p_new: fused direction
 
 }  // namespace hpc

@@ -962,6 +962,12 @@ int launch_mech(hpc_ctx* c, const MechCall& m) {
   k.gpm = (m.finest && c->gpm_active) ? c->F[m.level].gpm : nullptr;
   k.red = make_red(c, m.s_out0, m.s_out1, m.s_out2);
   k.err = c->scal + S_ERR;
+  k.dir_r = m.dir_r;
+  k.dir_m = m.invM;
+  k.p_new = m.p_new;
+  k.dir_first = m.dir_first;
+  k.s_rz = m.s_rz;
+  k.s_rz_prev = m.s_rz_prev;
   if (!m.finest || k.gpm) return launch_mech_tile(c, k, m.finest, m.epi);
   switch (m.epi) {
     case EPI_PLAIN: return run_mech<true, EPI_PLAIN, false>(c, k);
@@ -1034,6 +1040,12 @@ int launch_mech_f32(hpc_ctx* c, const MechCall32& m) {
     }
   }
   if (fin && !k.gpm) return HPC_ERR_ARG;  // the V-cycle runs on precomputed moduli
+  k.dir_r = m.dir_r;
+  k.dir_m = m.invM;
+  k.p_new = m.p_new;
+  k.dir_first = m.dir_first;
+  k.s_rz = m.s_rz;
+  k.s_rz_prev = m.s_rz_prev;
   return launch_mech_tile(c, k, fin, m.epi);
 }
 

@@ -156,7 +156,7 @@ static bool geometry_ok(const hpc_geometry* g, int nr = 1, int r = 0) {
 // Number of doubles per level allocated for a level with n padded slots.
 constexpr int kScalarFieldsPerLevel = 10;  // bulK G gc d H fd Ke Ge R dold
 constexpr int kVectorFieldsPerLevel = 4;   // u fu ru uold
-constexpr int kWork3 = 4, kWork1 = 4;      // preMu p w tmp3 / preMd pd wd tmp1
+constexpr int kWork3 = 4, kWork1 = 4;      // preMu p w p2 / preMd pd wd tmp1
 static size_t level_bytes(long long n) {
   return (size_t)n * sizeof(double) * (kScalarFieldsPerLevel + 3 * kVectorFieldsPerLevel + 3 * kWork3 + kWork1) +
          (size_t)n;  // choice
@@ -301,19 +301,31 @@ static int pcg_u_dev(hpc_ctx* c, int l, double small_k, double Ut, int nb, int t
   m.s_out1 = slot_rz(0);
   m.s_out2 = S_RNORM;
   if ((rc = launch_mech(c, m))) return rc;
+  const bool fuse = can_fuse_dir(c, m.finest);  // the apply forms the direction: p and p2 in turn
   for (int it = 0; it < nb; ++it) {
-    if ((rc = launch_dir_update(c, l, 3, F.ru, F.preMu, F.p, it == 0, slot_rz(it), slot_rz(it - 1)))) return rc;
+    double* p = fuse && (it & 1) ? F.p2 : F.p;
     MechCall q{};
     q.level = l;
     q.finest = m.finest;
     q.epi = EPI_PCG;
-    q.src = F.p;
     q.out = F.w;
     q.small_k = small_k;
     q.s_out0 = slot_pw(it);
     q.s_out1 = q.s_out2 = -1;
+    if (fuse) {
+      q.src = (it & 1) ? F.p : F.p2;
+      q.dir_r = F.ru;
+      q.invM = F.preMu;
+      q.p_new = p;
+      q.dir_first = it == 0;
+      q.s_rz = slot_rz(it);
+      q.s_rz_prev = slot_rz(it - 1);
+    } else {
+      q.src = p;
+      if ((rc = launch_dir_update(c, l, 3, F.ru, F.preMu, p, it == 0, slot_rz(it), slot_rz(it - 1)))) return rc;
+    }
     if ((rc = launch_mech(c, q))) return rc;
-    if ((rc = launch_mech_update(c, l, F.p, slot_rz(it), slot_pw(it), slot_rz(it + 1), slot_rn(it)))) return rc;
+    if ((rc = launch_mech_update(c, l, p, slot_rz(it), slot_pw(it), slot_rz(it + 1), slot_rn(it)))) return rc;
   }
   return HPC_OK;
 }
@@ -695,19 +707,32 @@ static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, bool u_zero = fals
     m.s_out2 = -1;
     if ((rc = launch_mech_f32(c, m))) return rc;
   }
+  const bool fuse = !c->tc_apply && can_fuse_dir(c, m.finest);
+  float* p2 = reinterpret_cast<float*>(c->F[l].p2);
   for (int it = 0; it < nb; ++it) {
-    if ((rc = launch_dir_update_f32(c, l, it == 0, slot_rz(it), slot_rz(it - 1)))) return rc;
+    float* p = fuse && (it & 1) ? p2 : F.p;
     MechCall32 q{};
     q.level = l;
     q.finest = m.finest;
     q.epi = EPI_PCG;
-    q.src = F.p;
     q.out = F.w;
     q.small_k = small_k;
     q.s_out0 = slot_pw(it);
     q.s_out1 = q.s_out2 = -1;
+    if (fuse) {
+      q.src = (it & 1) ? F.p : p2;
+      q.dir_r = F.ru;
+      q.invM = F.invM;
+      q.p_new = p;
+      q.dir_first = it == 0;
+      q.s_rz = slot_rz(it);
+      q.s_rz_prev = slot_rz(it - 1);
+    } else {
+      q.src = p;
+      if ((rc = launch_dir_update_f32(c, l, it == 0, slot_rz(it), slot_rz(it - 1)))) return rc;
+    }
     if ((rc = launch_mech_f32(c, q))) return rc;
-    if ((rc = launch_mech_update_f32(c, l, slot_rz(it), slot_pw(it), slot_rz(it + 1), slot_rn(it)))) return rc;
+    if ((rc = launch_mech_update_f32(c, l, p, slot_rz(it), slot_pw(it), slot_rz(it + 1), slot_rn(it)))) return rc;
   }
   return HPC_OK;
 }
@@ -1136,7 +1161,7 @@ static int create_ctx(hpc_ctx** out, const hpc_geometry* geo, int device, int nr
     const long long n = c->L[l].n;
     LevelFields& F = c->F[l];
     double** scal[] = {&F.bulK, &F.G, &F.gc, &F.d, &F.H, &F.fd, &F.Ke, &F.Ge, &F.R, &F.dold, &F.preMd, &F.pd, &F.wd, &F.tmp1};
-    double** vec[] = {&F.u, &F.fu, &F.ru, &F.uold, &F.preMu, &F.p, &F.w, &F.tmp3};
+    double** vec[] = {&F.u, &F.fu, &F.ru, &F.uold, &F.preMu, &F.p, &F.w, &F.p2};
     for (double** p : scal) {
       cudaError_t ae = ctx_alloc(c, (void**)p, sizeof(double) * n);
       if (ae != cudaSuccess) return fail(cuda_fail(ae, "cudaMallocAsync(level field)"));
@@ -1201,7 +1226,7 @@ int hpc_destroy(hpc_ctx* c) {
   for (int l = 0; l <= c->maxlevel && l < kMaxLevels; ++l) {
     LevelFields& F = c->F[l];
     void* ptrs[] = {F.bulK, F.G, F.gc, F.d, F.H, F.fd, F.Ke, F.Ge, F.R, F.dold, F.preMd, F.pd, F.wd, F.tmp1,
-                    F.u, F.fu, F.ru, F.uold, F.preMu, F.p, F.w, F.tmp3, F.choice, F.gpm};
+                    F.u, F.fu, F.ru, F.uold, F.preMu, F.p, F.w, F.p2, F.choice, F.gpm};
     for (void* p : ptrs) ctx_free(c, p);
   }
   ctx_free(c, c->d_old);

@@ -43,7 +43,8 @@ struct LevelFields {
   double *u, *fu, *ru, *uold;  // 3n each; component c at +c*n
   int8_t* choice;
   // work arrays
-  double *preMu, *p, *w, *tmp3;  // 3n; preMu holds the inverse diagonal while a solve runs
+  double *preMu, *p, *w, *p2;  // 3n; preMu holds the inverse diagonal while a solve runs; p2: with p, the two
+                               // PCG directions of a smoother (the FP32 cycle's use its bytes as floats)
   double *preMd, *pd, *wd, *tmp1;  // n;  preMd likewise
   uint8_t* bc_host_copy;           // host copies of the axis flags (nx+ny+nz bytes)
   double* gpm;  // finest level: Gauss-point moduli of the running mechanical solve, 16n (first use)
@@ -250,7 +251,16 @@ struct MechCall {
   int fine_level;
   // reduction destinations (scalar slots, -1 = none)
   int s_out0, s_out1, s_out2;
+  // PCG with the direction formed on the way (can_fuse_dir): p = dir_r M^-1 + beta src (beta from the slots, no
+  // src if dir_first), written to p_new, w = K p; M^-1 is invM
+  const double* dir_r;
+  double* p_new;
+  bool dir_first;
+  int s_rz, s_rz_prev;
 };
+// The tile kernels form the direction: not on a slab (its ghost planes of p come from the neighbours), nor
+// where the finest level runs on nodal moduli.
+inline bool can_fuse_dir(const hpc_ctx* c, bool finest) { return !c->slab && (!finest || c->gpm_active); }
 int launch_mech(hpc_ctx* c, const MechCall& m);
 int launch_mech_diag(hpc_ctx* c, int level, bool finest, double small_k, double* out);
 // Gauss-point moduli of the finest level into F[maxlevel].gpm (from bulK, G, d and the regimes)
@@ -270,10 +280,14 @@ struct MechCall32 {
   const float* rf;    // FAS: fine residual
   int fine_level;
   int s_out0, s_out1, s_out2;
+  const float* dir_r;  // PCG with the direction formed on the way, as in MechCall
+  float* p_new;
+  bool dir_first;
+  int s_rz, s_rz_prev;
 };
 int launch_mech_f32(hpc_ctx* c, const MechCall32& m);
 // FP32 mirror: u += alpha p, r -= alpha w on F32[level] (Dirichlet rows zero), alpha = scal[s_num]/scal[s_den]
-int launch_mech_update_f32(hpc_ctx* c, int level, int s_num, int s_den, int s_rz_next, int s_rn);
+int launch_mech_update_f32(hpc_ctx* c, int level, const float* p, int s_num, int s_den, int s_rz_next, int s_rn);
 // FP32 mirror: p = r M^-1 + beta p (beta from scal, 0 if first)
 int launch_dir_update_f32(hpc_ctx* c, int level, bool first, int s_rz, int s_rz_prev);
 int launch_bc_zero_f32(hpc_ctx* c, int level, float* v);  // zero the Dirichlet rows of a 3n vector

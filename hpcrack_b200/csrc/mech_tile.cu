@@ -17,6 +17,13 @@
 // thread, completion on the stage's mbarrier, or per-thread cp.async); the carried parts stay in
 // registers, two layers per loop turn so that they swap roles instead of being moved.
 //
+// The smoothers' applies form the PCG direction on the way (DIR): r, M^-1 and the old direction are staged
+// instead of the new one, each thread forms its share of a plane one layer before it is needed, and the
+// tile that owns a node writes the new direction (into the other of two arrays: neighbours still read the
+// old one).  That replaces a pass of 96 (48) bytes a node and its launch: an iteration's apply and
+// direction take 842 us on 257^3 in FP64 against 656 + 250, 532 us in FP32 against 401 + 125, and one
+// launch less where launches count; increments -1 to -5 %.
+//
 // What bounds it: FP64, the FP64 pipe (66 % of its cycles on 193^3; two warps per scheduler cannot hide
 // all dependent latencies); FP32, instruction issue (80 % of the slots).  Per launch on B200, with the
 // element-by-element strip kernel it replaced in brackets: 257^3 FP64 656 us (1043), FP32 401 us (759);
@@ -66,11 +73,12 @@ template <> struct TileRow<float> { static constexpr int BX = 20; };
 
 // Shared memory of a block: [0, 128) the stages' mbarriers; the stages' node planes and (finest) moduli
 // layers; the y exchange.
-template <typename T, bool GPM, int TY, int NS>
+// DIR: a stage also holds the planes of r and M^-1 the direction is formed from.
+template <typename T, bool GPM, int TY, int NS, bool DIR>
 struct TileSmem {
   static constexpr int BX = TileRow<T>::BX, NT = kTX * TY, XP = 20;  // XP: exchange row pitch (bank spread)
   static constexpr size_t up(size_t b) { return (b + 127) / 128 * 128; }
-  static constexpr size_t node = up(sizeof(T) * 3 * (TY + 1) * BX), mod = GPM ? up(sizeof(T) * 16 * TY * BX) : 0;
+  static constexpr size_t plane = up(sizeof(T) * 3 * (TY + 1) * BX), node = plane * (DIR ? 3 : 1), mod = GPM ? up(sizeof(T) * 16 * TY * BX) : 0;
   static constexpr size_t o_node = 128, o_mod = o_node + NS * node, o_exch = o_mod + NS * mod;
   static constexpr size_t total = o_exch + sizeof(T) * 2 * 3 * TY * XP;
   static constexpr size_t bytes = total + 128;  // + alignment of the dynamic base
@@ -118,9 +126,9 @@ __device__ __forceinline__ void plane_adjoint(const T (&ex)[2], const T (&dy)[2]
   f[2] = i1[0] + i1[1] - d1;
 }
 
-template <typename T, bool GPM, int EPI, bool ISO, bool TMA, int TY, int MINB, int NS>
+template <typename T, bool GPM, int EPI, bool ISO, bool TMA, int TY, int MINB, int NS, bool DIR>
 __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_constant__ MechKT<T> k) {
-  using S = TileSmem<T, GPM, TY, NS>;
+  using S = TileSmem<T, GPM, TY, NS, DIR>;
   constexpr int BX = S::BX, NT = S::NT, NY = TY + 1;
   extern __shared__ __align__(128) unsigned char tile_smem[];
   unsigned char* base = tile_smem + ((128u - (smem_u32(tile_smem) & 127u)) & 127u);
@@ -173,14 +181,22 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
         if (tid == 0) {
           const uint32_t bar = smem_u32(bars + (unsigned)j % NS);
           const bool mods = GPM && j >= 1;
-          const int bytes = (int)sizeof(T) * BX * (3 * NY + (mods ? 16 * TY : 0));
+          const bool old = !DIR || !k.dir_first;
+          const int bytes = (int)sizeof(T) * BX * (3 * NY * ((DIR ? 2 : 0) + (old ? 1 : 0)) + (mods ? 16 * TY : 0));
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-          asm volatile(
-              "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
-              "%4, %5}], [%6];" ::"r"(smem_u32(node_slot(j))),
-              "l"(&k.tmap), "r"(xs), "r"(y0 - 1), "r"(kk), "r"(0), "r"(bar)
-              : "memory");
+          auto copy = [&](const CUtensorMap* map, T* dst) {
+            asm volatile(
+                "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+                "%4, %5}], [%6];" ::"r"(smem_u32(dst)),
+                "l"(map), "r"(xs), "r"(y0 - 1), "r"(kk), "r"(0), "r"(bar)
+                : "memory");
+          };
+          if (old) copy(&k.tmap, node_slot(j));
+          if constexpr (DIR) {
+            copy(&k.rmap, node_slot(j) + S::plane / sizeof(T));
+            copy(&k.mmap, node_slot(j) + 2 * (S::plane / sizeof(T)));
+          }
           if (mods)
             asm volatile(
                 "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
@@ -190,16 +206,20 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
         }
       } else {
         // the nodes of a row one column apart, zeros outside the grid
-        T* dst = node_slot(j);
-        for (int q = tid; q < 3 * NY * 17; q += NT) {
-          const int c = q % 17, r = q / 17, ry = r % NY, m = r / NY;
-          const int gx = x0 - 1 + c, gy = y0 - 1 + ry;
-          const bool ok = gx >= 0 && gx < k.g.nx && gy >= 0 && gy < k.g.ny && kk >= 0 && kk < k.g.nz;
-          const T* src = k.fields[m] + (ok ? (long long)gx + (long long)gy * k.g.px + (long long)kk * k.g.plane : 0);
-          const unsigned d = smem_u32(dst + (m * NY + ry) * BX + off + c);
-          asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(sizeof(T)),
-                       "r"(ok ? (int)sizeof(T) : 0)
-                       : "memory");
+        for (int f = 0; f < (DIR ? 3 : 1); ++f) {
+          if (f == 0 && DIR && k.dir_first) continue;
+          T* dst = node_slot(j) + f * (S::plane / sizeof(T));
+          for (int q = tid; q < 3 * NY * 17; q += NT) {
+            const int c = q % 17, r = q / 17, ry = r % NY, m = r / NY;
+            const int gx = x0 - 1 + c, gy = y0 - 1 + ry;
+            const bool ok = gx >= 0 && gx < k.g.nx && gy >= 0 && gy < k.g.ny && kk >= 0 && kk < k.g.nz;
+            const T* src = f == 0 ? k.fields[m] : (f == 1 ? k.dir_r : k.dir_m) + m * k.g.n;
+            src += ok ? (long long)gx + (long long)gy * k.g.px + (long long)kk * k.g.plane : 0;
+            const unsigned d = smem_u32(dst + (m * NY + ry) * BX + off + c);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(sizeof(T)),
+                         "r"(ok ? (int)sizeof(T) : 0)
+                         : "memory");
+          }
         }
         if (GPM && j >= 1) {
           T* md = mod_slot(j) + row * BX + off + tx;
@@ -233,9 +253,29 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
       }
       return false;
     } else {
-      asm volatile("cp.async.wait_group %0;\n" ::"n"(NS - 1) : "memory");
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(DIR ? NS - 2 : NS - 1) : "memory");
       __syncthreads();
       return true;
+    }
+  };
+  // DIR: the direction at this thread's share of a staged plane's nodes, in place of p_old (0 beyond the
+  // grid's last column, where p_old's padding may hold anything)
+  constexpr int CN = 3 * NY * 17, CT = DIR ? (CN + NT - 1) / NT : 1;
+  int c_at[CT];
+  T beta = T(0);
+  auto form_direction = [&](int j) {
+    if constexpr (DIR) {
+      T* p = node_slot(j);
+      const T *r = p + S::plane / sizeof(T), *m = r + S::plane / sizeof(T);
+#pragma unroll
+      for (int t = 0; t < CT; ++t) {
+        if (c_at[t] < 0) continue;
+        const int o = c_at[t] & ~(1 << 30);
+        const T z = r[o] * m[o];
+        const T v = k.dir_first ? z : fma(beta, p[o], z);
+        p[o] = (c_at[t] & (1 << 30)) ? T(0) : v;
+      }
+      if (TMA) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next copy overwrites this plane
     }
   };
   // coarse levels: the element's moduli one layer ahead in registers
@@ -266,7 +306,7 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
         pre_m[m] = k.invM ? k.invM[n + m * k.g.n] : T(0);
       }
     }
-    if (!wait(li + 1)) bad = 1;
+    if (!DIR && !wait(li + 1)) bad = 1;
     // ---- upper node plane: in-plane parts; d/dz between the planes
     T gz[3][4];
     {
@@ -350,6 +390,10 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
       X0[m] = f[0] + __shfl_up_sync(kFull, f[1], 1, kTX);
       ex_w[m * TY * S::XP] = f[2] + __shfl_up_sync(kFull, f[3], 1, kTX);
     }
+    if (DIR && li + 2 <= nl) {  // the next layer's upper plane: the barrier publishes it
+      if (!wait(li + 2)) bad = 1;
+      form_direction(li + 2);
+    }
     bad = __syncthreads_or(bad);
     if (bad) return false;
     issue(li + 1 + NS);  // into the stage every thread has just read
@@ -358,15 +402,37 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
 #pragma unroll
       for (int m = 0; m < 3; ++m) tot[m] = X0[m] + ex_w[m * TY * S::XP - S::XP];
       node_epilogue<T, EPI>(k, x, y, kk, tot, a.own, pre_f, pre_m, red0, red1, red2);
+      if constexpr (DIR) {
+        const long long n = (long long)x + (long long)y * k.g.px + (long long)kk * k.g.plane;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) k.p_new[n + m * k.g.n] = a.own[m];
+      }
     }
     return true;
   };
 
 #pragma unroll
   for (int j = 0; j < NS; ++j) issue(j);
+  if constexpr (DIR) {  // under the first copies
+    if (!k.dir_first) beta = (T)(k.red.scal[k.s_rz] / k.red.scal[k.s_rz_prev]);
+#pragma unroll
+    for (int t = 0; t < CT; ++t) {
+      const int q = tid + t * NT;
+      c_at[t] = q < CN ? (q / 17) * BX + off + q % 17 : -1;
+      if (q < CN && x0 - 1 + q % 17 >= k.g.nx) c_at[t] |= 1 << 30;
+    }
+  }
   coarse_mod(z0 - 1);
   PlaneState<T> a, b;
-  if (!wait(0)) bad = 1;
+  if constexpr (DIR) {
+    if (TMA && !wait(0)) bad = 1;
+    if (!wait(1)) bad = 1;  // cp.async: planes 0 and 1
+    form_direction(0);
+    form_direction(1);
+    __syncthreads();
+  } else if (!wait(0)) {
+    bad = 1;
+  }
   {
     const T* nd = node_slot(0) + row * BX + off + tx;
 #pragma unroll
@@ -403,19 +469,22 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
 // FP64 7 % (703 against 656 us): a layer's arithmetic is too short to cover the copies.
 template <typename T> struct TileShape;
 template <> struct TileShape<double> { static constexpr int TY = 8, MINB = 2, NS = 3; };
-template <> struct TileShape<float> { static constexpr int TY = 16, MINB = 1, NS = 3; };
+template <> struct TileShape<float> { static constexpr int TY = 16, MINB = 2, NS = 3; };
 
-template <typename T, bool GPM, int EPI, bool ISO, bool TMA>
+template <typename T, bool GPM, int EPI, bool ISO, bool TMA, bool DIR>
 int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
   constexpr int TY = TileShape<T>::TY, NS = TileShape<T>::NS;
-  using S = TileSmem<T, GPM, TY, NS>;
-  auto kern = mech_tile_kernel<T, GPM, EPI, ISO, TMA, TY, TileShape<T>::MINB, NS>;
+  using S = TileSmem<T, GPM, TY, NS, DIR>;
+  auto kern = mech_tile_kernel<T, GPM, EPI, ISO, TMA, TY, TileShape<T>::MINB, NS, DIR>;
   int per_sm = 1, rc;
   if ((rc = kernel_cfg((const void*)kern, S::bytes, S::bytes, kTX * TY, &per_sm))) return rc;
   k.sg = tile_geo(k.g, TY, (long long)num_sms() * per_sm, (long long)c->partials_cap / 3);
   if ((size_t)k.sg.nstrips * 3 > c->partials_cap) return cuda_fail(cudaErrorInvalidValue, "partials buffer");
   if constexpr (TMA) {
     if ((rc = encode_tensor<T>(k.g, k.fields[0], 3, S::BX, TY + 1, 1, &k.tmap))) return rc;
+    if (DIR && ((rc = encode_tensor<T>(k.g, k.dir_r, 3, S::BX, TY + 1, 1, &k.rmap)) ||
+                (rc = encode_tensor<T>(k.g, k.dir_m, 3, S::BX, TY + 1, 1, &k.mmap))))
+      return rc;
     if (GPM && (rc = encode_tensor<T>(k.g, k.gpm, 16, S::BX, TY, 1, &k.gmap))) return rc;
   }
   timing_begin(c, cls);
@@ -425,11 +494,12 @@ int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
   return HPC_OK;
 }
 
-template <typename T, bool GPM, int EPI>
+template <typename T, bool GPM, int EPI, bool DIR = false>
 int run_tile_e(hpc_ctx* c, MechKT<T>& k, int cls) {
   const bool iso = k.g.hx == k.g.hy && k.g.hy == k.g.hz;
-  if (c->tma_stage) return iso ? run_tile<T, GPM, EPI, true, true>(c, k, cls) : run_tile<T, GPM, EPI, false, true>(c, k, cls);
-  return iso ? run_tile<T, GPM, EPI, true, false>(c, k, cls) : run_tile<T, GPM, EPI, false, false>(c, k, cls);
+  if (c->tma_stage)
+    return iso ? run_tile<T, GPM, EPI, true, true, DIR>(c, k, cls) : run_tile<T, GPM, EPI, false, true, DIR>(c, k, cls);
+  return iso ? run_tile<T, GPM, EPI, true, false, DIR>(c, k, cls) : run_tile<T, GPM, EPI, false, false, DIR>(c, k, cls);
 }
 
 }  // namespace
@@ -440,7 +510,7 @@ int launch_mech_tile(hpc_ctx* c, MechKT<T>& k, bool finest, int epi) {
   if (finest) {
     switch (epi) {
       case EPI_RESIDUAL: return run_tile_e<T, true, EPI_RESIDUAL>(c, k, HPC_KC_NONE);
-      case EPI_PCG: return run_tile_e<T, true, EPI_PCG>(c, k, pcg);
+      case EPI_PCG: return k.p_new ? run_tile_e<T, true, EPI_PCG, true>(c, k, pcg) : run_tile_e<T, true, EPI_PCG>(c, k, pcg);
       case EPI_REACTION:
         if constexpr (sizeof(T) == 8) return run_tile_e<T, true, EPI_REACTION>(c, k, HPC_KC_NONE);
         break;
@@ -450,7 +520,8 @@ int launch_mech_tile(hpc_ctx* c, MechKT<T>& k, bool finest, int epi) {
   }
   switch (epi) {
     case EPI_RESIDUAL: return run_tile_e<T, false, EPI_RESIDUAL>(c, k, HPC_KC_NONE);
-    case EPI_PCG: return run_tile_e<T, false, EPI_PCG>(c, k, HPC_KC_NONE);
+    case EPI_PCG:
+      return k.p_new ? run_tile_e<T, false, EPI_PCG, true>(c, k, HPC_KC_NONE) : run_tile_e<T, false, EPI_PCG>(c, k, HPC_KC_NONE);
     case EPI_FAS: return run_tile_e<T, false, EPI_FAS>(c, k, HPC_KC_NONE);
     case EPI_PLAIN: return run_tile_e<T, false, EPI_PLAIN>(c, k, HPC_KC_NONE);
     case EPI_REACTION:

@@ -977,16 +977,16 @@ int launch_to_f64(hpc_ctx* c, const float* src, double* dst, long long n) {
   return HPC_OK;
 }
 
-int launch_mech_update_f32(hpc_ctx* c, int level, int s_num, int s_den, int s_rz_next, int s_rn) {
+int launch_mech_update_f32(hpc_ctx* c, int level, const float* p, int s_num, int s_den, int s_rz_next, int s_rn) {
   const LevelGeo& g = c->L[level];
   const LevelF32& F = c->F32[level];
   const long long pairs = (long long)(g.px / 2) * g.ny * g.nz;
   const int grid = (int)std::min<long long>((pairs + kRowThreads - 1) / kRowThreads, (long long)num_sms_v() * 8);
   if (c->slab)
-    mech_update_kernel<float, true><<<grid, kRowThreads, 0, c->stream>>>(g, F.u, F.ru, F.p, F.w, F.invM, s_num, s_den,
+    mech_update_kernel<float, true><<<grid, kRowThreads, 0, c->stream>>>(g, F.u, F.ru, p, F.w, F.invM, s_num, s_den,
                                                                        make_red(c, s_rz_next, s_rn, -1));
   else
-    mech_update_kernel<float, false><<<grid, kRowThreads, 0, c->stream>>>(g, F.u, F.ru, F.p, F.w, F.invM, s_num,
+    mech_update_kernel<float, false><<<grid, kRowThreads, 0, c->stream>>>(g, F.u, F.ru, p, F.w, F.invM, s_num,
                                                                         s_den, make_red(c, s_rz_next, s_rn, -1));
   HPC_CHECK_LAUNCH(c);
   return HPC_OK;
