@@ -90,13 +90,14 @@ struct ClusterArgs {
   ClusterPlan p;
   IO* u;
   const IO* fu;
-  IO* ru;  // may be null
+  IO* ru;
   const T* invM;
   const T* Ke;  // element moduli; phase field: nodal gc and element H
   const T* Ge;
   T Ut;  // top value of u_z; phase field: the length scale lc
   int nb;
   double* scal;
+  int r_given;  // ru holds the first residual: no apply for it
   int s_rnorm, s_fnorm;  // |r|^2 of the first residual, |f|^2 (phase field); -1: not wanted
   double* err;  // set to 1 when a bounded wait ran out
 };
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
 
   // ---- initial residual r = f - K u, zero on Dirichlet rows
   if (tid == 0) expect(barB, (PF ? 3 : 2) * kPartBytes + zbytes);
-  apply();
+  if (!A.r_given) apply();
   double rz = 0.0, rn = 0.0, ff = 0.0;
 #pragma unroll
   for (int t = 0; t < kSlots; ++t) {
@@ -377,8 +378,8 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
     const long long n = node(a + q / PN, q % PN);
 #pragma unroll
     for (int m = 0; m < NC; ++m) {
-      const T fv = (T)A.fu[n + m * g.n];
-      const T rv = (info[t] >> m) & 1u ? T(0) : fv - w[t][m], z = rv * mi[t][m];
+      const T fv = A.r_given ? (T)A.ru[n + m * g.n] : (T)A.fu[n + m * g.n];
+      const T rv = (info[t] >> m) & 1u ? T(0) : (A.r_given ? fv : fv - w[t][m]), z = rv * mi[t][m];
       if (PF) ff = fma((double)fv, (double)fv, ff);
       r[t][m] = rv;
       rz = fma((double)rv, (double)z, rz);
@@ -474,7 +475,7 @@ __global__ void __launch_bounds__(kThreads, 1) cluster_pcg_kernel(const __grid_c
 #pragma unroll
     for (int m = 0; m < NC; ++m) {
       A.u[n + m * g.n] = (IO)u[t][m];
-      if (A.ru) A.ru[n + m * g.n] = (IO)r[t][m];
+      A.ru[n + m * g.n] = (IO)r[t][m];
     }
   }
   if (!ok && lane == 0) *A.err = 1.0;
@@ -548,25 +549,28 @@ int cluster_pcg_prepare(int device) {
 
 int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
                           const double* Ke, const double* Ge, double Ut, int nb) {
-  ClusterArgs<double, double> a{g, {}, u, fu, ru, invM, Ke, Ge, Ut, nb, c->scal, S_RNORM, -1, c->scal + S_ERR};
+  const int r_given = 0;
+  ClusterArgs<double, double> a{g, {}, u, fu, ru, invM, Ke, Ge, Ut, nb, c->scal, r_given, S_RNORM, -1, c->scal + S_ERR};
   return launch_cluster<false>(c, a);
 }
 
-int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb) {
+int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb, bool r_given) {
   const LevelFields& F = c->F[level];
-  return launch_cluster_pcg_on(c, c->L[level], F.u, F.fu, F.ru, F.preMu, F.Ke, F.Ge, Ut, nb);
-}
-
-int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb) {
-  const LevelF32& F = c->F32[level];
-  ClusterArgs<float, float> a{c->L[level], {}, F.u, F.fu, F.ru, F.invM, F.Ke, F.Ge, 0.f, nb, c->scal, -1, -1, c->scal + S_ERR};
+  ClusterArgs<double, double> a{c->L[level], {}, F.u, F.fu, F.ru, F.preMu, F.Ke, F.Ge, Ut, nb, c->scal, r_given, S_RNORM, -1,
+                                c->scal + S_ERR};
   return launch_cluster<false>(c, a);
 }
 
-int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb) {
+int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb, bool r_given) {
+  const LevelF32& F = c->F32[level];
+  ClusterArgs<float, float> a{c->L[level], {}, F.u, F.fu, F.ru, F.invM, F.Ke, F.Ge, 0.f, nb, c->scal, r_given, -1, -1, c->scal + S_ERR};
+  return launch_cluster<false>(c, a);
+}
+
+int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb, bool r_given) {
   const LevelFields& F = c->F[level];
   const LevelF32& G = c->F32[level];
-  ClusterArgs<double, float> a{c->L[level], {}, G.u, G.fu, nullptr, F.preMu, F.Ke, F.Ge, 0.0, nb, c->scal, S_RNORM, -1, c->scal + S_ERR};
+  ClusterArgs<double, float> a{c->L[level], {}, G.u, G.fu, G.ru, F.preMu, F.Ke, F.Ge, 0.0, nb, c->scal, r_given, S_RNORM, -1, c->scal + S_ERR};
   return launch_cluster<false>(c, a);
 }
 
@@ -578,7 +582,7 @@ bool cluster_pcg_d_fits(hpc_ctx* c, int level) {
 // pcg_d (phase_field_pcg.cpp:133-214) of a small level.
 int launch_cluster_pcg_d(hpc_ctx* c, int level, double lc, int nb) {
   const LevelFields& F = c->F[level];
-  ClusterArgs<double, double> a{c->L[level], {}, F.d, F.fd, F.R, F.preMd, F.gc, F.H, lc, nb, c->scal, S_RNORM, S_FDNORM,
+  ClusterArgs<double, double> a{c->L[level], {}, F.d, F.fd, F.R, F.preMd, F.gc, F.H, lc, nb, c->scal, 0, S_RNORM, S_FDNORM,
                                 c->scal + S_ERR};
   return launch_cluster<true>(c, a);
 }

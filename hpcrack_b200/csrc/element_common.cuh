@@ -20,16 +20,15 @@ struct StripGeo {
 template <typename T>
 struct MechKT {
   LevelGeo g;
-  LevelGeo gf;  // fine level (FAS)
   StripGeo sg;
   const T* fields[6];  // staged: u0,u1,u2 then K,G,d (finest) or Ke,Ge (coarse)
   T* out;
   const int8_t* choice;
   double small_k;
   T* fu;
+  T* r_out;
   int set_fnorm;
   const T* invM;
-  const T* rf;
   const T* gpm;  // finest level, precomputed Gauss-point moduli: K - 2G/3 at [g * n + e], G at [(8 + g) * n + e]
   RedTarget red;
   double* err;   // tensor-core kernel / TMA staging: set to 1 when a bounded wait ran out
@@ -49,7 +48,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 
 // What a kernel does with the finished operator row tot of node (x, ey, kk), by epilogue; own_p is the
 // applied vector at the node (EPI_PCG); pre_f and pre_m are f and (where k.invM is set) M^-1 at the node
-// (EPI_RESIDUAL).
+// (EPI_RESIDUAL), or pre_f what out holds there and pre_m M^-1 (EPI_FAS).
 template <typename T, int EPI>
 __device__ __forceinline__ void node_epilogue(const MechKT<T>& k, int x, int ey, int kk, const T (&tot)[3],
                                               const T (&own_p)[3], const T (&pre_f)[3], const T (&pre_m)[3],
@@ -95,13 +94,21 @@ __device__ __forceinline__ void node_epilogue(const MechKT<T>& k, int x, int ey,
       red0 = own ? s0 : red0;
     }
   } else if (EPI == EPI_FAS) {
-    // coarsen_f_standard_routine (multigrid_intergrid.cpp:124-342) fused with the coarse apply;
-    // a slab's lower ghost plane has no fine plane below it (its value comes from the neighbour)
-    const int fz = 2 * kk + k.g.zsh;
+    // the second half of coarsen_fu: out holds the full weighting of the fine residual.  With r_out that is
+    // also the first residual of the coarse smoother, f - K u for the injected u
+    const BcFlags bc = bc_flags(k.g, x, ey, kk);
+    const bool fix[3] = {bc.c0, bc.c1, bc.c2};
+    const bool own = owned_plane(k.g, kk);
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
-      k.out[n + m * N] =
-          tot[m] + (fz >= 0 ? full_weight(k.gf, k.rf + (long long)m * k.gf.n, 2 * x, 2 * ey, fz) : T(0));
+    for (int m = 0; m < 3; ++m) {
+      k.out[n + m * N] = tot[m] + pre_f[m];
+      if (k.r_out) {
+        const T rv = fix[m] ? T(0) : pre_f[m];
+        k.r_out[n + m * N] = rv;
+        const double s1 = fma((double)rv, (double)(rv * pre_m[m]), red1);
+        red1 = own ? s1 : red1;
+      }
+    }
   } else if (EPI == EPI_REACTION) {
     // Dirichlet_force_u (boundary_conditions.cpp:69-111)
     const BcFlags bc = bc_flags(k.g, x, ey, kk);

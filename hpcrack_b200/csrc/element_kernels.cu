@@ -204,11 +204,11 @@ __device__ __forceinline__ void assemble_row(const MechKT<T>& k, const ST& st, i
         for (int m = 0; m < 3; ++m) own_p[m] = st.at(si - 1, m, 0, lane);
       }
       T pre_f[3] = {T(0), T(0), T(0)}, pre_m[3] = {T(0), T(0), T(0)};
-      if (EPI == EPI_RESIDUAL) {
+      if (EPI == EPI_RESIDUAL || EPI == EPI_FAS) {
         const long long n = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
-          pre_f[m] = k.fu[n + m * k.g.n];
+          pre_f[m] = EPI == EPI_FAS ? k.out[n + m * k.g.n] : k.fu[n + m * k.g.n];
           if (k.invM) pre_m[m] = k.invM[n + m * k.g.n];
         }
       }
@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(kWarps * 32) mech_tc_kernel(MechKT<float> k) {
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   if (aborted && tid == 0 && k.err) *k.err = 1.0;
-  if (EPI == EPI_RESIDUAL || EPI == EPI_PCG) {
+  if (EPI == EPI_RESIDUAL || EPI == EPI_PCG || (EPI == EPI_FAS && k.red.slot[1] >= 0)) {
     double v[3] = {red0, red1, red2};
     grid_reduce<3>(v, k.red);
   }
@@ -945,12 +945,8 @@ static void mech_fields(hpc_ctx* c, int level, bool finest, bool diag, const dou
 }
 
 int launch_mech(hpc_ctx* c, const MechCall& m) {
-  // the restriction reads the fine residual around each coarse node: a slab takes the neighbours'
-  // planes first (SendRecv(rf), multigrid_intergrid.cpp:393)
-  if (m.epi == EPI_FAS) HPC_SLAB_HALO(c, m.fine_level, m.rf, 3, sizeof(double));
   MechK k{};
   k.g = c->L[m.level];
-  if (m.epi == EPI_FAS) k.gf = c->L[m.fine_level];
   mech_fields(c, m.level, m.finest, false, m.src, k);
   k.out = m.out;
   k.choice = c->F[m.level].choice;
@@ -958,10 +954,10 @@ int launch_mech(hpc_ctx* c, const MechCall& m) {
   k.fu = m.fu;
   k.set_fnorm = m.set_fnorm;
   k.invM = m.invM;
-  k.rf = m.rf;
   k.gpm = (m.finest && c->gpm_active) ? c->F[m.level].gpm : nullptr;
   k.red = make_red(c, m.s_out0, m.s_out1, m.s_out2);
   k.err = c->scal + S_ERR;
+  k.r_out = m.r_out;
   k.dir_r = m.dir_r;
   k.dir_m = m.invM;
   k.p_new = m.p_new;
@@ -1001,12 +997,10 @@ static int run_mech_tc(hpc_ctx* c, const MechKT<float>& k) {
 // Single-precision element operator of the precision form's V-cycle: the same kernels on the FP32
 // mirror of a level (LevelF32); residual, PCG apply and FAS right-hand side epilogues.
 int launch_mech_f32(hpc_ctx* c, const MechCall32& m) {
-  if (m.epi == EPI_FAS) HPC_SLAB_HALO(c, m.fine_level, m.rf, 3, sizeof(float));
   MechKT<float> k{};
   const LevelF32& F = c->F32[m.level];
   const LevelGeo& g = c->L[m.level];
   k.g = g;
-  if (m.epi == EPI_FAS) k.gf = c->L[m.fine_level];
   int f = 0;
   for (int q = 0; q < 3; ++q) k.fields[f++] = m.src + (long long)q * g.n;
   if (m.finest) {
@@ -1023,8 +1017,8 @@ int launch_mech_f32(hpc_ctx* c, const MechCall32& m) {
   k.small_k = m.small_k;
   k.fu = m.fu;
   k.set_fnorm = 0;
+  k.r_out = m.r_out;
   k.invM = m.invM;
-  k.rf = m.rf;
   k.gpm = (m.finest && c->gpm_active) ? F.gpm : nullptr;
   k.red = make_red(c, m.s_out0, m.s_out1, m.s_out2);
   k.err = c->scal + S_ERR;

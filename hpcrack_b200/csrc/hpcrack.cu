@@ -276,17 +276,22 @@ int pf_diags(hpc_ctx* c, int top, double lc) {
   return rc ? rc : check_zero_diags(c, top, "Precondition_M");
 }
 
+// Whether the smoother of level l runs in one thread-block cluster (a split gathers its coarsest level only).
+static bool cluster_smooths(hpc_ctx* c, int l) {
+  return c->fused_coarsest && slab_coarsest_mode(c) == 0 && cluster_pcg_fits(c, l);
+}
+
 // pcg_u (mechanical_pcg.cpp:223-330) with preMu of level l already built.  Device scalars only.
-static int pcg_u_dev(hpc_ctx* c, int l, double small_k, double Ut, int nb, int t) {
+// start: what is known of u and r - nothing (START_PLAIN), that u has its Dirichlet values (START_BC), or that F.ru and
+// slot_rz(0) hold the first residual as well (START_R: left by the FAS apply above it).
+enum SmootherStart { START_PLAIN, START_BC, START_R };
+static int pcg_u_dev(hpc_ctx* c, int l, double small_k, double Ut, int nb, int t, SmootherStart start = START_PLAIN) {
   if (nb > kMaxRelax) return arg_fail("nb_relax too large");
-  if (c->fused_coarsest) {
-    const int mode = slab_coarsest_mode(c);  // a split gathers its coarsest level only
-    if (mode == 1 && l == 0) return slab_coarsest(c, Ut, nb);
-    if (mode == 0 && cluster_pcg_fits(c, l)) return launch_cluster_pcg(c, l, Ut, nb);
-  }
+  if (cluster_smooths(c, l)) return launch_cluster_pcg(c, l, Ut, nb, start == START_R);
+  if (c->fused_coarsest && l == 0 && slab_coarsest_mode(c) == 1) return slab_coarsest(c, Ut, nb);
   LevelFields& F = c->F[l];
   int rc;
-  if ((rc = launch_bc(c, l, F.u, nullptr, 0, Ut))) return rc;  // Dirichlet_BD
+  if (start == START_PLAIN && (rc = launch_bc(c, l, F.u, nullptr, 0, Ut))) return rc;  // Dirichlet_BD
   MechCall m{};
   m.level = l;
   m.finest = is_finest(c, l);
@@ -300,7 +305,7 @@ static int pcg_u_dev(hpc_ctx* c, int l, double small_k, double Ut, int nb, int t
   m.s_out0 = m.set_fnorm ? S_FNORM : -1;
   m.s_out1 = slot_rz(0);
   m.s_out2 = S_RNORM;
-  if ((rc = launch_mech(c, m))) return rc;
+  if (start != START_R && (rc = launch_mech(c, m))) return rc;
   const bool fuse = can_fuse_dir(c, m.finest);  // the apply forms the direction: p and p2 in turn
   for (int it = 0; it < nb; ++it) {
     double* p = fuse && (it & 1) ? F.p2 : F.p;
@@ -364,56 +369,59 @@ static int pcg_d_dev(hpc_ctx* c, int l, double lc, int nb) {
   return HPC_OK;
 }
 
-static int cycle_u_dev(hpc_ctx* c, int l, const hpc_mg& mg, double small_k, double Ut, int t, long long* iters);
+static int cycle_u_dev(hpc_ctx* c, int l, const hpc_mg& mg, double small_k, double Ut, int t, long long* iters,
+                       SmootherStart start = START_PLAIN);
 static int cycle_d_dev(hpc_ctx* c, int l, const hpc_mg& mg, double lc, long long* iters);
 
 // The part of cycle_u(l) between its pre- and post-smoothing: coarsen_u, coarsen_fu, gamma cycles on
 // level l-1, refine_u (mechanical_multigrid.cpp:38-48).  Below the finest level t plays no role.
 static int coarse_part_u(hpc_ctx* c, int l, const hpc_mg& mg, double small_k, double Ut, int t, long long* iters) {
   int rc;
-  if ((rc = launch_inject_u(c, l, Ut))) return rc;  // coarsen_u
-  MechCall f{};                                      // coarsen_fu: fu_c = K_c u_c + FW(ru_f)
+  if ((rc = launch_coarsen_u(c, l, Ut))) return rc;  // coarsen_u, and the full weighting of coarsen_fu
+  // a split's gathered coarsest solve forms its own residual; a cluster's its own sums
+  const bool give_r = slab_coarsest_mode(c) == 0 || l > 1, sums = give_r && !cluster_smooths(c, l - 1);
+  MechCall f{};  // coarsen_fu: fu_c = K_c u_c + FW(ru_f), and with it the coarse smoother's first residual
   f.level = l - 1;
   f.finest = false;
   f.epi = EPI_FAS;
   f.src = c->F[l - 1].u;
   f.out = c->F[l - 1].fu;
   f.small_k = small_k;
-  f.rf = c->F[l].ru;
-  f.fine_level = l;
-  f.s_out0 = f.s_out1 = f.s_out2 = -1;
+  f.r_out = give_r ? c->F[l - 1].ru : nullptr;
+  f.invM = sums ? c->F[l - 1].preMu : nullptr;
+  f.s_out0 = f.s_out2 = -1;
+  f.s_out1 = sums ? slot_rz(0) : -1;
   if ((rc = launch_mech(c, f))) return rc;
   for (int j = 1; j <= mg.gamma; ++j)
-    if ((rc = cycle_u_dev(c, l - 1, mg, small_k, Ut, t, iters))) return rc;
+    if ((rc = cycle_u_dev(c, l - 1, mg, small_k, Ut, t, iters, j == 1 && give_r ? START_R : START_BC))) return rc;
   return launch_prolong(c, l, c->F[l - 1].u, c->F[l - 1].uold, c->F[l].u, 3, true, Ut);  // refine_u
 }
 
 // cycle_u (mechanical_multigrid.cpp:18-54); returns smoother iterations via *iters.
-static int cycle_u_dev(hpc_ctx* c, int l, const hpc_mg& mg, double small_k, double Ut, int t, long long* iters) {
+static int cycle_u_dev(hpc_ctx* c, int l, const hpc_mg& mg, double small_k, double Ut, int t, long long* iters,
+                       SmootherStart start) {
   int rc;
   if (l == 0) {
     *iters += mg.nu0;
-    return pcg_u_dev(c, 0, small_k, Ut, mg.nu0, t);
+    return pcg_u_dev(c, 0, small_k, Ut, mg.nu0, t, start);
   }
-  if ((rc = pcg_u_dev(c, l, small_k, Ut, mg.nu1, t))) return rc;
+  if ((rc = pcg_u_dev(c, l, small_k, Ut, mg.nu1, t, start))) return rc;
   *iters += mg.nu1;
   if ((rc = coarse_part_u(c, l, mg, small_k, Ut, t, iters))) return rc;
   *iters += mg.nu2;
-  return pcg_u_dev(c, l, small_k, Ut, mg.nu2, t);
+  return pcg_u_dev(c, l, small_k, Ut, mg.nu2, t, START_BC);
 }
 
 // The part of cycle_d(l) between its pre- and post-smoothing (phase_field_multigrid.cpp:39-43).
 static int coarse_part_d(hpc_ctx* c, int l, const hpc_mg& mg, double lc, long long* iters) {
   int rc;
-  if ((rc = launch_inject_d(c, l))) return rc;  // coarsen_d
+  if ((rc = launch_coarsen_d(c, l))) return rc;  // coarsen_d, and the full weighting of coarsen_f_d
   PfCall f{};                                    // coarsen_f_d
   f.level = l - 1;
   f.epi = EPI_FAS;
   f.src = c->F[l - 1].d;
   f.out = c->F[l - 1].fd;
   f.lc = lc;
-  f.rf = c->F[l].R;
-  f.fine_level = l;
   f.s_out0 = f.s_out1 = f.s_out2 = -1;
   if ((rc = launch_pf(c, f))) return rc;
   for (int j = 1; j <= mg.gamma; ++j)
@@ -497,7 +505,7 @@ int cycle_u_top(hpc_ctx* c, const hpc_mg& mg, double small_k, double Ut, int t, 
   if ((rc = run_graphed(c, c->gmech, mg, small_k, Ut, allow_capture,
                         [&] { return coarse_part_u(c, L, mg, small_k, Ut, t, &it); }, graph_flags(c))))
     return rc;
-  return pcg_u_dev(c, L, small_k, Ut, mg.nu2, t);
+  return pcg_u_dev(c, L, small_k, Ut, mg.nu2, t, START_BC);
 }
 
 int cycle_d_top(hpc_ctx* c, const hpc_mg& mg, double lc, bool allow_capture) {
@@ -682,11 +690,11 @@ int f32_material(hpc_ctx* c) {
 
 // pcg_u (mechanical_pcg.cpp:223-330) on the FP32 mirror, homogeneous Dirichlet values.
 // u_zero: the unknown is known to be zero (the finest pre-smoother of the correction), so the first
-// residual is f itself and needs no operator apply.
-static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, bool u_zero = false) {
+// residual is f itself and needs no operator apply.  start: as pcg_u_dev's (u always has its Dirichlet zeros).
+static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, SmootherStart start, bool u_zero = false) {
   if (nb > kMaxRelax) return arg_fail("nb_relax too large");
-  if (c->fused_coarsest && slab_coarsest_mode(c) == 0 && !c->tc_apply && cluster_pcg_fits(c, l))
-    return launch_cluster_pcg_f32(c, l, nb);
+  if (!c->tc_apply && cluster_smooths(c, l))
+    return launch_cluster_pcg_f32(c, l, nb, start == START_R);
   LevelF32& F = c->F32[l];
   int rc;
   MechCall32 m{};
@@ -694,8 +702,7 @@ static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, bool u_zero = fals
   m.finest = is_finest(c, l);
   if (u_zero) {
     if ((rc = launch_residual_zero_f32(c, l, slot_rz(0)))) return rc;
-  } else {
-    if ((rc = launch_bc_zero_f32(c, l, F.u))) return rc;
+  } else if (start != START_R) {
     m.epi = EPI_RESIDUAL;
     m.src = F.u;
     m.out = F.ru;
@@ -738,22 +745,22 @@ static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, bool u_zero = fals
 }
 
 // The coarsest level in FP64: pcg_u with nu0 iterations on the FP64 arrays of level 0.
-static int coarsest64(hpc_ctx* c, const hpc_mg& mg, double small_k) {
+static int coarsest64(hpc_ctx* c, const hpc_mg& mg, double small_k, SmootherStart start) {
   const long long n3 = 3 * c->L[0].n;
   int rc;
-  if (c->fused_coarsest && slab_coarsest_mode(c) == 0 && cluster_pcg_fits(c, 0))
-    return launch_cluster_pcg_mixed(c, 0, mg.nu0);
+  if (cluster_smooths(c, 0))
+    return launch_cluster_pcg_mixed(c, 0, mg.nu0, start == START_R);
   if ((rc = launch_to_f64(c, c->F32[0].u, c->F[0].u, n3))) return rc;
   if ((rc = launch_to_f64(c, c->F32[0].fu, c->F[0].fu, n3))) return rc;
   if ((rc = pcg_u_dev(c, 0, small_k, 0.0, mg.nu0, 1))) return rc;
   return launch_to_f32(c, c->F[0].u, c->F32[0].u, n3);
 }
 
-static int cycle_u32(hpc_ctx* c, int l, const hpc_mg& mg, double small_k);
+static int cycle_u32(hpc_ctx* c, int l, const hpc_mg& mg, double small_k, SmootherStart start);
 
 static int coarse_part_u32(hpc_ctx* c, int l, const hpc_mg& mg, double small_k) {
   int rc;
-  if ((rc = launch_inject_u_f32(c, l))) return rc;
+  if ((rc = launch_coarsen_u_f32(c, l))) return rc;
   MechCall32 f{};
   f.level = l - 1;
   f.finest = false;
@@ -761,21 +768,23 @@ static int coarse_part_u32(hpc_ctx* c, int l, const hpc_mg& mg, double small_k) 
   f.src = c->F32[l - 1].u;
   f.out = c->F32[l - 1].fu;
   f.small_k = small_k;
-  f.rf = c->F32[l].ru;
-  f.fine_level = l;
-  f.s_out0 = f.s_out1 = f.s_out2 = -1;
+  f.r_out = c->F32[l - 1].ru;
+  const bool sums = !(cluster_smooths(c, l - 1) && (l == 1 || !c->tc_apply));
+  f.invM = sums ? c->F32[l - 1].invM : nullptr;
+  f.s_out0 = f.s_out2 = -1;
+  f.s_out1 = sums ? slot_rz(0) : -1;
   if ((rc = launch_mech_f32(c, f))) return rc;
   for (int j = 1; j <= mg.gamma; ++j)
-    if ((rc = cycle_u32(c, l - 1, mg, small_k))) return rc;
+    if ((rc = cycle_u32(c, l - 1, mg, small_k, j == 1 ? START_R : START_BC))) return rc;
   return launch_prolong_f32(c, l);
 }
 
-static int cycle_u32(hpc_ctx* c, int l, const hpc_mg& mg, double small_k) {
+static int cycle_u32(hpc_ctx* c, int l, const hpc_mg& mg, double small_k, SmootherStart start) {
   int rc;
-  if (l == 0) return coarsest64(c, mg, small_k);
-  if ((rc = pcg_u32(c, l, small_k, mg.nu1))) return rc;
+  if (l == 0) return coarsest64(c, mg, small_k, start);
+  if ((rc = pcg_u32(c, l, small_k, mg.nu1, start))) return rc;
   if ((rc = coarse_part_u32(c, l, mg, small_k))) return rc;
-  return pcg_u32(c, l, small_k, mg.nu2);
+  return pcg_u32(c, l, small_k, mg.nu2, START_BC);
 }
 
 // ---------------------------------------------------------------- flexible PCG (precision form)
@@ -826,9 +835,9 @@ int fcg_iteration(hpc_ctx* c, const hpc_mg& mg, double small_k, int k, bool mixe
     HPC_CUDA(cudaMemsetAsync(G.u, 0, 3 * (size_t)g.n * sizeof(float), c->stream));
     if ((r2 = launch_to_f32(c, c->fcg.r, G.fu, 3 * g.n))) return r2;
     if (L == 0) {
-      if ((r2 = cycle_u32(c, 0, mg, small_k))) return r2;
+      if ((r2 = cycle_u32(c, 0, mg, small_k, START_BC))) return r2;
     } else {
-      if ((r2 = pcg_u32(c, L, small_k, mg.nu1, true))) return r2;
+      if ((r2 = pcg_u32(c, L, small_k, mg.nu1, START_BC, true))) return r2;
       if (coarse_graph) {
         if ((r2 = run_graphed(c, c->g32, mg, small_k, 0.0, k > 0, [&] { return coarse_part_u32(c, L, mg, small_k); },
                               graph_flags(c))))
@@ -836,7 +845,7 @@ int fcg_iteration(hpc_ctx* c, const hpc_mg& mg, double small_k, int k, bool mixe
       } else if ((r2 = coarse_part_u32(c, L, mg, small_k))) {
         return r2;
       }
-      if ((r2 = pcg_u32(c, L, small_k, mg.nu2))) return r2;
+      if ((r2 = pcg_u32(c, L, small_k, mg.nu2, START_BC))) return r2;
     }
   } else {
     HPC_CUDA(cudaMemsetAsync(F.u, 0, vbytes, c->stream));

@@ -240,15 +240,15 @@ struct MechCall {
   bool finest;
   int epi;
   const double* src;  // u (PLAIN / RESIDUAL / FAS / REACTION) or p (PCG)
-  double* out;        // Fi (PLAIN), r (RESIDUAL), w (PCG), fc (FAS), fu (REACTION: BC slots only)
+  double* out;        // Fi (PLAIN), r (RESIDUAL), w (PCG), fc (FAS: += K u), fu (REACTION: BC slots only)
   double small_k;
+  // FAS: r_out, also r = the weighted residual (Dirichlet rows zero) - what
+  // f - K u is for the injected u - and (r, M^-1 r) into s_out1 where invM is set
+  double* r_out;
   // RESIDUAL: r = fu - K u, zero at Dirichlet nodes; optionally fu[bc] = (K u)[bc] and f_norm.
   double* fu;
   bool set_fnorm;     // t == 0 on the finest level (mechanical_pcg.cpp:252-258)
   const double* invM; // RESIDUAL: inverse diagonal for rz = sum r^2 invM (null: no rz)
-  // FAS: fc = K_c u_c + full-weighting(rf)
-  const double* rf;
-  int fine_level;
   // reduction destinations (scalar slots, -1 = none)
   int s_out0, s_out1, s_out2;
   // PCG with the direction formed on the way (can_fuse_dir): p = dir_r M^-1 + beta src (beta from the slots, no
@@ -276,9 +276,8 @@ struct MechCall32 {
   float* out;
   double small_k;
   float* fu;          // RESIDUAL: right-hand side
+  float* r_out;       // FAS: the first residual, as in MechCall
   const float* invM;  // RESIDUAL: inverse diagonal for (r, M^-1 r)
-  const float* rf;    // FAS: fine residual
-  int fine_level;
   int s_out0, s_out1, s_out2;
   const float* dir_r;  // PCG with the direction formed on the way, as in MechCall
   float* p_new;
@@ -290,10 +289,8 @@ int launch_mech_f32(hpc_ctx* c, const MechCall32& m);
 int launch_mech_update_f32(hpc_ctx* c, int level, const float* p, int s_num, int s_den, int s_rz_next, int s_rn);
 // FP32 mirror: p = r M^-1 + beta p (beta from scal, 0 if first)
 int launch_dir_update_f32(hpc_ctx* c, int level, bool first, int s_rz, int s_rz_prev);
-int launch_bc_zero_f32(hpc_ctx* c, int level, float* v);  // zero the Dirichlet rows of a 3n vector
 // FP32 mirror: r = f (Dirichlet rows zero) and (r, M^-1 r) for a correction whose unknown is zero
 int launch_residual_zero_f32(hpc_ctx* c, int level, int s_rz);
-int launch_inject_u_f32(hpc_ctx* c, int lf);             // u_c = u_f(2i), Dirichlet rows 0, uold_c = u_c
 int launch_prolong_f32(hpc_ctx* c, int lf);              // u_f += P(u_c - uold_c), Dirichlet rows 0
 int launch_to_f32(hpc_ctx* c, const double* src, float* dst, long long n);
 int launch_to_f64(hpc_ctx* c, const float* src, double* dst, long long n);
@@ -307,8 +304,6 @@ struct PfCall {
   double lc;
   const double* fd;     // RESIDUAL: R = fd - A d
   const double* invM;   // RESIDUAL: inverse diagonal for rz (null: no rz)
-  const double* rf;
-  int fine_level;
   int s_out0, s_out1, s_out2;
 };
 int launch_pf(hpc_ctx* c, const PfCall& p);
@@ -347,9 +342,12 @@ cudaError_t kernel_binary_version(int* version);
 int launch_axpby(hpc_ctx* c, double* y, const double* a, const double* b, double sa, double sb, long long n);
 // Transfers
 int launch_inject(hpc_ctx* c, int lf, const double* f, double* co, int ncomp);
-int launch_inject_u(hpc_ctx* c, int lf, double Ut);  // u_c = u_f(2i), BC, uold_c = u_c (coarsen_u)
-int launch_inject_d(hpc_ctx* c, int lf);             // d_c = d_f(2i), dold_c = d_c (coarsen_d)
 int launch_restrict(hpc_ctx* c, int lf, const double* rf, const double* Fic, double* fc, int ncomp);
+// Injection u_c = uold_c = u_f(2i) (Dirichlet values set) and fc = full weighting of the fine residual, the
+// first half of the FAS right-hand side (EPI_FAS adds K_c u_c)
+int launch_coarsen_u(hpc_ctx* c, int lf, double Ut);
+int launch_coarsen_u_f32(hpc_ctx* c, int lf);
+int launch_coarsen_d(hpc_ctx* c, int lf);
 int launch_prolong(hpc_ctx* c, int lf, const double* uc, const double* ucold, double* uf, int ncomp,
                    bool apply_bc, double Ut);
 // Material / history
@@ -374,11 +372,12 @@ int upload_shape_table(const double* N64);
 bool cluster_pcg_fits(hpc_ctx* c, int level);
 bool cluster_pcg_fits_geo(const LevelGeo& g);
 int cluster_pcg_prepare(int device);
-int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb);
+// r_given: F.ru holds the first residual.
+int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb, bool r_given);
 int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
                           const double* Ke, const double* Ge, double Ut, int nb);
-int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb);
-int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb);
+int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb, bool r_given);
+int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb, bool r_given);
 // The same for pcg_d, any level that fits.
 bool cluster_pcg_d_fits(hpc_ctx* c, int level);
 int launch_cluster_pcg_d(hpc_ctx* c, int level, double lc, int nb);

@@ -296,13 +296,13 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
     const int kk = z0 - 1 + li;
     const T lam_c = lam_n, G_c = G_n;
     if (!GPM) coarse_mod(kk + 1);
-    // the residual's f and M^-1 of this plane's node: in flight under the arithmetic
+    // the residual's f and M^-1 of this plane's node (FAS: what out holds): in flight under the arithmetic
     T pre_f[3], pre_m[3];
-    if (EPI == EPI_RESIDUAL && out_node && kk >= z0) {
+    if ((EPI == EPI_RESIDUAL || EPI == EPI_FAS) && out_node && kk >= z0) {
       const long long n = (long long)x + (long long)y * k.g.px + (long long)kk * k.g.plane;
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
-        pre_f[m] = k.fu[n + m * k.g.n];
+        pre_f[m] = EPI == EPI_FAS ? k.out[n + m * k.g.n] : k.fu[n + m * k.g.n];
         pre_m[m] = k.invM ? k.invM[n + m * k.g.n] : T(0);
       }
     }
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
   }
   if constexpr (!TMA) asm volatile("cp.async.wait_all;\n" ::: "memory");
   if (TMA && bad && tid == 0 && k.err) *k.err = 1.0;
-  if (EPI == EPI_RESIDUAL || EPI == EPI_PCG) {
+  if (EPI == EPI_RESIDUAL || EPI == EPI_PCG || (EPI == EPI_FAS && k.red.slot[1] >= 0)) {
     double v[3] = {red0, red1, red2};
     grid_reduce<3>(v, k.red);
   }

@@ -23,14 +23,13 @@ constexpr size_t kPlane = (sizeof(double) * kNY * kBX + 127) / 128 * 128;
 constexpr size_t kOExch = 128 + kStages * 2 * kPlane, kSmem = kOExch + sizeof(double) * 2 * kTY * kXP + 128;
 
 struct PfTileK {
-  LevelGeo g, gf;
+  LevelGeo g;
   int tx, ty;  // tiles per axis
   const double *x, *gc, *H;
   double* out;
   double lc;
   const double* fd;
   const double* invM;
-  const double* rf;
   RedTarget red;
   double* err;
   alignas(64) CUtensorMap xmap;
@@ -168,10 +167,10 @@ __global__ void __launch_bounds__(kNT, 2) pf_tile_kernel(const __grid_constant__
     const double h = h_n;
     history(kk + 1);
     double pre_f = 0.0, pre_m = 0.0;
-    if (EPI == EPI_RESIDUAL && out_node && kk >= z0) {
+    if ((EPI == EPI_RESIDUAL || EPI == EPI_FAS) && out_node && kk >= z0) {
       const long long n = nidx(k.g, x, y, kk);
-      pre_f = k.fd[n];
-      if (k.invM) pre_m = k.invM[n];
+      pre_f = EPI == EPI_FAS ? k.out[n] : k.fd[n];
+      if (EPI == EPI_RESIDUAL && k.invM) pre_m = k.invM[n];
     }
     if (!wait(li + 1)) bad = 1;
     load_plane(li + 1, b);
@@ -262,8 +261,7 @@ __global__ void __launch_bounds__(kNT, 2) pf_tile_kernel(const __grid_constant__
         const double s0 = fma(a.own, tot, red0);
         red0 = own ? s0 : red0;
       } else if (EPI == EPI_FAS) {
-        const int fz = 2 * kk + k.g.zsh;
-        k.out[n] = tot + (fz >= 0 ? full_weight(k.gf, k.rf, 2 * x, 2 * y, fz) : 0.0);
+        k.out[n] = tot + pre_f;  // out holds the full weighting of the fine residual
       }
     }
     return true;
@@ -322,10 +320,8 @@ int run_pf_e(hpc_ctx* c, PfTileK& k, int cls) {
 }  // namespace
 
 int launch_pf(hpc_ctx* c, const PfCall& p) {
-  if (p.epi == EPI_FAS) HPC_SLAB_HALO(c, p.fine_level, p.rf, 1, sizeof(double));  // SendRecv(rf), :356
   PfTileK k{};
   k.g = c->L[p.level];
-  if (p.epi == EPI_FAS) k.gf = c->L[p.fine_level];
   k.x = p.src;
   k.gc = c->F[p.level].gc;
   k.H = c->F[p.level].H;
@@ -333,7 +329,6 @@ int launch_pf(hpc_ctx* c, const PfCall& p) {
   k.lc = p.lc;
   k.fd = p.fd;
   k.invM = p.invM;
-  k.rf = p.rf;
   k.red = make_red(c, p.s_out0, p.s_out1, p.s_out2);
   k.err = c->scal + S_ERR;
   switch (p.epi) {

@@ -380,56 +380,6 @@ int launch_inject(hpc_ctx* c, int lf, const double* f, double* co, int ncomp) {
   return HPC_OK;
 }
 
-// coarsen_u (:106-121): inject, Dirichlet_BD on the coarse level, save uold.
-template <typename T>
-__global__ void inject_u_kernel(LevelGeo gc, LevelGeo gf, const T* uf, T* uc, T* uold, T Ut) {
-  FOR_NODES(gc) {
-    const int fz = 2 * kz + gc.zsh;
-    if (fz < 0) continue;
-    const long long nc = nidx(gc, i, j, kz), nf = nidx(gf, 2 * i, 2 * j, fz);
-    T v[3] = {uf[nf], uf[nf + gf.n], uf[nf + 2 * gf.n]};
-    if (gc.bz[kz]) {
-      const BcFlags bc = bc_flags(gc, i, j, kz);
-      if (bc.c0) v[0] = T(0);
-      if (bc.c1) v[1] = T(0);
-      if (bc.c2) v[2] = bc.top ? Ut : T(0);
-    }
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      uc[nc + m * gc.n] = v[m];
-      uold[nc + m * gc.n] = v[m];
-    }
-  }
-}
-int launch_inject_u(hpc_ctx* c, int lf, double Ut) {
-  inject_u_kernel<<<row_grid(c->L[lf - 1]), kRowThreads, 0, c->stream>>>(
-      c->L[lf - 1], c->L[lf], c->F[lf].u, c->F[lf - 1].u, c->F[lf - 1].uold, Ut);
-  HPC_CHECK_LAUNCH(c);
-  HPC_SLAB_HALO(c, lf - 1, c->F[lf - 1].u, 3, sizeof(double));  // SendRecv(uc), multigrid_intergrid.cpp:116
-  HPC_SLAB_HALO(c, lf - 1, c->F[lf - 1].uold, 3, sizeof(double));
-  return HPC_OK;
-}
-
-// coarsen_d (:92-103)
-__global__ void inject_d_kernel(LevelGeo gc, LevelGeo gf, const double* df, double* dc, double* dold) {
-  FOR_NODES(gc) {
-    const int fz = 2 * kz + gc.zsh;
-    if (fz < 0) continue;
-    const long long nc = nidx(gc, i, j, kz), nf = nidx(gf, 2 * i, 2 * j, fz);
-    const double v = df[nf];
-    dc[nc] = v;
-    dold[nc] = v;
-  }
-}
-int launch_inject_d(hpc_ctx* c, int lf) {
-  inject_d_kernel<<<row_grid(c->L[lf - 1]), kRowThreads, 0, c->stream>>>(c->L[lf - 1], c->L[lf], c->F[lf].d,
-                                                                          c->F[lf - 1].d, c->F[lf - 1].dold);
-  HPC_CHECK_LAUNCH(c);
-  HPC_SLAB_HALO(c, lf - 1, c->F[lf - 1].d, 1, sizeof(double));  // SendRecv(dc), multigrid_intergrid.cpp:99
-  HPC_SLAB_HALO(c, lf - 1, c->F[lf - 1].dold, 1, sizeof(double));
-  return HPC_OK;
-}
-
 // coarsen_f_standard_routine (:124-342), standalone form (full_weight in device_common.cuh).
 __global__ void restrict_kernel(LevelGeo gc, LevelGeo gf, const double* rf, const double* Fic, double* fc, int ncomp) {
   FOR_NODES(gc) {
@@ -449,53 +399,167 @@ int launch_restrict(hpc_ctx* c, int lf, const double* rf, const double* Fic, dou
   return HPC_OK;
 }
 
-// refine_standard_routine (:416-520) as a gather over fine nodes, with the reference's term order;
-// optionally followed by Dirichlet_BD on the fine level (refine_u, :536-549).
-template <typename T>
-__global__ void prolong_kernel(LevelGeo gc, LevelGeo gf, const T* uc, const T* ucold, T* uf, int ncomp, int apply_bc,
-                               T Ut) {
-  FOR_NODES(gf) {
+// coarsen_u / coarsen_d (:92-121) and the full weighting of coarsen_fu / coarsen_f_d (:124-342, without the
+// K_c u_c part, which the FAS apply adds) in one pass: uc = uold = uf(2i) with the coarse Dirichlet values
+// (BC), fc = weighted rf.  The weights are (1/2, 1, 1/2) along each axis, neighbours outside the grid 0: a
+// thread owns a coarse column (i, j) over a few coarse planes and weights every fine plane once, the odd ones for
+// both coarse planes they touch.  A row's three values come from one aligned pair and the left lane.
+// Bound by the fine residual's read (134 us at 257^3 FP32).  The weighting used to sit in the FAS apply, 27
+// dependent loads per node and component at 8 to 16 warps an SM, next to a separate injection; with this pass
+// and the residual the apply hands down, increments of 257^3 FAS took 1376 ms, now 1322, of 129^3 19.7 and
+// 19.0, of 97^3 in the precision form 115.5 and 110.
+// On a z slab, coarse plane kc lies on fine plane 2 kc + zsh; a lower ghost plane without a fine plane below
+// it gets fc = 0 and leaves u to the ghost exchange.
+template <typename T, bool BC>
+__global__ void coarsen_kernel(LevelGeo gc, LevelGeo gf, const T* rf, T* fc, const T* uf, T* uc, T* uold, int ncomp,
+                               int planes, T Ut) {
+  using V2 = typename Vec2<T>::type;
+  const int lane = threadIdx.x & 31, warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int wx = (gc.nx + 31) / 32, wz = (gc.nz + planes - 1) / planes;
+  const int total = wx * gc.ny * wz * ncomp;
+  if (warp >= total) return;  // the whole warp
+  const int i = (warp % wx) * 32 + lane, j = (warp / wx) % gc.ny, k0 = (warp / (wx * gc.ny)) % wz * planes;
+  const int m = warp / (wx * gc.ny * wz);
+  const bool in = i < gc.nx;
+  const T* r = rf + (long long)m * gf.n;
+  const T* u = uf + (long long)m * gf.n;
+  auto plane = [&](int fz) -> T {
+    T s = T(0);
+    if (fz < 0 || fz >= gf.nz) return s;
+#pragma unroll
+    for (int dj = -1; dj <= 1; ++dj) {
+      const int fy = 2 * j + dj;
+      if (fy < 0 || fy >= gf.ny) continue;  // uniform over the warp
+      const long long n = nidx(gf, 2 * i, fy, fz);
+      V2 v{T(0), T(0)};
+      if (in) v = *reinterpret_cast<const V2*>(r + n);  // a padding slot beyond the last column holds 0
+      T left = __shfl_up_sync(kFull, v.y, 1);
+      if (lane == 0) left = i > 0 ? r[n - 1] : T(0);
+      const T row = v.x + T(0.5) * (left + v.y);
+      s += dj == 0 ? row : T(0.5) * row;
+    }
+    return s;
+  };
+  const int k1 = min(k0 + planes, gc.nz);
+  T below = plane(2 * k0 + gc.zsh - 1);
+  for (int k = k0; k < k1; ++k) {
+    const int fz = 2 * k + gc.zsh;
+    T uv = in && fz >= 0 ? u[nidx(gf, 2 * i, 2 * j, fz)] : T(0);
+    const T mid = plane(fz), above = plane(fz + 1);
+    if (in) {
+      const long long n = nidx(gc, i, j, k) + (long long)m * gc.n;
+      fc[n] = fz >= 0 ? mid + T(0.5) * (below + above) : T(0);
+      if (fz >= 0) {
+        if (BC && gc.bz[k]) {
+          const BcFlags b = bc_flags(gc, i, j, k);
+          if ((m == 0 && b.c0) || (m == 1 && b.c1)) uv = T(0);
+          if (m == 2 && b.c2) uv = b.top ? Ut : T(0);
+        }
+        uc[n] = uv;
+        uold[n] = uv;
+      }
+    }
+    below = above;
+  }
+}
+template <typename T, bool BC>
+static int run_coarsen(hpc_ctx* c, int lf, const T* rf, T* fc, const T* uf, T* uc, T* uold, int ncomp, T Ut) {
+  HPC_SLAB_HALO(c, lf, rf, ncomp, sizeof(T));  // SendRecv(rf), multigrid_intergrid.cpp:356,393
+  const LevelGeo& gc = c->L[lf - 1];
+  // planes a warp: enough that an odd fine plane is weighted once, few enough to fill the chip
+  const long long cols = (long long)((gc.nx + 31) / 32) * gc.ny * ncomp;
+  int planes = 8;
+  while (planes > 1 && cols * ((gc.nz + planes - 1) / planes) < (long long)num_sms_v() * 32) planes /= 2;
+  const long long warps = cols * ((gc.nz + planes - 1) / planes);
+  coarsen_kernel<T, BC><<<(int)((warps * 32 + kRowThreads - 1) / kRowThreads), kRowThreads, 0, c->stream>>>(
+      gc, c->L[lf], rf, fc, uf, uc, uold, ncomp, planes, Ut);
+  HPC_CHECK_LAUNCH(c);
+  HPC_SLAB_HALO(c, lf - 1, uc, ncomp, sizeof(T));  // SendRecv(uc), :99,116
+  HPC_SLAB_HALO(c, lf - 1, uold, ncomp, sizeof(T));
+  return HPC_OK;
+}
+int launch_coarsen_u(hpc_ctx* c, int lf, double Ut) {
+  const LevelFields &f = c->F[lf], &o = c->F[lf - 1];
+  return run_coarsen<double, true>(c, lf, f.ru, o.fu, f.u, o.u, o.uold, 3, Ut);
+}
+int launch_coarsen_u_f32(hpc_ctx* c, int lf) {
+  const LevelF32 &f = c->F32[lf], &o = c->F32[lf - 1];
+  return run_coarsen<float, true>(c, lf, f.ru, o.fu, f.u, o.u, o.uold, 3, 0.0f);
+}
+int launch_coarsen_d(hpc_ctx* c, int lf) {
+  const LevelFields &f = c->F[lf], &o = c->F[lf - 1];
+  return run_coarsen<double, false>(c, lf, f.R, o.fd, f.d, o.d, o.dold, 1, 0.0);
+}
+
+// refine_standard_routine (:416-520) as a gather over pairs of fine nodes (2i, 2i + 1) of a row, with the
+// reference's term order; optionally followed by Dirichlet_BD on the fine level (refine_u, :536-549).
+// A pair shares its coarse corners and is one aligned 16-byte (FP32: 8-byte) access: bound by HBM
+// (one node per thread, with eight branches, ran at a quarter of that rate).
+template <typename T, int NC>
+__global__ void prolong_kernel(LevelGeo gc, LevelGeo gf, const T* uc, const T* ucold, T* uf, int apply_bc, T Ut) {
+  using V2 = typename Vec2<T>::type;
+  const unsigned half = (unsigned)(gf.nx + 1) / 2u, npairs = half * (unsigned)gf.ny * (unsigned)gf.nz;
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < npairs; q += gridDim.x * blockDim.x) {
+    const unsigned row = q / half;
+    const int i = (int)(q - row * half), kz = (int)(row / (unsigned)gf.ny), j = (int)(row - (unsigned)kz * (unsigned)gf.ny);
     const int zq = kz - gc.zsh;  // fine plane counted from the coarse grid's plane 0
-    const int ox = i & 1, oy = j & 1, oz = zq & 1;
-    const int ic = (i + 1) >> 1, jc = (j + 1) >> 1, kc = (zq + 1) >> 1;
-    const long long nf = nidx(gf, i, j, kz);
-    BcFlags bc{false, false, false, false};
-    if (apply_bc && gf.bz[kz]) bc = bc_flags(gf, i, j, kz);
-    for (int m = 0; m < ncomp; ++m) {
+    const int oy = j & 1, oz = zq & 1, jc = (j + 1) >> 1, kc = (zq + 1) >> 1;
+    const bool odd = 2 * i + 1 < gf.nx;  // the pair's second node is a node (else a padding slot: unchanged)
+    const long long nf = nidx(gf, 2 * i, j, kz);
+    const long long c0 = nidx(gc, i, jc, kc), up = odd ? 1 : 0, dy = gc.px, dz = gc.plane;
+    BcFlags b0{false, false, false, false}, b1 = b0;
+    if (apply_bc && gf.bz[kz]) {
+      b0 = bc_flags(gf, 2 * i, j, kz);
+      if (odd) b1 = bc_flags(gf, 2 * i + 1, j, kz);
+    }
+#pragma unroll
+    for (int m = 0; m < NC; ++m) {
       const T* a = uc + m * gc.n;
       const T* o = ucold + m * gc.n;
-      auto E = [&](int x, int y, int z) -> T {
-        const long long q = nidx(gc, x, y, z);
-        return a[q] - o[q];
-      };
-      T add;
-      if (!ox && !oy && !oz) add = E(ic, jc, kc);
-      else if (ox && !oy && !oz) add = T(0.5) * (E(ic, jc, kc) + E(ic - 1, jc, kc));
-      else if (!ox && oy && !oz) add = T(0.5) * (E(ic, jc, kc) + E(ic, jc - 1, kc));
-      else if (!ox && !oy && oz) add = T(0.5) * (E(ic, jc, kc) + E(ic, jc, kc - 1));
-      else if (ox && oy && !oz)
-        add = T(0.25) * (E(ic, jc, kc) + E(ic, jc - 1, kc) + E(ic - 1, jc, kc) + E(ic - 1, jc - 1, kc));
-      else if (ox && !oy && oz)
-        add = T(0.25) * (E(ic, jc, kc) + E(ic - 1, jc, kc - 1) + E(ic, jc, kc - 1) + E(ic - 1, jc, kc));
-      else if (!ox && oy && oz)
-        add = T(0.25) * (E(ic, jc, kc) + E(ic, jc - 1, kc - 1) + E(ic, jc, kc - 1) + E(ic, jc - 1, kc));
-      else
-        add = T(0.125) * (E(ic, jc, kc) + E(ic, jc - 1, kc) + E(ic - 1, jc, kc) + E(ic - 1, jc - 1, kc) +
-                          E(ic, jc, kc - 1) + E(ic - 1, jc, kc - 1) + E(ic, jc - 1, kc - 1) + E(ic - 1, jc - 1, kc - 1));
-      T v = uf[nf + m * gf.n] + add;
-      if (apply_bc) {
-        if (m == 0 && bc.c0) v = T(0);
-        if (m == 1 && bc.c1) v = T(0);
-        if (m == 2 && bc.c2) v = bc.top ? Ut : T(0);
+      auto E = [&](long long n) -> T { return a[n] - o[n]; };
+      T add0, add1;  // corner l<x><y><z>: x, y, z steps back from (i + 1, jc, kc)
+      const T r000 = E(c0 + up), l000 = E(c0);
+      if (!oy && !oz) {
+        add0 = l000;
+        add1 = T(0.5) * (r000 + l000);
+      } else if (oy != oz) {
+        const long long d = oy ? dy : dz;
+        const T r1 = E(c0 + up - d), l1 = E(c0 - d);
+        add0 = T(0.5) * (l000 + l1);
+        add1 = oy ? T(0.25) * (r000 + r1 + l000 + l1) : T(0.25) * (r000 + l1 + r1 + l000);
+      } else {
+        const T ry = E(c0 + up - dy), ly = E(c0 - dy), rz = E(c0 + up - dz), lz = E(c0 - dz);
+        const T ryz = E(c0 + up - dy - dz), lyz = E(c0 - dy - dz);
+        add0 = T(0.25) * (l000 + lyz + lz + ly);
+        add1 = T(0.125) * (r000 + ry + l000 + ly + rz + lz + ryz + lyz);
       }
-      uf[nf + m * gf.n] = v;
+      V2 v = *reinterpret_cast<const V2*>(uf + nf + m * gf.n);
+      v.x += add0;
+      if (odd) v.y += add1;
+      if (apply_bc) {
+        if (m == 0 && b0.c0) v.x = T(0);
+        if (m == 0 && b1.c0) v.y = T(0);
+        if (m == 1 && b0.c1) v.x = T(0);
+        if (m == 1 && b1.c1) v.y = T(0);
+        if (m == 2 && b0.c2) v.x = b0.top ? Ut : T(0);
+        if (m == 2 && b1.c2) v.y = b1.top ? Ut : T(0);
+      }
+      *reinterpret_cast<V2*>(uf + nf + m * gf.n) = v;
     }
   }
 }
+// Threads of a kernel over the node pairs of a level.
+static int pair_grid(const LevelGeo& g) {
+  const long long pairs = (long long)((g.nx + 1) / 2) * g.ny * g.nz;
+  return (int)std::min<long long>((pairs + kRowThreads - 1) / kRowThreads, (long long)num_sms_v() * 8);
+}
 int launch_prolong(hpc_ctx* c, int lf, const double* uc, const double* ucold, double* uf, int ncomp, bool apply_bc,
                    double Ut) {
-  prolong_kernel<<<row_grid(c->L[lf]), kRowThreads, 0, c->stream>>>(c->L[lf - 1], c->L[lf], uc, ucold, uf, ncomp,
-                                                                     apply_bc ? 1 : 0, Ut);
+  const LevelGeo &gc = c->L[lf - 1], &gf = c->L[lf];
+  if (ncomp == 3)
+    prolong_kernel<double, 3><<<pair_grid(gf), kRowThreads, 0, c->stream>>>(gc, gf, uc, ucold, uf, apply_bc ? 1 : 0, Ut);
+  else
+    prolong_kernel<double, 1><<<pair_grid(gf), kRowThreads, 0, c->stream>>>(gc, gf, uc, ucold, uf, 0, 0.0);
   HPC_CHECK_LAUNCH(c);
   HPC_SLAB_HALO(c, lf, uf, ncomp, sizeof(double));  // SendRecv(uf), multigrid_intergrid.cpp:531,547
   return HPC_OK;
@@ -1000,23 +1064,9 @@ int launch_dir_update_f32(hpc_ctx* c, int level, bool first, int s_rz, int s_rz_
   HPC_SLAB_HALO(c, level, F.p, 3, sizeof(float));
   return HPC_OK;
 }
-int launch_bc_zero_f32(hpc_ctx* c, int level, float* v) {
-  const LevelGeo& g = c->L[level];
-  bc_kernel<float><<<row_grid(g), kRowThreads, 0, c->stream>>>(g, v, nullptr, 2, 0.0f);
-  HPC_CHECK_LAUNCH(c);
-  return HPC_OK;
-}
-int launch_inject_u_f32(hpc_ctx* c, int lf) {
-  inject_u_kernel<float><<<row_grid(c->L[lf - 1]), kRowThreads, 0, c->stream>>>(
-      c->L[lf - 1], c->L[lf], c->F32[lf].u, c->F32[lf - 1].u, c->F32[lf - 1].uold, 0.0f);
-  HPC_CHECK_LAUNCH(c);
-  HPC_SLAB_HALO(c, lf - 1, c->F32[lf - 1].u, 3, sizeof(float));
-  HPC_SLAB_HALO(c, lf - 1, c->F32[lf - 1].uold, 3, sizeof(float));
-  return HPC_OK;
-}
 int launch_prolong_f32(hpc_ctx* c, int lf) {
-  prolong_kernel<float><<<row_grid(c->L[lf]), kRowThreads, 0, c->stream>>>(
-      c->L[lf - 1], c->L[lf], c->F32[lf - 1].u, c->F32[lf - 1].uold, c->F32[lf].u, 3, 1, 0.0f);
+  prolong_kernel<float, 3><<<pair_grid(c->L[lf]), kRowThreads, 0, c->stream>>>(
+      c->L[lf - 1], c->L[lf], c->F32[lf - 1].u, c->F32[lf - 1].uold, c->F32[lf].u, 1, 0.0f);
   HPC_CHECK_LAUNCH(c);
   HPC_SLAB_HALO(c, lf, c->F32[lf].u, 3, sizeof(float));
   return HPC_OK;
