@@ -282,9 +282,32 @@ static bool cluster_smooths(hpc_ctx* c, int l) {
 }
 
 // pcg_u (mechanical_pcg.cpp:223-330) with preMu of level l already built.  Device scalars only.
-// start: what is known of u and r - nothing (START_PLAIN), that u has its Dirichlet values (START_BC), or that F.ru and
-// slot_rz(0) hold the first residual as well (START_R: left by the FAS apply above it).
-enum SmootherStart { START_PLAIN, START_BC, START_R };
+// start: what is known of u and r - nothing (START_PLAIN), that u has its Dirichlet values (START_BC), that F.ru and
+// slot_rz(0) hold the first residual as well (START_R: left by the FAS apply above it), or those and that u counts as
+// zero whatever it holds (START_ZERO).
+enum SmootherStart { START_PLAIN, START_BC, START_R, START_ZERO };
+// The update after iteration `it` of nb.  With alternating directions (pairs) u takes two steps at a time; r_unread: the
+// caller has no use for the last residual.
+template <typename T>
+static int smoother_update(hpc_ctx* c, int l, T* u, T* r, const T* p, const T* p_other, const T* w, const T* invM, int it,
+                           int nb, bool pairs, bool u_zero, bool r_unread) {
+  const bool odd = (it & 1) != 0, last = it == nb - 1;
+  MechUpdate<T> a{};
+  a.u = pairs && !odd && !last ? nullptr : u;
+  a.r = last && r_unread ? nullptr : r;
+  a.p = p;
+  a.p_prev = pairs && odd ? p_other : nullptr;
+  a.w = w;
+  a.invM = invM;
+  a.s_num = slot_rz(it);
+  a.s_den = slot_pw(it);
+  a.s_num0 = pairs && odd ? slot_rz(it - 1) : 0;
+  a.s_den0 = pairs && odd ? slot_pw(it - 1) : 0;
+  a.s_rz_next = slot_rz(it + 1);
+  a.s_rn = slot_rn(it);
+  a.u_zero = u_zero && it <= (pairs ? 1 : 0);
+  return launch_mech_update(c, l, a);
+}
 static int pcg_u_dev(hpc_ctx* c, int l, double small_k, double Ut, int nb, int t, SmootherStart start = START_PLAIN) {
   if (nb > kMaxRelax) return arg_fail("nb_relax too large");
   if (cluster_smooths(c, l)) return launch_cluster_pcg(c, l, Ut, nb, start == START_R);
@@ -305,7 +328,8 @@ static int pcg_u_dev(hpc_ctx* c, int l, double small_k, double Ut, int nb, int t
   m.s_out0 = m.set_fnorm ? S_FNORM : -1;
   m.s_out1 = slot_rz(0);
   m.s_out2 = S_RNORM;
-  if (start != START_R && (rc = launch_mech(c, m))) return rc;
+  if (start < START_R && (rc = launch_mech(c, m))) return rc;
+  if (start == START_ZERO && nb == 0) HPC_CUDA(cudaMemsetAsync(F.u, 0, 3 * (size_t)c->L[l].n * sizeof(double), c->stream));
   const bool fuse = can_fuse_dir(c, m.finest);  // the apply forms the direction: p and p2 in turn
   for (int it = 0; it < nb; ++it) {
     double* p = fuse && (it & 1) ? F.p2 : F.p;
@@ -330,7 +354,8 @@ static int pcg_u_dev(hpc_ctx* c, int l, double small_k, double Ut, int nb, int t
       if ((rc = launch_dir_update(c, l, 3, F.ru, F.preMu, p, it == 0, slot_rz(it), slot_rz(it - 1)))) return rc;
     }
     if ((rc = launch_mech(c, q))) return rc;
-    if ((rc = launch_mech_update(c, l, p, slot_rz(it), slot_pw(it), slot_rz(it + 1), slot_rn(it)))) return rc;
+    if ((rc = smoother_update<double>(c, l, F.u, F.ru, p, q.src, F.w, F.preMu, it, nb, fuse, start == START_ZERO, false)))
+      return rc;
   }
   return HPC_OK;
 }
@@ -496,12 +521,13 @@ static int run_graphed(hpc_ctx* c, hpc_ctx::CoarseGraph& g, const hpc_mg& mg, do
 
 // Top-level cycles of the solves: the finest level's smoothing is launched directly (its kernels
 // are large and individually timed), everything below it is replayed as one graph.
-int cycle_u_top(hpc_ctx* c, const hpc_mg& mg, double small_k, double Ut, int t, bool allow_capture) {
+int cycle_u_top(hpc_ctx* c, const hpc_mg& mg, double small_k, double Ut, int t, bool allow_capture, bool u_zero) {
   const int L = c->maxlevel;
   long long it = 0;
-  if (L == 0) return cycle_u_dev(c, 0, mg, small_k, Ut, t, &it);
+  const SmootherStart start = u_zero ? START_ZERO : START_PLAIN;
+  if (L == 0) return cycle_u_dev(c, 0, mg, small_k, Ut, t, &it, start);
   int rc;
-  if ((rc = pcg_u_dev(c, L, small_k, Ut, mg.nu1, t))) return rc;
+  if ((rc = pcg_u_dev(c, L, small_k, Ut, mg.nu1, t, start))) return rc;
   if ((rc = run_graphed(c, c->gmech, mg, small_k, Ut, allow_capture,
                         [&] { return coarse_part_u(c, L, mg, small_k, Ut, t, &it); }, graph_flags(c))))
     return rc;
@@ -689,9 +715,8 @@ int f32_material(hpc_ctx* c) {
 }
 
 // pcg_u (mechanical_pcg.cpp:223-330) on the FP32 mirror, homogeneous Dirichlet values.
-// u_zero: the unknown is known to be zero (the finest pre-smoother of the correction), so the first
-// residual is f itself and needs no operator apply.  start: as pcg_u_dev's (u always has its Dirichlet zeros).
-static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, SmootherStart start, bool u_zero = false) {
+// start: as pcg_u_dev's (u always has its Dirichlet zeros).  post: nobody reads the residual it ends with.
+static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, SmootherStart start, bool post) {
   if (nb > kMaxRelax) return arg_fail("nb_relax too large");
   if (!c->tc_apply && cluster_smooths(c, l))
     return launch_cluster_pcg_f32(c, l, nb, start == START_R);
@@ -700,9 +725,7 @@ static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, SmootherStart star
   MechCall32 m{};
   m.level = l;
   m.finest = is_finest(c, l);
-  if (u_zero) {
-    if ((rc = launch_residual_zero_f32(c, l, slot_rz(0)))) return rc;
-  } else if (start != START_R) {
+  if (start < START_R) {
     m.epi = EPI_RESIDUAL;
     m.src = F.u;
     m.out = F.ru;
@@ -714,6 +737,7 @@ static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, SmootherStart star
     m.s_out2 = -1;
     if ((rc = launch_mech_f32(c, m))) return rc;
   }
+  if (start == START_ZERO && nb == 0) HPC_CUDA(cudaMemsetAsync(F.u, 0, 3 * (size_t)c->L[l].n * sizeof(float), c->stream));
   const bool fuse = !c->tc_apply && can_fuse_dir(c, m.finest);
   float* p2 = reinterpret_cast<float*>(c->F[l].p2);
   for (int it = 0; it < nb; ++it) {
@@ -739,7 +763,8 @@ static int pcg_u32(hpc_ctx* c, int l, double small_k, int nb, SmootherStart star
       if ((rc = launch_dir_update_f32(c, l, it == 0, slot_rz(it), slot_rz(it - 1)))) return rc;
     }
     if ((rc = launch_mech_f32(c, q))) return rc;
-    if ((rc = launch_mech_update_f32(c, l, p, slot_rz(it), slot_pw(it), slot_rz(it + 1), slot_rn(it)))) return rc;
+    if ((rc = smoother_update<float>(c, l, F.u, F.ru, p, q.src, F.w, F.invM, it, nb, fuse, start == START_ZERO, post)))
+      return rc;
   }
   return HPC_OK;
 }
@@ -782,9 +807,9 @@ static int coarse_part_u32(hpc_ctx* c, int l, const hpc_mg& mg, double small_k) 
 static int cycle_u32(hpc_ctx* c, int l, const hpc_mg& mg, double small_k, SmootherStart start) {
   int rc;
   if (l == 0) return coarsest64(c, mg, small_k, start);
-  if ((rc = pcg_u32(c, l, small_k, mg.nu1, start))) return rc;
+  if ((rc = pcg_u32(c, l, small_k, mg.nu1, start, false))) return rc;
   if ((rc = coarse_part_u32(c, l, mg, small_k))) return rc;
-  return pcg_u32(c, l, small_k, mg.nu2, START_BC);
+  return pcg_u32(c, l, small_k, mg.nu2, START_BC, true);
 }
 
 // ---------------------------------------------------------------- flexible PCG (precision form)
@@ -826,18 +851,18 @@ int fcg_iteration(hpc_ctx* c, const hpc_mg& mg, double small_k, int k, bool mixe
   const int L = c->maxlevel;
   LevelFields& F = c->F[L];
   const LevelGeo& g = c->L[L];
-  const size_t vbytes = sizeof(double) * 3 * (size_t)g.n;
   int r2;
   // z = V-cycle on A z = r from z = 0 with homogeneous Dirichlet values: u is the cycle's unknown,
   // fu its right-hand side
   if (mixed) {  // the same cycle on the FP32 mirror; z comes back to F.u in FP64
     const LevelF32& G = c->F32[L];
-    HPC_CUDA(cudaMemsetAsync(G.u, 0, 3 * (size_t)g.n * sizeof(float), c->stream));
-    if ((r2 = launch_to_f32(c, c->fcg.r, G.fu, 3 * g.n))) return r2;
     if (L == 0) {
+      HPC_CUDA(cudaMemsetAsync(G.u, 0, 3 * (size_t)g.n * sizeof(float), c->stream));
+      if ((r2 = launch_to_f32(c, c->fcg.r, G.fu, 3 * g.n))) return r2;
       if ((r2 = cycle_u32(c, 0, mg, small_k, START_BC))) return r2;
     } else {
-      if ((r2 = pcg_u32(c, L, small_k, mg.nu1, START_BC, true))) return r2;
+      if ((r2 = launch_zero_start_f32(c, L, c->fcg.r, slot_rz(0)))) return r2;
+      if ((r2 = pcg_u32(c, L, small_k, mg.nu1, START_ZERO, false))) return r2;
       if (coarse_graph) {
         if ((r2 = run_graphed(c, c->g32, mg, small_k, 0.0, k > 0, [&] { return coarse_part_u32(c, L, mg, small_k); },
                               graph_flags(c))))
@@ -845,12 +870,11 @@ int fcg_iteration(hpc_ctx* c, const hpc_mg& mg, double small_k, int k, bool mixe
       } else if ((r2 = coarse_part_u32(c, L, mg, small_k))) {
         return r2;
       }
-      if ((r2 = pcg_u32(c, L, small_k, mg.nu2, START_BC))) return r2;
+      if ((r2 = pcg_u32(c, L, small_k, mg.nu2, START_BC, true))) return r2;
     }
   } else {
-    HPC_CUDA(cudaMemsetAsync(F.u, 0, vbytes, c->stream));
-    HPC_CUDA(cudaMemcpyAsync(F.fu, c->fcg.r, vbytes, cudaMemcpyDeviceToDevice, c->stream));
-    if ((r2 = cycle_u_top(c, mg, small_k, 0.0, 1, k > 0))) return r2;
+    if ((r2 = launch_zero_start(c, L, c->fcg.r, slot_rz(0)))) return r2;
+    if ((r2 = cycle_u_top(c, mg, small_k, 0.0, 1, k > 0, true))) return r2;
   }
   // delta_k = (z, r_k), gamma_k = (z, r_{k-1}); p = z + beta p.  The precision form reads z from the
   // FP32 cycle directly (its FP64 copy would be exact).
@@ -877,10 +901,17 @@ int fcg_iteration(hpc_ctx* c, const hpc_mg& mg, double small_k, int k, bool mixe
   q.s_out0 = slot_fpw(k);
   q.s_out1 = q.s_out2 = -1;
   if ((r2 = launch_mech(c, q))) return r2;
-  // r_{k-1} kept for the flexible beta; x += alpha p, r -= alpha w, alpha = delta_k / (p, w)
-  HPC_CUDA(cudaMemcpyAsync(c->fcg.rp, c->fcg.r, vbytes, cudaMemcpyDeviceToDevice, c->stream));
-  return launch_mech_update_on(c, L, c->fcg.x, c->fcg.r, c->fcg.p, F.w, F.preMu, slot_fdelta(k), slot_fpw(k),
-                               slot_fdummy(k), slot_frn(k));
+  // x += alpha p, r -= alpha w, alpha = delta_k / (p, w); r_{k-1} kept for the flexible beta
+  MechUpdate<double> a{};
+  a.u = c->fcg.x;
+  a.r = c->fcg.r;
+  a.r_old = c->fcg.rp;
+  a.p = c->fcg.p;
+  a.w = F.w;
+  a.s_num = slot_fdelta(k);
+  a.s_den = slot_fpw(k);
+  a.s_rn = slot_frn(k);
+  return launch_mech_update(c, L, a);
 }
 
 // The mechanical solve of u_entire (mechanical_displacement.cpp:25-115) by flexible PCG on the finest

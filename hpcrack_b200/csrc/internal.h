@@ -89,7 +89,6 @@ inline int slot_fdelta(int k) { return S_FCG + (k & 1); }
 inline int slot_fgamma(int k) { return S_FCG + 2 + (k & 1); }
 inline int slot_fpw(int k) { return S_FCG + 4 + (k & 1); }
 inline int slot_frn(int k) { return S_FCG + 6 + (k & 1); }
-inline int slot_fdummy(int k) { return S_FCG + 8 + (k & 1); }
 
 }  // namespace hpc
 
@@ -285,12 +284,12 @@ struct MechCall32 {
   int s_rz, s_rz_prev;
 };
 int launch_mech_f32(hpc_ctx* c, const MechCall32& m);
-// FP32 mirror: u += alpha p, r -= alpha w on F32[level] (Dirichlet rows zero), alpha = scal[s_num]/scal[s_den]
-int launch_mech_update_f32(hpc_ctx* c, int level, const float* p, int s_num, int s_den, int s_rz_next, int s_rn);
 // FP32 mirror: p = r M^-1 + beta p (beta from scal, 0 if first)
 int launch_dir_update_f32(hpc_ctx* c, int level, bool first, int s_rz, int s_rz_prev);
-// FP32 mirror: r = f (Dirichlet rows zero) and (r, M^-1 r) for a correction whose unknown is zero
-int launch_residual_zero_f32(hpc_ctx* c, int level, int s_rz);
+// f = src (in the level's or the FP32 mirror's precision), ru = f with Dirichlet rows zero, (ru, M^-1 ru) into
+// scal[s_rz]: a correction whose unknown is zero
+int launch_zero_start(hpc_ctx* c, int level, const double* src, int s_rz);
+int launch_zero_start_f32(hpc_ctx* c, int level, const double* src, int s_rz);
 int launch_prolong_f32(hpc_ctx* c, int lf);              // u_f += P(u_c - uold_c), Dirichlet rows 0
 int launch_to_f32(hpc_ctx* c, const double* src, float* dst, long long n);
 int launch_to_f64(hpc_ctx* c, const float* src, double* dst, long long n);
@@ -310,12 +309,20 @@ int launch_pf(hpc_ctx* c, const PfCall& p);
 int launch_pf_diag(hpc_ctx* c, int level, double lc, double* out);
 
 // Vector kernels (vector_kernels.cu).
-// Mechanical CG update: alpha = scal[s_rz]/scal[s_pw]; u += alpha p; r -= alpha w; r = 0 on Dirichlet
-// nodes; scal[s_rz_next] = sum r^2/preM; scal[s_rn] = sum r^2.
-int launch_mech_update(hpc_ctx* c, int level, const double* p, int s_rz, int s_pw, int s_rz_next, int s_rn);
-// Same on explicit arrays: x += alpha p, r -= alpha w (Dirichlet rows zero), alpha = scal[s_num]/scal[s_den].
-int launch_mech_update_on(hpc_ctx* c, int level, double* x, double* r, const double* p, const double* w,
-                          const double* invM, int s_num, int s_den, int s_rz_next, int s_rn);
+// Mechanical CG update with alpha = scal[s_num] / scal[s_den]: u += alpha p and, with p_prev, the step before it
+// (alpha from s_num0, s_den0); r -= alpha w, r = 0 on Dirichlet nodes; scal[s_rz_next] = (r, M^-1 r), scal[s_rn] =
+// (r, r).  u or r null: that half is left alone.  u_zero: u counts as zero and is not read.  r_old: takes the old r,
+// and (r, M^-1 r) is not formed.
+template <typename T>
+struct MechUpdate {
+  T *u, *r;
+  const T *p, *p_prev, *w, *invM;
+  T* r_old;
+  int s_num, s_den, s_num0, s_den0, s_rz_next, s_rn;
+  int u_zero;
+};
+template <typename T>
+int launch_mech_update(hpc_ctx* c, int level, const MechUpdate<T>& a);
 // sums (a, b) and (a, c) over a 3n vector of a level into scal[s0], scal[s1] (c may be null)
 int launch_dot2(hpc_ctx* c, int level, const double* a, const double* b, const double* cv, int s0, int s1);
 int launch_dot2(hpc_ctx* c, int level, const float* a, const double* b, const double* cv, int s0, int s1);
@@ -393,7 +400,7 @@ int mech_diags_enqueue(hpc_ctx* c, int top, double small_k);
 int pf_diags_enqueue(hpc_ctx* c, int top, double lc);
 int mech_material(hpc_ctx* c, double small_k);
 int gp_material(hpc_ctx* c, double small_k);
-int cycle_u_top(hpc_ctx* c, const hpc_mg& mg, double small_k, double Ut, int t, bool allow_capture);
+int cycle_u_top(hpc_ctx* c, const hpc_mg& mg, double small_k, double Ut, int t, bool allow_capture, bool u_zero = false);
 int cycle_d_top(hpc_ctx* c, const hpc_mg& mg, double lc, bool allow_capture);
 int ensure_f32(hpc_ctx* c);
 int f32_material(hpc_ctx* c);

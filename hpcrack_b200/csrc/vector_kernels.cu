@@ -43,6 +43,21 @@ int row_grid(const LevelGeo& g, int per_sm = 8) {
              kz = (int)(_f / ((unsigned)(g).nx * (unsigned)(g).ny)), _once = 1;                        \
          _once; _once = 0)
 
+// The same over the pairs (i, i + 1) of x-adjacent slots that hold a node, n the first one's slot: 16-byte accesses,
+// the x pitch is a multiple of 4.  A row's last pair may hold a padding slot.
+#define FOR_PAIRS(g)                                                                                              \
+  for (unsigned _h = (unsigned)((g).nx + 1) / 2u, _q = blockIdx.x * blockDim.x + threadIdx.x,                      \
+                _pairs = _h * (unsigned)(g).ny * (unsigned)(g).nz;                                                 \
+       _q < _pairs; _q += gridDim.x * blockDim.x)                                                                  \
+    for (int _row = (int)(_q / _h), i = 2 * (int)(_q - (unsigned)_row * _h), kz = _row / (g).ny, j = _row - kz * (g).ny, \
+             _once = 1;                                                                                            \
+         _once; _once = 0)                                                                                         \
+      for (const long long n = nidx(g, i, j, kz); _once; _once = 0)
+int pair_grid(const LevelGeo& g) {
+  const long long pairs = (long long)((g.nx + 1) / 2) * g.ny * g.nz;
+  return (int)std::min<long long>((pairs + kRowThreads - 1) / kRowThreads, (long long)num_sms_v() * 8);
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------------------------
@@ -55,13 +70,21 @@ template <typename T> struct Vec2;
 template <> struct Vec2<double> { using type = double2; };
 template <> struct Vec2<float> { using type = float2; };
 
+// A call touches only what it needs, because every vector is a pass over HBM (5.0 to 6.5 TB/s at 257^3, a copy
+// reaches 6.5):
+//   X  what happens to u: 0 nothing, 1 u += alpha p, 2 u += alpha' p' + alpha p with the iteration before, whose
+//      direction still stands in the other array (the applies alternate between two).  Two iterations then
+//      move 4 + 8 vectors instead of 7 + 7: 161 + 262 us on 257^3 in FP32 against 2 x 248.
+//   R  what happens to r: 0 nothing (a last update whose residual nobody reads: 124 us), 1 r -= alpha w with
+//      (r, M^-1 r) and (r, r), 2 the outer iteration's: no M^-1, the old r kept in r_old (471 us on 257^3 in
+//      FP64; an update without it and a copy took 457 + 125).
 // SLAB: sums over owned planes only (a z-slab context); the whole-specimen instance keeps the register
 // budget of the plain loop (48 against 58 with the test).
-template <typename T, bool SLAB = false>
-__global__ void mech_update_kernel(LevelGeo g, T* u, T* r, const T* p, const T* w, const T* invM, int s_rz, int s_pw,
-                                   RedTarget red) {
+template <typename T, bool SLAB, int X, int R>
+__global__ void mech_update_kernel(LevelGeo g, MechUpdate<T> a, RedTarget red) {
   using V2 = typename Vec2<T>::type;
-  const T alpha = (T)(red.scal[s_rz] / red.scal[s_pw]);
+  const T alpha = (T)(red.scal[a.s_num] / red.scal[a.s_den]);
+  const T alpha0 = X == 2 ? (T)(red.scal[a.s_num0] / red.scal[a.s_den0]) : T(0);
   double rz = 0.0, rn = 0.0;
   const unsigned half = (unsigned)g.px / 2u, npairs = half * (unsigned)g.ny * (unsigned)g.nz;
   for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < npairs; q += gridDim.x * blockDim.x) {
@@ -71,7 +94,7 @@ __global__ void mech_update_kernel(LevelGeo g, T* u, T* r, const T* p, const T* 
     const long long n = (long long)row * g.px + i;
     const double rz0 = rz, rn0 = rn;
     bool fix[2][3] = {{false, false, false}, {false, false, false}};
-    if (g.bz[kz]) {
+    if (R && g.bz[kz]) {
 #pragma unroll
       for (int h = 0; h < 2; ++h)
         if (i + h < g.nx) {
@@ -81,56 +104,90 @@ __global__ void mech_update_kernel(LevelGeo g, T* u, T* r, const T* p, const T* 
           fix[h][2] = bc.c2;
         }
     }
+    // every load before the first store, which they could not be moved across
+    V2 pv[3], p0[3], uv[3], wv[3], rv[3], mv[3];
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       const long long o = n + (long long)m * g.n;
-      const V2 pv = *reinterpret_cast<const V2*>(p + o);
-      const V2 wv = *reinterpret_cast<const V2*>(w + o);
-      const V2 mv = *reinterpret_cast<const V2*>(invM + o);
-      V2 uv = *reinterpret_cast<const V2*>(u + o);
-      V2 rv = *reinterpret_cast<const V2*>(r + o);
-      uv.x = fma(pv.x, alpha, uv.x);
-      uv.y = fma(pv.y, alpha, uv.y);
-      rv.x = fix[0][m] ? T(0) : fma(-wv.x, alpha, rv.x);
-      rv.y = fix[1][m] ? T(0) : fma(-wv.y, alpha, rv.y);
-      *reinterpret_cast<V2*>(u + o) = uv;
-      *reinterpret_cast<V2*>(r + o) = rv;
-      rz = fma((double)rv.x, (double)(rv.x * mv.x), rz);
-      rz = fma((double)rv.y, (double)(rv.y * mv.y), rz);
-      rn = fma((double)rv.x, (double)rv.x, rn);
-      rn = fma((double)rv.y, (double)rv.y, rn);
+      if (X) pv[m] = *reinterpret_cast<const V2*>(a.p + o);
+      if (X == 2) p0[m] = *reinterpret_cast<const V2*>(a.p_prev + o);
+      uv[m] = V2{T(0), T(0)};
+      if (X && !a.u_zero) uv[m] = *reinterpret_cast<const V2*>(a.u + o);
+      if (R) {
+        wv[m] = *reinterpret_cast<const V2*>(a.w + o);
+        rv[m] = *reinterpret_cast<const V2*>(a.r + o);
+      }
+      if (R == 1) mv[m] = *reinterpret_cast<const V2*>(a.invM + o);
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const long long o = n + (long long)m * g.n;
+      if (X) {
+        V2 x = uv[m];
+        if (X == 2) {
+          x.x = fma(p0[m].x, alpha0, x.x);
+          x.y = fma(p0[m].y, alpha0, x.y);
+        }
+        x.x = fma(pv[m].x, alpha, x.x);
+        x.y = fma(pv[m].y, alpha, x.y);
+        if (i + 1 >= g.nx) {  // padding slots stay zero: the applies stage them, and those of p may hold anything
+          x.y = T(0);
+          if (i >= g.nx) x.x = T(0);
+        }
+        *reinterpret_cast<V2*>(a.u + o) = x;
+      }
+      if (R) {
+        V2 r = rv[m];
+        if (R == 2) *reinterpret_cast<V2*>(a.r_old + o) = r;
+        r.x = fix[0][m] ? T(0) : fma(-wv[m].x, alpha, r.x);
+        r.y = fix[1][m] ? T(0) : fma(-wv[m].y, alpha, r.y);
+        *reinterpret_cast<V2*>(a.r + o) = r;
+        if (R == 1) {
+          rz = fma((double)r.x, (double)(r.x * mv[m].x), rz);
+          rz = fma((double)r.y, (double)(r.y * mv[m].y), rz);
+        }
+        rn = fma((double)r.x, (double)r.x, rn);
+        rn = fma((double)r.y, (double)r.y, rn);
+      }
     }
     if (SLAB && !owned_plane(g, kz)) {  // a ghost plane adds nothing (its values may be anything)
       rz = rz0;
       rn = rn0;
     }
   }
-  double v[3] = {rz, rn, 0.0};
-  grid_reduce<3>(v, red);
+  if (R) {
+    double v[2] = {rz, rn};
+    grid_reduce<2>(v, red);
+  }
 }
 
-int launch_mech_update_on(hpc_ctx* c, int level, double* x, double* r, const double* p, const double* w,
-                          const double* invM, int s_num, int s_den, int s_rz_next, int s_rn) {
+template <typename T, int X, int R>
+static void run_update(hpc_ctx* c, int level, const MechUpdate<T>& a) {
   const LevelGeo& g = c->L[level];
   const long long pairs = (long long)(g.px / 2) * g.ny * g.nz;
   const int grid = (int)std::min<long long>((pairs + kRowThreads - 1) / kRowThreads, (long long)num_sms_v() * 8);
-  const int cls = level == c->maxlevel ? HPC_KC_MECH_UPDATE_FINEST : HPC_KC_NONE;
-  timing_begin(c, cls);
+  const RedTarget red = R ? make_red(c, R == 1 ? a.s_rz_next : -1, a.s_rn, -1) : RedTarget{nullptr, nullptr, c->scal, {-1, -1, -1}};
   if (c->slab)
-    mech_update_kernel<double, true><<<grid, kRowThreads, 0, c->stream>>>(g, x, r, p, w, invM, s_num, s_den,
-                                                                        make_red(c, s_rz_next, s_rn, -1));
+    mech_update_kernel<T, true, X, R><<<grid, kRowThreads, 0, c->stream>>>(g, a, red);
   else
-    mech_update_kernel<double, false><<<grid, kRowThreads, 0, c->stream>>>(g, x, r, p, w, invM, s_num, s_den,
-                                                                         make_red(c, s_rz_next, s_rn, -1));
+    mech_update_kernel<T, false, X, R><<<grid, kRowThreads, 0, c->stream>>>(g, a, red);
+}
+template <typename T>
+int launch_mech_update(hpc_ctx* c, int level, const MechUpdate<T>& a) {
+  const int cls = sizeof(T) == 8 && level == c->maxlevel ? HPC_KC_MECH_UPDATE_FINEST : HPC_KC_NONE;
+  timing_begin(c, cls);
+  if (a.r_old) run_update<T, 1, 2>(c, level, a);
+  else if (!a.u) run_update<T, 0, 1>(c, level, a);
+  else if (a.p_prev && a.r) run_update<T, 2, 1>(c, level, a);
+  else if (a.p_prev) run_update<T, 2, 0>(c, level, a);
+  else if (a.r) run_update<T, 1, 1>(c, level, a);
+  else run_update<T, 1, 0>(c, level, a);
   timing_end(c, cls);
   HPC_CHECK_LAUNCH(c);
   return HPC_OK;
 }
-
-int launch_mech_update(hpc_ctx* c, int level, const double* p, int s_rz, int s_pw, int s_rz_next, int s_rn) {
-  const LevelFields& F = c->F[level];
-  return launch_mech_update_on(c, level, F.u, F.ru, p, F.w, F.preMu, s_rz, s_pw, s_rz_next, s_rn);
-}
+template int launch_mech_update(hpc_ctx*, int, const MechUpdate<double>&);
+template int launch_mech_update(hpc_ctx*, int, const MechUpdate<float>&);
 
 // ---------------------------------------------------------------------------------------------
 // Flexible PCG of the precision form: two dot products in one pass, the flexible direction update
@@ -139,16 +196,22 @@ int launch_mech_update(hpc_ctx* c, int level, const double* p, int s_rz, int s_p
 // sums are the same bits without the conversion pass).
 template <typename TA>
 __global__ void dot2_kernel(LevelGeo g, const TA* a, const double* b, const double* cv, RedTarget red) {
+  using A2 = typename Vec2<TA>::type;
   double s0 = 0.0, s1 = 0.0;
-  FOR_NODES(g) {
+  FOR_PAIRS(g) {
     if (!owned_plane(g, kz)) continue;
-    const long long n = nidx(g, i, j, kz);
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       const long long o = n + (long long)m * g.n;
-      const double av = (double)a[o];
-      s0 = fma(av, b[o], s0);
-      if (cv) s1 = fma(av, cv[o], s1);
+      const A2 av = *reinterpret_cast<const A2*>(a + o);
+      const double2 bv = *reinterpret_cast<const double2*>(b + o);
+      s0 = fma((double)av.x, bv.x, s0);
+      if (i + 1 < g.nx) s0 = fma((double)av.y, bv.y, s0);
+      if (cv) {
+        const double2 c2 = *reinterpret_cast<const double2*>(cv + o);
+        s1 = fma((double)av.x, c2.x, s1);
+        if (i + 1 < g.nx) s1 = fma((double)av.y, c2.y, s1);
+      }
     }
   }
   double v[2] = {s0, s1};
@@ -158,7 +221,7 @@ __global__ void dot2_kernel(LevelGeo g, const TA* a, const double* b, const doub
 template <typename TA>
 static int launch_dot2_t(hpc_ctx* c, int level, const TA* a, const double* b, const double* cv, int s0, int s1) {
   const LevelGeo& g = c->L[level];
-  dot2_kernel<TA><<<row_grid(g), kRowThreads, 0, c->stream>>>(g, a, b, cv, make_red(c, s0, cv ? s1 : -1, -1));
+  dot2_kernel<TA><<<pair_grid(g), kRowThreads, 0, c->stream>>>(g, a, b, cv, make_red(c, s0, cv ? s1 : -1, -1));
   HPC_CHECK_LAUNCH(c);
   return HPC_OK;
 }
@@ -172,14 +235,23 @@ int launch_dot2(hpc_ctx* c, int level, const float* a, const double* b, const do
 template <typename TZ>
 __global__ void fcg_dir_kernel(LevelGeo g, const TZ* z, double* p, int first, const double* scal, int s_delta,
                                int s_gamma, int s_delta_prev) {
+  using Z2 = typename Vec2<TZ>::type;
   const double beta = first ? 0.0 : (scal[s_delta] - scal[s_gamma]) / scal[s_delta_prev];
-  FOR_NODES(g) {
-    const long long n = nidx(g, i, j, kz);
+  FOR_PAIRS(g) {
+    Z2 zv[3];  // every load before the first store
+    double2 pv[3];
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       const long long o = n + (long long)m * g.n;
-      const double zv = (double)z[o];
-      p[o] = first ? zv : fma(beta, p[o], zv);
+      zv[m] = *reinterpret_cast<const Z2*>(z + o);
+      if (!first) pv[m] = *reinterpret_cast<const double2*>(p + o);
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      double2 v{(double)zv[m].x, (double)zv[m].y};
+      if (!first) v = double2{fma(beta, pv[m].x, v.x), fma(beta, pv[m].y, v.y)};
+      if (i + 1 >= g.nx) v.y = 0.0;  // padding slots stay zero
+      *reinterpret_cast<double2*>(p + n + (long long)m * g.n) = v;
     }
   }
 }
@@ -188,7 +260,7 @@ template <typename TZ>
 static int launch_fcg_dir_t(hpc_ctx* c, int level, const TZ* z, double* p, bool first, int s_delta, int s_gamma,
                             int s_delta_prev) {
   const LevelGeo& g = c->L[level];
-  fcg_dir_kernel<TZ><<<row_grid(g), kRowThreads, 0, c->stream>>>(g, z, p, first ? 1 : 0, c->scal, s_delta, s_gamma,
+  fcg_dir_kernel<TZ><<<pair_grid(g), kRowThreads, 0, c->stream>>>(g, z, p, first ? 1 : 0, c->scal, s_delta, s_gamma,
                                                                 s_delta_prev);
   HPC_CHECK_LAUNCH(c);
   HPC_SLAB_HALO(c, level, p, 3, sizeof(double));  // the apply of p reads its ghost planes
@@ -512,8 +584,10 @@ __global__ void prolong_kernel(LevelGeo gc, LevelGeo gf, const T* uc, const T* u
       b0 = bc_flags(gf, 2 * i, j, kz);
       if (odd) b1 = bc_flags(gf, 2 * i + 1, j, kz);
     }
+    V2 fv[NC], add[NC];  // every load before the first store
 #pragma unroll
     for (int m = 0; m < NC; ++m) {
+      fv[m] = *reinterpret_cast<const V2*>(uf + nf + m * gf.n);
       const T* a = uc + m * gc.n;
       const T* o = ucold + m * gc.n;
       auto E = [&](long long n) -> T { return a[n] - o[n]; };
@@ -533,9 +607,13 @@ __global__ void prolong_kernel(LevelGeo gc, LevelGeo gf, const T* uc, const T* u
         add0 = T(0.25) * (l000 + lyz + lz + ly);
         add1 = T(0.125) * (r000 + ry + l000 + ly + rz + lz + ryz + lyz);
       }
-      V2 v = *reinterpret_cast<const V2*>(uf + nf + m * gf.n);
-      v.x += add0;
-      if (odd) v.y += add1;
+      add[m] = V2{add0, add1};
+    }
+#pragma unroll
+    for (int m = 0; m < NC; ++m) {
+      V2 v = fv[m];
+      v.x += add[m].x;
+      if (odd) v.y += add[m].y;
       if (apply_bc) {
         if (m == 0 && b0.c0) v.x = T(0);
         if (m == 0 && b1.c0) v.y = T(0);
@@ -547,11 +625,6 @@ __global__ void prolong_kernel(LevelGeo gc, LevelGeo gf, const T* uc, const T* u
       *reinterpret_cast<V2*>(uf + nf + m * gf.n) = v;
     }
   }
-}
-// Threads of a kernel over the node pairs of a level.
-static int pair_grid(const LevelGeo& g) {
-  const long long pairs = (long long)((g.nx + 1) / 2) * g.ny * g.nz;
-  return (int)std::min<long long>((pairs + kRowThreads - 1) / kRowThreads, (long long)num_sms_v() * 8);
 }
 int launch_prolong(hpc_ctx* c, int lf, const double* uc, const double* ucold, double* uf, int ncomp, bool apply_bc,
                    double Ut) {
@@ -1041,20 +1114,6 @@ int launch_to_f64(hpc_ctx* c, const float* src, double* dst, long long n) {
   return HPC_OK;
 }
 
-int launch_mech_update_f32(hpc_ctx* c, int level, const float* p, int s_num, int s_den, int s_rz_next, int s_rn) {
-  const LevelGeo& g = c->L[level];
-  const LevelF32& F = c->F32[level];
-  const long long pairs = (long long)(g.px / 2) * g.ny * g.nz;
-  const int grid = (int)std::min<long long>((pairs + kRowThreads - 1) / kRowThreads, (long long)num_sms_v() * 8);
-  if (c->slab)
-    mech_update_kernel<float, true><<<grid, kRowThreads, 0, c->stream>>>(g, F.u, F.ru, p, F.w, F.invM, s_num, s_den,
-                                                                       make_red(c, s_rz_next, s_rn, -1));
-  else
-    mech_update_kernel<float, false><<<grid, kRowThreads, 0, c->stream>>>(g, F.u, F.ru, p, F.w, F.invM, s_num,
-                                                                        s_den, make_red(c, s_rz_next, s_rn, -1));
-  HPC_CHECK_LAUNCH(c);
-  return HPC_OK;
-}
 int launch_dir_update_f32(hpc_ctx* c, int level, bool first, int s_rz, int s_rz_prev) {
   const LevelGeo& g = c->L[level];
   const LevelF32& F = c->F32[level];
@@ -1074,39 +1133,62 @@ int launch_prolong_f32(hpc_ctx* c, int lf) {
 }  // namespace hpc
 
 namespace hpc {
-// The residual of the correction problem when its unknown is still zero: r = f with Dirichlet rows
-// zero, (r, M^-1 r) into a slot - the first residual of the precision form's finest pre-smoother,
-// without an operator apply.
-__global__ void residual_zero_f32_kernel(LevelGeo g, const float* f, const float* invM, float* r, RedTarget red) {
+// The start of a V-cycle as preconditioner, whose unknown is still zero: f = the outer residual, in the
+// cycle's precision; its first residual r = f with Dirichlet rows zero, without an operator apply; (r, M^-1 r)
+// into a slot.  One pass instead of a copy, a fill of u and another pass (FP64: and an apply of zeros).
+template <typename T>
+__global__ void zero_start_kernel(LevelGeo g, const double* src, const T* invM, T* f, T* r, RedTarget red) {
+  using V2 = typename Vec2<T>::type;
   double rz = 0.0;
-  FOR_NODES(g) {
-    const long long n = nidx(g, i, j, kz);
-    bool fix[3] = {false, false, false};
+  FOR_PAIRS(g) {
+    bool fix[2][3] = {{false, false, false}, {false, false, false}};
     if (g.bz[kz]) {
-      const BcFlags bc = bc_flags(g, i, j, kz);
-      fix[0] = bc.c0;
-      fix[1] = bc.c1;
-      fix[2] = bc.c2;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (i + h < g.nx) {
+          const BcFlags bc = bc_flags(g, i + h, j, kz);
+          fix[h][0] = bc.c0;
+          fix[h][1] = bc.c1;
+          fix[h][2] = bc.c2;
+        }
+    }
+    const bool own = owned_plane(g, kz);
+    double2 sv[3];
+    V2 mvs[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const long long o = n + (long long)m * g.n;
+      sv[m] = *reinterpret_cast<const double2*>(src + o);
+      mvs[m] = *reinterpret_cast<const V2*>(invM + o);
     }
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       const long long o = n + (long long)m * g.n;
-      const float rv = fix[m] ? 0.f : f[o];
-      r[o] = rv;
-      const double s1 = fma((double)rv, (double)(rv * invM[o]), rz);
-      rz = owned_plane(g, kz) ? s1 : rz;
+      const V2 fv{(T)sv[m].x, (T)sv[m].y};
+      const V2 rv{fix[0][m] ? T(0) : fv.x, fix[1][m] ? T(0) : fv.y};
+      const V2 mv = mvs[m];
+      *reinterpret_cast<V2*>(f + o) = fv;
+      *reinterpret_cast<V2*>(r + o) = rv;
+      const double s0 = fma((double)rv.x, (double)(rv.x * mv.x), rz), s1 = fma((double)rv.y, (double)(rv.y * mv.y), s0);
+      rz = own ? s1 : rz;
     }
   }
   double v[1] = {rz};
   grid_reduce<1>(v, red);
 }
-
-int launch_residual_zero_f32(hpc_ctx* c, int level, int s_rz) {
-  const LevelGeo& g = c->L[level];
-  const LevelF32& F = c->F32[level];
-  residual_zero_f32_kernel<<<row_grid(g), kRowThreads, 0, c->stream>>>(g, F.fu, F.invM, F.ru,
-                                                                       make_red(c, s_rz, -1, -1));
+template <typename T>
+static int run_zero_start(hpc_ctx* c, int level, const double* src, const T* invM, T* f, T* r, int s_rz) {
+  zero_start_kernel<T><<<pair_grid(c->L[level]), kRowThreads, 0, c->stream>>>(c->L[level], src, invM, f, r,
+                                                                             make_red(c, s_rz, -1, -1));
   HPC_CHECK_LAUNCH(c);
   return HPC_OK;
+}
+int launch_zero_start(hpc_ctx* c, int level, const double* src, int s_rz) {
+  const LevelFields& F = c->F[level];
+  return run_zero_start(c, level, src, F.preMu, F.fu, F.ru, s_rz);
+}
+int launch_zero_start_f32(hpc_ctx* c, int level, const double* src, int s_rz) {
+  const LevelF32& F = c->F32[level];
+  return run_zero_start(c, level, src, F.invM, F.fu, F.ru, s_rz);
 }
 }  // namespace hpc
