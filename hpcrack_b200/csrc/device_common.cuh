@@ -128,14 +128,16 @@ __device__ __forceinline__ bool owned_plane(const LevelGeo& g, int k) { return k
 struct BcFlags {
   bool c0, c1, c2, top;
 };
-__device__ __forceinline__ BcFlags bc_flags(const LevelGeo& g, int i, int j, int k) {
-  const uint8_t fx = g.bx[i], fy = g.by[j], fz = g.bz[k];
+__device__ __forceinline__ BcFlags bc_flags_of(uint8_t fx, uint8_t fy, uint8_t fz) {
   BcFlags b;
   b.c0 = (fz & 1) && (fx & 1) && (fy & 1);  // z == za && x == (xa+xb)/2 && y == ya
   b.c1 = (fz & 1) && (fx & 2) && (fy & 2);  // z == za && x == xb && y == (ya+yb)/2
   b.c2 = (fz & 3) != 0;                     // z == za || z == zb
   b.top = (fz & 2) != 0;                    // z == zb (the later assignment wins: Ut)
   return b;
+}
+__device__ __forceinline__ BcFlags bc_flags(const LevelGeo& g, int i, int j, int k) {
+  return bc_flags_of(g.bx[i], g.by[j], g.bz[k]);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -48,18 +48,18 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 
 // What a kernel does with the finished operator row tot of node (x, ey, kk), by epilogue; own_p is the
 // applied vector at the node (EPI_PCG); pre_f and pre_m are f and (where k.invM is set) M^-1 at the node
-// (EPI_RESIDUAL), or pre_f what out holds there and pre_m M^-1 (EPI_FAS).
+// (EPI_RESIDUAL), or pre_f what out holds there and pre_m M^-1 (EPI_FAS); bc
+// the node's Dirichlet flags (those three and EPI_REACTION).
 template <typename T, int EPI>
 __device__ __forceinline__ void node_epilogue(const MechKT<T>& k, int x, int ey, int kk, const T (&tot)[3],
                                               const T (&own_p)[3], const T (&pre_f)[3], const T (&pre_m)[3],
-                                              double& red0, double& red1, double& red2) {
+                                              const BcFlags& bc, double& red0, double& red1, double& red2) {
   const long long n = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
   const long long N = k.g.n;
   if (EPI == EPI_PLAIN) {
 #pragma unroll
     for (int m = 0; m < 3; ++m) k.out[n + m * N] = tot[m];
   } else if (EPI == EPI_RESIDUAL) {
-    const BcFlags bc = bc_flags(k.g, x, ey, kk);
     const bool fix[3] = {bc.c0, bc.c1, bc.c2};
     // a slab's ghost planes keep the sums as they are (a select: ghost values may be anything)
     const bool own = owned_plane(k.g, kk);
@@ -96,7 +96,6 @@ __device__ __forceinline__ void node_epilogue(const MechKT<T>& k, int x, int ey,
   } else if (EPI == EPI_FAS) {
     // the second half of coarsen_fu: out holds the full weighting of the fine residual.  With r_out that is
     // also the first residual of the coarse smoother, f - K u for the injected u
-    const BcFlags bc = bc_flags(k.g, x, ey, kk);
     const bool fix[3] = {bc.c0, bc.c1, bc.c2};
     const bool own = owned_plane(k.g, kk);
 #pragma unroll
@@ -111,7 +110,6 @@ __device__ __forceinline__ void node_epilogue(const MechKT<T>& k, int x, int ey,
     }
   } else if (EPI == EPI_REACTION) {
     // Dirichlet_force_u (boundary_conditions.cpp:69-111)
-    const BcFlags bc = bc_flags(k.g, x, ey, kk);
     if (bc.c0) k.out[n] = tot[0];
     if (bc.c1) k.out[n + N] = tot[1];
     if (bc.c2) k.out[n + 2 * N] = tot[2];

@@ -212,7 +212,8 @@ __device__ __forceinline__ void assemble_row(const MechKT<T>& k, const ST& st, i
           if (k.invM) pre_m[m] = k.invM[n + m * k.g.n];
         }
       }
-      node_epilogue<T, EPI>(k, x, ey, kk, tot, own_p, pre_f, pre_m, red0, red1, red2);
+      const BcFlags bc = EPI == EPI_PCG || EPI == EPI_PLAIN ? BcFlags{} : bc_flags(k.g, x, ey, kk);
+      node_epilogue<T, EPI>(k, x, ey, kk, tot, own_p, pre_f, pre_m, bc, red0, red1, red2);
     }
   }
 #pragma unroll

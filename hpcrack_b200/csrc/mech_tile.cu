@@ -22,7 +22,13 @@
 // tile that owns a node writes the new direction (into the other of two arrays: neighbours still read the
 // old one).  That replaces a pass of 96 (48) bytes a node and its launch: an iteration's apply and
 // direction take 842 us on 257^3 in FP64 against 656 + 250, 532 us in FP32 against 401 + 125, and one
-// launch less where launches count; increments -1 to -5 %.
+// launch less where launches count; increments -1 to -5 %.  A plane is formed in units of 16 bytes, one
+// (FP32) or two (FP64) a thread; single nodes took 4 rounds of loads, masks and stores.
+//
+// The residual's f and M^-1 are staged the same way, and the Dirichlet flags read ahead.  As loads of each
+// thread from global memory they came due at the end of the layer they were issued in, which is shorter than
+// DRAM's latency under load: 935 us a residual on 257^3 in FP64, 591 in FP32.  Both changes: increments of
+// 257^3 1300 -> 1268 ms (FAS, crack), 358 -> 349 (precision form), 257x129x65 154 -> 149, 129^3 18.8 -> 18.55.
 //
 // What bounds it: FP64, the FP64 pipe (66 % of its cycles on 193^3; two warps per scheduler cannot hide
 // all dependent latencies); FP32, instruction issue (80 % of the slots).  Per launch on B200, with the
@@ -67,18 +73,21 @@ constexpr int kTX = kTileX;  // element columns of a tile in x: a half-warp, 128
 constexpr unsigned kTileWaitPolls = 1u << 24;  // far above any copy's latency; then the kernel reports
 
 // Columns staged per row: the 17 nodes of a tile plus the offset to the copy's 16-byte aligned start.
+template <typename T> struct TileVec;
+template <> struct TileVec<double> { using type = double2; };
+template <> struct TileVec<float> { using type = float4; };
 template <typename T> struct TileRow;
 template <> struct TileRow<double> { static constexpr int BX = 18; };
 template <> struct TileRow<float> { static constexpr int BX = 20; };
 
 // Shared memory of a block: [0, 128) the stages' mbarriers; the stages' node planes and (finest) moduli
 // layers; the y exchange.
-// DIR: a stage also holds the planes of r and M^-1 the direction is formed from.
-template <typename T, bool GPM, int TY, int NS, bool DIR>
+// EX: a stage also holds two more planes: r and M^-1 the direction is formed from, or the residual's f and M^-1.
+template <typename T, bool GPM, int TY, int NS, bool EX>
 struct TileSmem {
   static constexpr int BX = TileRow<T>::BX, NT = kTX * TY, XP = 20;  // XP: exchange row pitch (bank spread)
   static constexpr size_t up(size_t b) { return (b + 127) / 128 * 128; }
-  static constexpr size_t plane = up(sizeof(T) * 3 * (TY + 1) * BX), node = plane * (DIR ? 3 : 1), mod = GPM ? up(sizeof(T) * 16 * TY * BX) : 0;
+  static constexpr size_t plane = up(sizeof(T) * 3 * (TY + 1) * BX), node = plane * (EX ? 3 : 1), mod = GPM ? up(sizeof(T) * 16 * TY * BX) : 0;
   static constexpr size_t o_node = 128, o_mod = o_node + NS * node, o_exch = o_mod + NS * mod;
   static constexpr size_t total = o_exch + sizeof(T) * 2 * 3 * TY * XP;
   static constexpr size_t bytes = total + 128;  // + alignment of the dynamic base
@@ -90,6 +99,7 @@ struct TileSmem {
 template <typename T>
 struct PlaneState {
   T ex[3][2], dy[3][2], iy[3][4], aex[3][2], ady[3][2], sz[3][4], own[3];
+  T f[3], im[3];  // residual: f and M^-1 at the thread's own node
 };
 
 // In-plane part of one node plane, per component: ex[p] = d/dx at in-plane Gauss row p, dy[q] = d/dy at
@@ -128,7 +138,8 @@ __device__ __forceinline__ void plane_adjoint(const T (&ex)[2], const T (&dy)[2]
 
 template <typename T, bool GPM, int EPI, bool ISO, bool TMA, int TY, int MINB, int NS, bool DIR>
 __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_constant__ MechKT<T> k) {
-  using S = TileSmem<T, GPM, TY, NS, DIR>;
+  constexpr bool RES = EPI == EPI_RESIDUAL, EX = DIR || RES;
+  using S = TileSmem<T, GPM, TY, NS, EX>;
   constexpr int BX = S::BX, NT = S::NT, NY = TY + 1;
   extern __shared__ __align__(128) unsigned char tile_smem[];
   unsigned char* base = tile_smem + ((128u - (smem_u32(tile_smem) & 127u)) & 127u);
@@ -166,6 +177,8 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
   const int off = (x0 - 1) - xs;
   const bool xy_elem = x >= 0 && x <= k.g.nx - 2 && y >= 0 && y <= k.g.ny - 2;
   const bool out_node = tx >= 1 && row >= 1 && x < k.g.nx && y < k.g.ny;
+  constexpr bool BC = EPI != EPI_PCG && EPI != EPI_PLAIN;  // Dirichlet flags wanted
+  const uint8_t fx = BC && out_node ? k.g.bx[x] : 0, fy = BC && out_node ? k.g.by[y] : 0;
 
   auto node_slot = [&](int j) {
     return reinterpret_cast<T*>(base + S::o_node + (size_t)((unsigned)j % NS) * S::node);
@@ -181,8 +194,9 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
         if (tid == 0) {
           const uint32_t bar = smem_u32(bars + (unsigned)j % NS);
           const bool mods = GPM && j >= 1;
-          const bool old = !DIR || !k.dir_first;
-          const int bytes = (int)sizeof(T) * BX * (3 * NY * ((DIR ? 2 : 0) + (old ? 1 : 0)) + (mods ? 16 * TY : 0));
+          const bool old = !DIR || !k.dir_first, minv = EX && k.dir_m;
+          const int planes = (old ? 1 : 0) + (EX ? 1 : 0) + (minv ? 1 : 0);
+          const int bytes = (int)sizeof(T) * BX * (3 * NY * planes + (mods ? 16 * TY : 0));
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
           auto copy = [&](const CUtensorMap* map, T* dst) {
@@ -193,9 +207,9 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
                 : "memory");
           };
           if (old) copy(&k.tmap, node_slot(j));
-          if constexpr (DIR) {
+          if constexpr (EX) {
             copy(&k.rmap, node_slot(j) + S::plane / sizeof(T));
-            copy(&k.mmap, node_slot(j) + 2 * (S::plane / sizeof(T)));
+            if (minv) copy(&k.mmap, node_slot(j) + 2 * (S::plane / sizeof(T)));
           }
           if (mods)
             asm volatile(
@@ -206,8 +220,8 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
         }
       } else {
         // the nodes of a row one column apart, zeros outside the grid
-        for (int f = 0; f < (DIR ? 3 : 1); ++f) {
-          if (f == 0 && DIR && k.dir_first) continue;
+        for (int f = 0; f < (EX ? 3 : 1); ++f) {
+          if ((f == 0 && DIR && k.dir_first) || (f == 2 && !k.dir_m)) continue;
           T* dst = node_slot(j) + f * (S::plane / sizeof(T));
           for (int q = tid; q < 3 * NY * 17; q += NT) {
             const int c = q % 17, r = q / 17, ry = r % NY, m = r / NY;
@@ -258,22 +272,34 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
       return true;
     }
   };
-  // DIR: the direction at this thread's share of a staged plane's nodes, in place of p_old (0 beyond the
-  // grid's last column, where p_old's padding may hold anything)
-  constexpr int CN = 3 * NY * 17, CT = DIR ? (CN + NT - 1) / NT : 1;
-  int c_at[CT];
+  // DIR: the direction at this thread's share of a staged plane, 16 bytes at a time, in place of p_old (0 beyond
+  // the grid's last column, where p_old's padding may hold anything; without tensor copies the columns no
+  // thread reads hold anything too)
+  using V = typename TileVec<T>::type;
+  constexpr int CN = 3 * NY * BX / A16, CT = DIR ? (CN + NT - 1) / NT : 1;  // 16-byte units of a plane
+  static_assert(BX % A16 == 0, "a unit stays in its row");
+  int c_in[CT];  // the unit's columns inside the grid
   T beta = T(0);
   auto form_direction = [&](int j) {
     if constexpr (DIR) {
-      T* p = node_slot(j);
-      const T *r = p + S::plane / sizeof(T), *m = r + S::plane / sizeof(T);
+      V* p = reinterpret_cast<V*>(node_slot(j));
+      const V *r = p + S::plane / sizeof(V), *m = r + S::plane / sizeof(V);
 #pragma unroll
       for (int t = 0; t < CT; ++t) {
-        if (c_at[t] < 0) continue;
-        const int o = c_at[t] & ~(1 << 30);
-        const T z = r[o] * m[o];
-        const T v = k.dir_first ? z : fma(beta, p[o], z);
-        p[o] = (c_at[t] & (1 << 30)) ? T(0) : v;
+        const int q = tid + t * NT;
+        if (CN % NT != 0 && q >= CN) continue;
+        const V rv = r[q], mv = m[q];
+        V pv{};
+        if (!k.dir_first) pv = p[q];
+        T *pe = reinterpret_cast<T*>(&pv);
+        const T *re = reinterpret_cast<const T*>(&rv), *me = reinterpret_cast<const T*>(&mv);
+#pragma unroll
+        for (int e = 0; e < A16; ++e) {
+          const T z = re[e] * me[e];
+          const T v = k.dir_first ? z : fma(beta, pe[e], z);
+          pe[e] = e < c_in[t] ? v : T(0);
+        }
+        p[q] = pv;
       }
       if (TMA) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next copy overwrites this plane
     }
@@ -296,14 +322,22 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
     const int kk = z0 - 1 + li;
     const T lam_c = lam_n, G_c = G_n;
     if (!GPM) coarse_mod(kk + 1);
-    // the residual's f and M^-1 of this plane's node (FAS: what out holds): in flight under the arithmetic
+    const uint8_t fz = BC && out_node && kk >= z0 ? k.g.bz[kk] : 0;
+    // FAS: what out holds at this plane's node, in flight under the arithmetic
     T pre_f[3], pre_m[3];
-    if ((EPI == EPI_RESIDUAL || EPI == EPI_FAS) && out_node && kk >= z0) {
+    if (EPI == EPI_FAS && out_node && kk >= z0) {
       const long long n = (long long)x + (long long)y * k.g.px + (long long)kk * k.g.plane;
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
-        pre_f[m] = EPI == EPI_FAS ? k.out[n + m * k.g.n] : k.fu[n + m * k.g.n];
+        pre_f[m] = k.out[n + m * k.g.n];
         pre_m[m] = k.invM ? k.invM[n + m * k.g.n] : T(0);
+      }
+    }
+    if constexpr (RES) {  // staged with this plane, read when it was the upper one
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        pre_f[m] = a.f[m];
+        pre_m[m] = a.im[m];
       }
     }
     if (!DIR && !wait(li + 1)) bad = 1;
@@ -316,6 +350,10 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
         const T v[4] = {nd[m * NY * BX], nd[m * NY * BX + 1], nd[m * NY * BX + BX], nd[m * NY * BX + BX + 1]};
         plane_forward(v, s.t, b.ex[m], b.dy[m], b.iy[m]);
         b.own[m] = v[0];
+        if constexpr (RES) {
+          b.f[m] = nd[S::plane / sizeof(T) + m * NY * BX];
+          b.im[m] = k.dir_m ? nd[2 * (S::plane / sizeof(T)) + m * NY * BX] : T(0);
+        }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           gz[m][q] = b.iy[m][q] - a.iy[m][q];
@@ -401,7 +439,7 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
       T tot[3];
 #pragma unroll
       for (int m = 0; m < 3; ++m) tot[m] = X0[m] + ex_w[m * TY * S::XP - S::XP];
-      node_epilogue<T, EPI>(k, x, y, kk, tot, a.own, pre_f, pre_m, red0, red1, red2);
+      node_epilogue<T, EPI>(k, x, y, kk, tot, a.own, pre_f, pre_m, bc_flags_of(fx, fy, fz), red0, red1, red2);
       if constexpr (DIR) {
         const long long n = (long long)x + (long long)y * k.g.px + (long long)kk * k.g.plane;
 #pragma unroll
@@ -416,11 +454,7 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
   if constexpr (DIR) {  // under the first copies
     if (!k.dir_first) beta = (T)(k.red.scal[k.s_rz] / k.red.scal[k.s_rz_prev]);
 #pragma unroll
-    for (int t = 0; t < CT; ++t) {
-      const int q = tid + t * NT;
-      c_at[t] = q < CN ? (q / 17) * BX + off + q % 17 : -1;
-      if (q < CN && x0 - 1 + q % 17 >= k.g.nx) c_at[t] |= 1 << 30;
-    }
+    for (int t = 0; t < CT; ++t) c_in[t] = k.g.nx - (xs + (tid + t * NT) % (BX / A16) * A16);
   }
   coarse_mod(z0 - 1);
   PlaneState<T> a, b;
@@ -474,7 +508,12 @@ template <> struct TileShape<float> { static constexpr int TY = 16, MINB = 2, NS
 template <typename T, bool GPM, int EPI, bool ISO, bool TMA, bool DIR>
 int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
   constexpr int TY = TileShape<T>::TY, NS = TileShape<T>::NS;
-  using S = TileSmem<T, GPM, TY, NS, DIR>;
+  constexpr bool EX = DIR || EPI == EPI_RESIDUAL;
+  using S = TileSmem<T, GPM, TY, NS, EX>;
+  if (EPI == EPI_RESIDUAL) {
+    k.dir_r = k.fu;
+    k.dir_m = k.invM;
+  }
   auto kern = mech_tile_kernel<T, GPM, EPI, ISO, TMA, TY, TileShape<T>::MINB, NS, DIR>;
   int per_sm = 1, rc;
   if ((rc = kernel_cfg((const void*)kern, S::bytes, S::bytes, kTX * TY, &per_sm))) return rc;
@@ -482,8 +521,8 @@ int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
   if ((size_t)k.sg.nstrips * 3 > c->partials_cap) return cuda_fail(cudaErrorInvalidValue, "partials buffer");
   if constexpr (TMA) {
     if ((rc = encode_tensor<T>(k.g, k.fields[0], 3, S::BX, TY + 1, 1, &k.tmap))) return rc;
-    if (DIR && ((rc = encode_tensor<T>(k.g, k.dir_r, 3, S::BX, TY + 1, 1, &k.rmap)) ||
-                (rc = encode_tensor<T>(k.g, k.dir_m, 3, S::BX, TY + 1, 1, &k.mmap))))
+    if (EX && ((rc = encode_tensor<T>(k.g, k.dir_r, 3, S::BX, TY + 1, 1, &k.rmap)) ||
+               (k.dir_m && (rc = encode_tensor<T>(k.g, k.dir_m, 3, S::BX, TY + 1, 1, &k.mmap)))))
       return rc;
     if (GPM && (rc = encode_tensor<T>(k.g, k.gpm, 16, S::BX, TY, 1, &k.gmap))) return rc;
   }
