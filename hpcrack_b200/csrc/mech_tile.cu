@@ -35,10 +35,13 @@
 // element-by-element strip kernel it replaced in brackets: 257^3 FP64 656 us (1043), FP32 401 us (759);
 // 129^3 109 (196), 68 (151); 65^3 28 (63), 21 (53); 33^3 16 (25), 15 (23).  At 176 (88) bytes a node the
 // 257^3 applies move 4.6 (3.7) TB/s.
+// Coarse levels with equal spacing work in sum/difference modes (ModeState): fewer operations, fewer registers, 3
+// blocks per SM in FP64.  What bounds a level of 33^3 to 65^3 is the march itself, 6 to 10 dependent layers.
 // Every node is written once, by the tile that owns it, with the same arithmetic wherever tile and
 // chunk boundaries fall: no atomics, deterministic, independent of the chunk height except for the
 // order of the reductions.
 #include <algorithm>
+#include <type_traits>
 
 #include "element_common.cuh"
 
@@ -102,6 +105,34 @@ struct PlaneState {
   T f[3], im[3];  // residual: f and M^-1 at the thread's own node
 };
 
+// The same where moduli are element-constant and the spacing is equal (the coarse levels): in the
+// sum/difference modes of mech_modes a plane's part is its 4 nodes (v) and its in-plane modes x, y and xy (h) on
+// the way in, and the lower layer's share of the modes (acc) on the way out.  About 160 operations an element
+// instead of 365: a PCG apply of 129^3 takes 67 us in FP32 (96), of 65^3 16.5 (21.5).
+template <typename T>
+struct ModeState {
+  T v[3][4], h[3][3], acc[3][4], own[3], f[3], im[3];
+};
+
+// In-plane modes x, y, xy of a component's 4 nodes v[a + 2b].  Differences are taken before sums, here and along
+// z (see haar).
+template <typename T>
+__device__ __forceinline__ void plane_modes(const T (&v)[4], T (&h)[3]) {
+  const T d0 = v[1] - v[0], d1 = v[3] - v[2];
+  h[0] = d0 + d1;
+  h[1] = (v[2] - v[0]) + (v[3] - v[1]);
+  h[2] = d1 - d0;
+}
+// The transpose, with the constant mode h[0].
+template <typename T>
+__device__ __forceinline__ void plane_modes_adjoint(const T (&h)[4], T (&f)[4]) {
+  const T a0 = h[0] - h[2], a1 = h[0] + h[2], b0 = h[1] - h[3], b1 = h[1] + h[3];
+  f[0] = a0 - b0;
+  f[1] = a0 + b0;
+  f[2] = a1 - b1;
+  f[3] = a1 + b1;
+}
+
 // In-plane part of one node plane, per component: ex[p] = d/dx at in-plane Gauss row p, dy[q] = d/dy at
 // Gauss column q, iy[q + 2p] = value.  v[a + 2b] = node (a, b).
 template <typename T>
@@ -138,7 +169,8 @@ __device__ __forceinline__ void plane_adjoint(const T (&ex)[2], const T (&dy)[2]
 
 template <typename T, bool GPM, int EPI, bool ISO, bool TMA, int TY, int MINB, int NS, bool DIR>
 __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_constant__ MechKT<T> k) {
-  constexpr bool RES = EPI == EPI_RESIDUAL, EX = DIR || RES;
+  constexpr bool RES = EPI == EPI_RESIDUAL, EX = DIR || RES, MODES = !GPM && ISO;
+  using State = typename std::conditional<MODES, ModeState<T>, PlaneState<T>>::type;
   using S = TileSmem<T, GPM, TY, NS, EX>;
   constexpr int BX = S::BX, NT = S::NT, NY = TY + 1;
   extern __shared__ __align__(128) unsigned char tile_smem[];
@@ -318,7 +350,7 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
 
   // One element layer li: state a of the node plane below it -> state b of the plane above; the plane
   // below is finished.  False when a wait ran out.
-  auto layer = [&](int li, const PlaneState<T>& a, PlaneState<T>& b) -> bool {
+  auto layer = [&](int li, const State& a, State& b) -> bool {
     const int kk = z0 - 1 + li;
     const T lam_c = lam_n, G_c = G_n;
     if (!GPM) coarse_mod(kk + 1);
@@ -341,92 +373,130 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
       }
     }
     if (!DIR && !wait(li + 1)) bad = 1;
-    // ---- upper node plane: in-plane parts; d/dz between the planes
-    T gz[3][4];
-    {
-      const T* nd = node_slot(li + 1) + row * BX + off + tx;
-#pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        const T v[4] = {nd[m * NY * BX], nd[m * NY * BX + 1], nd[m * NY * BX + BX], nd[m * NY * BX + BX + 1]};
-        plane_forward(v, s.t, b.ex[m], b.dy[m], b.iy[m]);
-        b.own[m] = v[0];
-        if constexpr (RES) {
-          b.f[m] = nd[S::plane / sizeof(T) + m * NY * BX];
-          b.im[m] = k.dir_m ? nd[2 * (S::plane / sizeof(T)) + m * NY * BX] : T(0);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          gz[m][q] = b.iy[m][q] - a.iy[m][q];
-          if (!ISO) gz[m][q] *= s.ih[2];
-        }
-      }
-    }
-    // ---- stresses of the layer by Gauss level r; lo: the lower plane's adjoint with the layer below
-    T lo_ex[3][2], lo_dy[3][2];
-    const T* mod = mod_slot(li + 1) + row * BX + off + tx;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      T gx[3][2], gy[3][2], sx[3][2], sy[3][2];
-#pragma unroll
-      for (int m = 0; m < 3; ++m)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          gx[m][q] = fma(s.t[r], b.ex[m][q] - a.ex[m][q], a.ex[m][q]);
-          gy[m][q] = fma(s.t[r], b.dy[m][q] - a.dy[m][q], a.dy[m][q]);
-          if (!ISO) {
-            gx[m][q] *= s.ih[0];
-            gy[m][q] *= s.ih[1];
-          }
-        }
-#pragma unroll
-      for (int p = 0; p < 2; ++p)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int i = q + 2 * p;
-          const T lam = GPM ? mod[(i + 4 * r) * TY * BX] : lam_c, G = GPM ? mod[(8 + i + 4 * r) * TY * BX] : G_c;
-          const T exx = gx[0][p], eyy = gy[1][q], ezz = gz[2][i];
-          const T lt = lam * (exx + eyy + ezz), G2 = G + G;
-          const T sxy = G * (gx[1][p] + gy[0][q]), sxz = G * (gx[2][p] + gz[0][i]), syz = G * (gy[2][q] + gz[1][i]);
-          const T sxx = fma(G2, exx, lt), syy = fma(G2, eyy, lt), szz = fma(G2, ezz, lt);
-          sx[0][p] = q ? sx[0][p] + sxx : sxx;
-          sx[1][p] = q ? sx[1][p] + sxy : sxy;
-          sx[2][p] = q ? sx[2][p] + sxz : sxz;
-          sy[0][q] = p ? sy[0][q] + sxy : sxy;
-          sy[1][q] = p ? sy[1][q] + syy : syy;
-          sy[2][q] = p ? sy[2][q] + syz : syz;
-          b.sz[0][i] = r ? b.sz[0][i] + sxz : sxz;
-          b.sz[1][i] = r ? b.sz[1][i] + syz : syz;
-          b.sz[2][i] = r ? b.sz[2][i] + szz : szz;
-        }
-#pragma unroll
-      for (int m = 0; m < 3; ++m)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          if (!ISO) {
-            sx[m][q] *= s.ih[0];
-            sy[m][q] *= s.ih[1];
-          }
-          // 1 - t[r] = t[1 - r]
-          lo_ex[m][q] = fma(s.t[1 - r], sx[m][q], r ? lo_ex[m][q] : a.aex[m][q]);
-          lo_dy[m][q] = fma(s.t[1 - r], sy[m][q], r ? lo_dy[m][q] : a.ady[m][q]);
-          b.aex[m][q] = r ? fma(s.t[1], sx[m][q], b.aex[m][q]) : s.t[0] * sx[m][q];
-          b.ady[m][q] = r ? fma(s.t[1], sy[m][q], b.ady[m][q]) : s.t[0] * sy[m][q];
-        }
-    }
-    // ---- lower plane finished: back to its nodes, x-neighbours by shuffle, y-neighbours by exchange
     T X0[3];
     T* ex_w = exch + (size_t)(li & 1) * 3 * TY * S::XP + row * S::XP + tx;
+    const T* nd = node_slot(li + 1) + row * BX + off + tx;
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      T iy[4], f[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (!ISO) b.sz[m][q] *= s.ih[2];
-        iy[q] = a.sz[m][q] - b.sz[m][q];
+      b.own[m] = nd[m * NY * BX];
+      if constexpr (RES) {
+        b.f[m] = nd[S::plane / sizeof(T) + m * NY * BX];
+        b.im[m] = k.dir_m ? nd[2 * (S::plane / sizeof(T)) + m * NY * BX] : T(0);
       }
-      plane_adjoint(lo_ex[m], lo_dy[m], iy, s.t, f);
+    }
+    auto combine = [&](int m, const T(&f)[4]) {  // x-neighbours by shuffle, y-neighbours by exchange
       X0[m] = f[0] + __shfl_up_sync(kFull, f[1], 1, kTX);
       ex_w[m * TY * S::XP] = f[2] + __shfl_up_sync(kFull, f[3], 1, kTX);
+    };
+    if constexpr (MODES) {
+      T M[3][8];
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        b.v[m][0] = b.own[m];
+        b.v[m][1] = nd[m * NY * BX + 1];
+        b.v[m][2] = nd[m * NY * BX + BX];
+        b.v[m][3] = nd[m * NY * BX + BX + 1];
+        plane_modes(b.v[m], b.h[m]);
+        M[m][4] = ((b.v[m][0] - a.v[m][0]) + (b.v[m][1] - a.v[m][1])) + ((b.v[m][2] - a.v[m][2]) + (b.v[m][3] - a.v[m][3]));
+#pragma unroll
+        for (int q = 1; q < 4; ++q) {
+          M[m][q] = a.h[m][q - 1] + b.h[m][q - 1];
+          M[m][4 + q] = b.h[m][q - 1] - a.h[m][q - 1];
+        }
+      }
+      mech_modes(M, lam_c, G_c);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        T lo[4], f[4];
+        lo[0] = a.acc[m][0] - M[m][4];
+        b.acc[m][0] = M[m][4];
+#pragma unroll
+        for (int q = 1; q < 4; ++q) {
+          lo[q] = a.acc[m][q] + (M[m][q] - M[m][4 + q]);
+          b.acc[m][q] = M[m][q] + M[m][4 + q];
+        }
+        plane_modes_adjoint(lo, f);
+        combine(m, f);
+      }
+    } else {
+      // ---- upper node plane: in-plane parts; d/dz between the planes
+      T gz[3][4];
+      {
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          const T v[4] = {b.own[m], nd[m * NY * BX + 1], nd[m * NY * BX + BX], nd[m * NY * BX + BX + 1]};
+          plane_forward(v, s.t, b.ex[m], b.dy[m], b.iy[m]);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            gz[m][q] = b.iy[m][q] - a.iy[m][q];
+            if (!ISO) gz[m][q] *= s.ih[2];
+          }
+        }
+      }
+      // ---- stresses of the layer by Gauss level r; lo: the lower plane's adjoint with the layer below
+      T lo_ex[3][2], lo_dy[3][2];
+      const T* mod = mod_slot(li + 1) + row * BX + off + tx;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        T gx[3][2], gy[3][2], sx[3][2], sy[3][2];
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            gx[m][q] = fma(s.t[r], b.ex[m][q] - a.ex[m][q], a.ex[m][q]);
+            gy[m][q] = fma(s.t[r], b.dy[m][q] - a.dy[m][q], a.dy[m][q]);
+            if (!ISO) {
+              gx[m][q] *= s.ih[0];
+              gy[m][q] *= s.ih[1];
+            }
+          }
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int i = q + 2 * p;
+            const T lam = GPM ? mod[(i + 4 * r) * TY * BX] : lam_c, G = GPM ? mod[(8 + i + 4 * r) * TY * BX] : G_c;
+            const T exx = gx[0][p], eyy = gy[1][q], ezz = gz[2][i];
+            const T lt = lam * (exx + eyy + ezz), G2 = G + G;
+            const T sxy = G * (gx[1][p] + gy[0][q]), sxz = G * (gx[2][p] + gz[0][i]), syz = G * (gy[2][q] + gz[1][i]);
+            const T sxx = fma(G2, exx, lt), syy = fma(G2, eyy, lt), szz = fma(G2, ezz, lt);
+            sx[0][p] = q ? sx[0][p] + sxx : sxx;
+            sx[1][p] = q ? sx[1][p] + sxy : sxy;
+            sx[2][p] = q ? sx[2][p] + sxz : sxz;
+            sy[0][q] = p ? sy[0][q] + sxy : sxy;
+            sy[1][q] = p ? sy[1][q] + syy : syy;
+            sy[2][q] = p ? sy[2][q] + syz : syz;
+            b.sz[0][i] = r ? b.sz[0][i] + sxz : sxz;
+            b.sz[1][i] = r ? b.sz[1][i] + syz : syz;
+            b.sz[2][i] = r ? b.sz[2][i] + szz : szz;
+          }
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            if (!ISO) {
+              sx[m][q] *= s.ih[0];
+              sy[m][q] *= s.ih[1];
+            }
+            // 1 - t[r] = t[1 - r]
+            lo_ex[m][q] = fma(s.t[1 - r], sx[m][q], r ? lo_ex[m][q] : a.aex[m][q]);
+            lo_dy[m][q] = fma(s.t[1 - r], sy[m][q], r ? lo_dy[m][q] : a.ady[m][q]);
+            b.aex[m][q] = r ? fma(s.t[1], sx[m][q], b.aex[m][q]) : s.t[0] * sx[m][q];
+            b.ady[m][q] = r ? fma(s.t[1], sy[m][q], b.ady[m][q]) : s.t[0] * sy[m][q];
+          }
+      }
+      // ---- lower plane finished: back to its nodes
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        T iy[4], f[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (!ISO) b.sz[m][q] *= s.ih[2];
+          iy[q] = a.sz[m][q] - b.sz[m][q];
+        }
+        plane_adjoint(lo_ex[m], lo_dy[m], iy, s.t, f);
+        combine(m, f);
+      }
     }
     if (DIR && li + 2 <= nl) {  // the next layer's upper plane: the barrier publishes it
       if (!wait(li + 2)) bad = 1;
@@ -457,7 +527,7 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
     for (int t = 0; t < CT; ++t) c_in[t] = k.g.nx - (xs + (tid + t * NT) % (BX / A16) * A16);
   }
   coarse_mod(z0 - 1);
-  PlaneState<T> a, b;
+  State a, b;
   if constexpr (DIR) {
     if (TMA && !wait(0)) bad = 1;
     if (!wait(1)) bad = 1;  // cp.async: planes 0 and 1
@@ -472,12 +542,21 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       const T v[4] = {nd[m * NY * BX], nd[m * NY * BX + 1], nd[m * NY * BX + BX], nd[m * NY * BX + BX + 1]};
-      plane_forward(v, s.t, a.ex[m], a.dy[m], a.iy[m]);
       a.own[m] = v[0];
+      if constexpr (MODES) {
+        plane_modes(v, a.h[m]);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) a.sz[m][q] = T(0);
+        for (int q = 0; q < 4; ++q) {
+          a.v[m][q] = v[q];
+          a.acc[m][q] = T(0);
+        }
+      } else {
+        plane_forward(v, s.t, a.ex[m], a.dy[m], a.iy[m]);
 #pragma unroll
-      for (int q = 0; q < 2; ++q) a.aex[m][q] = a.ady[m][q] = T(0);
+        for (int q = 0; q < 4; ++q) a.sz[m][q] = T(0);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) a.aex[m][q] = a.ady[m][q] = T(0);
+      }
     }
   }
   bad = __syncthreads_or(bad);
@@ -501,20 +580,25 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
 // state in shared memory, whose traffic then binds (815 us).  FP32: 16 rows, 2 blocks of 256 threads (125
 // registers); with 8 rows the tiles overlap more (410 against 401 us).  Two stages instead of three cost
 // FP64 7 % (703 against 656 us): a layer's arithmetic is too short to cover the copies.
-template <typename T> struct TileShape;
-template <> struct TileShape<double> { static constexpr int TY = 8, MINB = 2, NS = 3; };
-template <> struct TileShape<float> { static constexpr int TY = 16, MINB = 2, NS = 3; };
+// In modes (coarse levels) FP64 needs 160 registers, so a third block fits: 65^3 FAS increments 5.67 ms against 5.75
+// with 2; in FP32 a third block spills: 97^3 precision form 98.9 ms against 98.2 with 2.
+template <typename T, bool MODES> struct TileShape;
+template <> struct TileShape<double, false> { static constexpr int TY = 8, MINB = 2, NS = 3; };
+template <> struct TileShape<float, false> { static constexpr int TY = 16, MINB = 2, NS = 3; };
+template <> struct TileShape<double, true> { static constexpr int TY = 8, MINB = 3, NS = 3; };
+template <> struct TileShape<float, true> { static constexpr int TY = 16, MINB = 2, NS = 3; };
 
 template <typename T, bool GPM, int EPI, bool ISO, bool TMA, bool DIR>
 int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
-  constexpr int TY = TileShape<T>::TY, NS = TileShape<T>::NS;
+  using Shape = TileShape<T, !GPM && ISO>;
+  constexpr int TY = Shape::TY, NS = Shape::NS;
   constexpr bool EX = DIR || EPI == EPI_RESIDUAL;
   using S = TileSmem<T, GPM, TY, NS, EX>;
   if (EPI == EPI_RESIDUAL) {
     k.dir_r = k.fu;
     k.dir_m = k.invM;
   }
-  auto kern = mech_tile_kernel<T, GPM, EPI, ISO, TMA, TY, TileShape<T>::MINB, NS, DIR>;
+  auto kern = mech_tile_kernel<T, GPM, EPI, ISO, TMA, TY, Shape::MINB, NS, DIR>;
   int per_sm = 1, rc;
   if ((rc = kernel_cfg((const void*)kern, S::bytes, S::bytes, kTX * TY, &per_sm))) return rc;
   k.sg = tile_geo(k.g, TY, (long long)num_sms() * per_sm, (long long)c->partials_cap / 3);
