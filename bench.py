@@ -37,21 +37,20 @@ FALLBACK_HBM_GBS = 6650.0
 # the regime (2) and the result (24) = 74 B/node, the compulsory traffic of y = K(d) u.  The roofline
 # is reported on this basis.  The apply as the mechanical solves run it reads the Gauss-point moduli
 # precomputed once per solve instead of bulK, G, d and the regime: p and w (24 B each) plus K_g, G_g
-# (16 doubles per element = 128 B) = 176 B/node, reported beside it (the kernel trades FP64
+# (16 doubles per element = 128 B) and, with the PCG direction formed on the way, r, M^-1 and the new
+# direction (72 B) = 248 B/node, reported beside it (the kernel trades FP64
 # instructions, its bound, for bytes).
 APPLY_BYTES_PER_NODE = 74
-PCG_APPLY_BYTES_PER_NODE = 176
-# ncu counters of the FP64 apply (one capture of the 193^3 level, the same kernel the bench times):
-# FP64 pipe active 60.7 % of active cycles, issue active 56.1 %, top stall "wait" (fixed-latency
-# dependencies) 1.36 per issued instruction.
-APPLY_FP64_PIPE_ACTIVE = 0.607
+PCG_APPLY_BYTES_PER_NODE = 248
+# ncu counter of the FP64 tile apply (one capture of the 193^3 level, without the direction): FP64 pipe
+# active 66 % of active cycles.
+APPLY_FP64_PIPE_ACTIVE = 0.66
 MECH_SOLVERS = {"fas": 0, "fcg": 1, "mixed": 2}
 
-# DRAM bytes (read + write) per launch of the finest PCG apply: one ncu capture of the kernel on the
-# 193^3 level (7,189,057 nodes) measured 1339.8 MB read + 165.9 MB written, 209.4 B/node (the
-# Gauss-point moduli of strip-edge elements are read twice); other sizes scale that per-node figure
-# by their node count.
-PCG_APPLY_TRAFFIC_PER_NODE = (1339.779e6 + 165.902848e6) / 193 ** 3
+# DRAM bytes (read + write) per launch of the finest PCG apply: ncu on a 257x129x65 specimen (2,154,945
+# nodes) measured 561 MB, 260 B/node (the moduli and planes that neighbouring tiles share are mostly
+# fetched once); other sizes scale that per-node figure by their node count.
+PCG_APPLY_TRAFFIC_PER_NODE = 561e6 / (257 * 129 * 65)
 
 
 def parse_args():
@@ -597,13 +596,13 @@ def run_b200(args, rank, world, local):
         peak, src = peaks()
         kname = ("mech_tile_kernel<Gauss-point moduli, PCG, " +
                  ("planes staged by TMA tensor copies" if TMA_STAGING else "planes staged by per-thread cp.async") +
-                 "> (w = K(d) p, (p, w))")
+                 "> (p = M^-1 r + beta p, w = K(d) p, (p, w))")
         basis = "algorithmic: u 24 + bulK,G,d 24 + regime 2 + out 24 B per finest node"
         roofline = {"bound": "hbm", "kernel": kname,
                     "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "peak_source": src, "bytes_per_node": alg, "bytes_basis": basis,
                     "traffic": PCG_APPLY_TRAFFIC_PER_NODE * N,
-                    "traffic_note": "bytes per launch: ncu dram bytes per node of the 193^3 capture x nodes; above "
+                    "traffic_note": "bytes per launch: ncu dram bytes per node of a 257x129x65 capture x nodes; above "
                                     "the algorithmic bytes because the kernel reads precomputed Gauss-point moduli",
                     "read_layout": {"bytes_per_node": read, "achieved": achieved_read,
                                     "frac": achieved_read / peak,

@@ -1,5 +1,6 @@
-// Element-operator kernels: mechanical K(d) u and diag K(d), phase-field A_d x and diag A_d, with
-// fused epilogues (residual, (p, K p), FAS right-hand side, reactions).
+// Element-operator kernels on warp strips: the mechanical K(d) u with nodal material (the single-call entry
+// points and single-level hierarchies; solves run the column tiles of mech_tile.cu), diag K(d), diag A_d, and the
+// tensor-core form of the FP32 apply; the dispatch between strips and tiles.
 //
 // Tiling ("warp strip"): a warp owns a strip of 32 node columns in x (31 elements, 30 output
 // nodes), wy element rows in y (wy-1 output node rows) and cz output node planes in z, and
@@ -204,7 +205,7 @@ __device__ __forceinline__ void assemble_row(const MechKT<T>& k, const ST& st, i
         for (int m = 0; m < 3; ++m) own_p[m] = st.at(si - 1, m, 0, lane);
       }
       T pre_f[3] = {T(0), T(0), T(0)}, pre_m[3] = {T(0), T(0), T(0)};
-      if (EPI == EPI_RESIDUAL || EPI == EPI_FAS) {
+      if (EPI == EPI_RESIDUAL || EPI == EPI_FAS) {  // FAS: the tensor-core kernel's coarse levels
         const long long n = (long long)x + (long long)ey * k.g.px + (long long)kk * k.g.plane;
 #pragma unroll
         for (int m = 0; m < 3; ++m) {

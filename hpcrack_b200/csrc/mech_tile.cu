@@ -21,13 +21,13 @@
 // instead of the new one, each thread forms its share of a plane one layer before it is needed, and the
 // tile that owns a node writes the new direction (into the other of two arrays: neighbours still read the
 // old one).  That replaces a pass of 96 (48) bytes a node and its launch: an iteration's apply and
-// direction take 842 us on 257^3 in FP64 against 656 + 250, 532 us in FP32 against 401 + 125, and one
+// direction take 842 us on 257^3 in FP64 against 656 + 250, 513 us in FP32 against 401 + 125, and one
 // launch less where launches count; increments -1 to -5 %.  A plane is formed in units of 16 bytes, one
 // (FP32) or two (FP64) a thread; single nodes took 4 rounds of loads, masks and stores.
 //
 // The residual's f and M^-1 are staged the same way, and the Dirichlet flags read ahead.  As loads of each
 // thread from global memory they came due at the end of the layer they were issued in, which is shorter than
-// DRAM's latency under load: 935 us a residual on 257^3 in FP64, 591 in FP32.  Both changes: increments of
+// DRAM's latency under load: 935 us a residual on 257^3 in FP64, 591 in FP32, now 866 and 557.  Both changes: increments of
 // 257^3 1300 -> 1268 ms (FAS, crack), 358 -> 349 (precision form), 257x129x65 154 -> 149, 129^3 18.8 -> 18.55.
 //
 // What bounds it: FP64, the FP64 pipe (66 % of its cycles on 193^3; two warps per scheduler cannot hide

@@ -26,10 +26,10 @@ MECH_FAS, MECH_FCG, MECH_MIXED = 0, 1, 2  # hpc_step_params.mech_solver
 # reference's V(4, 2) pays off once the cycle is a preconditioner (257^3 specimen, precision form:
 # V(4,2) 1.15 solves/s, V(4,4) 1.31)
 PRECISION_MG = (50, 4, 4, 1)
-# Coarsest iterations when the coarsest level is too large for the one-block solver: there each
+# Coarsest iterations when the coarsest level is larger than coarsest_in_one_block's rule: there each
 # iteration costs three launches, and a 20-iteration coarse solve is the better preconditioner per
 # unit time (64-specimen mix: 50 iterations 4.2-4.8 solves/s, 20 iterations 5.9; 10 iterations 2.3).
-# With a one-block coarsest solve (e.g. 9^3 under a 257^3 specimen) 50 stays best (1.35 vs 0.84).
+# With a small coarsest level (e.g. 9^3 under a 257^3 specimen) 50 stays best (1.35 vs 0.84).
 PRECISION_NU0_LARGE_COARSEST = 20
 
 

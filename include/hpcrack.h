@@ -125,7 +125,8 @@ const char* hpc_last_error(void);
  * 0 visits every element. */
 int hpc_set_choice_quirk(hpc_ctx* ctx, int reproduce);
 /* No counterpart in the reference: 1 makes this context measure the strip shape (element rows x
- * planes per warp) of each element kernel on each level size at its first use, by timing the
+ * planes per warp) of each strip kernel (nodal-material applies, diagonals; the tiled applies of the
+ * solves have one shape) on each level size at its first use, by timing the
  * candidates on the live data, instead of taking the latency model's choice; measured shapes are
  * shared by every context of the process.  Results differ from the model's shapes only in the
  * rounding of the reductions (the grid changes); the default 0 keeps runs reproducible. */
