@@ -125,7 +125,8 @@ int num_sms();
 // {px, ny, nz, ncomp}, x fastest, with the given box.
 template <typename T>
 int encode_tensor(const LevelGeo& g, const T* src, int ncomp, int bx, int by, int bz, CUtensorMap* map);
-constexpr int kTileX = 16;  // element columns of a tile in x
+constexpr int kTileX = 16;    // element columns of a tile in x
+constexpr int kMinTileY = 8;  // the fewest element rows of a tile
 // Tiles of a level, `ty` element rows high, and their z chunks (tz) for `slots` resident blocks; at most cap
 // blocks where one chunk allows it.
 StripGeo tile_geo(const LevelGeo& g, int ty, long long slots, long long cap);

@@ -1080,7 +1080,7 @@ static int footprint(const hpc_geometry* geo, int nr, int r, size_t* bytes) {
   const HostLevel& f = lv[geo->maxlevel];
   const size_t nf = (size_t)f.px * f.ny * f.nz;
   total += nf * sizeof(double);  // d_old
-  total += sizeof(double) * (kScalarPool + 3 * 8192) + 64;
+  total += sizeof(double) * (kScalarPool + partials_doubles(f.nx, f.ny)) + 64;
   // allocated on first use: Gauss-point moduli (16 n), flexible-PCG vectors (5 x 3n), the FP32
   // mirror of every level (7 x 3n + material) with its Gauss-point moduli, the checkpoint (6 dense)
   total += nf * sizeof(double) * (16 + 15);
@@ -1221,7 +1221,7 @@ static int create_ctx(hpc_ctx** out, const hpc_geometry* geo, int device, int nr
     cudaError_t ae = ctx_alloc(c, (void**)&c->d_old, sizeof(double) * n);
     if (ae != cudaSuccess) return fail(cuda_fail(ae, "cudaMallocAsync(d_old)"));
     cudaMemsetAsync(c->d_old, 0, sizeof(double) * n, c->stream);
-    c->partials_cap = 3 * 8192;
+    c->partials_cap = partials_doubles(c->L[c->maxlevel].nx, c->L[c->maxlevel].ny);
     if ((ae = ctx_alloc(c, (void**)&c->scal, sizeof(double) * kScalarPool)) != cudaSuccess) return fail(cuda_fail(ae, "scal"));
     cudaMemsetAsync(c->scal, 0, sizeof(double) * kScalarPool, c->stream);
     if ((ae = ctx_alloc(c, (void**)&c->partials, sizeof(double) * c->partials_cap)) != cudaSuccess)

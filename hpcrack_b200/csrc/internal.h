@@ -306,6 +306,9 @@ struct PfCall {
   int s_out0, s_out1, s_out2;
 };
 int launch_pf(hpc_ctx* c, const PfCall& p);
+// Doubles of reduction partials a context with nx x ny nodes a plane needs: three sums of every block of the widest
+// launch on its finest level (mech_tile.cu).
+size_t partials_doubles(int nx, int ny);
 int launch_pf_diag(hpc_ctx* c, int level, double lc, double* out);
 
 // Vector kernels (vector_kernels.cu).

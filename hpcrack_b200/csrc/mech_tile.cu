@@ -70,6 +70,13 @@ StripGeo tile_geo(const LevelGeo& g, int ty, long long slots, long long cap) {
   return s;
 }
 
+// One chunk's blocks are a plane's tiles, however many (1025 x 865 nodes: 8556); tile_geo cuts into more chunks only
+// while the grid fits, and the persistent grids of the strip and vector kernels are smaller.
+size_t partials_doubles(int nx, int ny) {
+  const size_t tx = (size_t)(nx + kTileX - 2) / (kTileX - 1), ty = (size_t)(ny + kMinTileY - 2) / (kMinTileY - 1);
+  return 3 * std::max<size_t>(8192, tx * ty);
+}
+
 namespace {
 
 constexpr int kTX = kTileX;  // element columns of a tile in x: a half-warp, 128 B (64 B) of FP64 (FP32) per row
@@ -587,6 +594,7 @@ template <> struct TileShape<double, false> { static constexpr int TY = 8, MINB 
 template <> struct TileShape<float, false> { static constexpr int TY = 16, MINB = 2, NS = 3; };
 template <> struct TileShape<double, true> { static constexpr int TY = 8, MINB = 3, NS = 3; };
 template <> struct TileShape<float, true> { static constexpr int TY = 16, MINB = 2, NS = 3; };
+static_assert(TileShape<double, false>::TY >= kMinTileY && TileShape<double, true>::TY >= kMinTileY, "partials_doubles");
 
 template <typename T, bool GPM, int EPI, bool ISO, bool TMA, bool DIR>
 int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
