@@ -594,7 +594,7 @@ int check_wait_error(hpc_ctx* c) {
   const int rc = read_scalars(c, S_ERR, 1, &err);
   return rc ? rc : wait_error(c, err);
 }
-// The end of a smoother or cycle call: one scalar, and whether a wait ran out.
+// The end of a residual, smoother or cycle call: one scalar, and whether a wait ran out.
 static int read_result(hpc_ctx* c, int slot, double* out) {
   double s[S_ERR + 1];
   const int rc = read_scalars(c, 0, S_ERR + 1, s);
@@ -1555,7 +1555,7 @@ int hpc_internal_force(hpc_ctx* c, int level, int src_field, int dst_field, doub
   m.small_k = small_k;
   m.s_out0 = m.s_out1 = m.s_out2 = -1;
   int rc = launch_mech(c, m);
-  return rc ? rc : hpc_sync(c);
+  return rc ? rc : check_wait_error(c);
 }
 
 int hpc_prem_u(hpc_ctx* c, int level, int dst_field, double small_k) {
@@ -1579,7 +1579,7 @@ int hpc_fld(hpc_ctx* c, int level, int src_field, int dst_field, double lc) {
   p.lc = lc;
   p.s_out0 = p.s_out1 = p.s_out2 = -1;
   int rc = launch_pf(c, p);
-  return rc ? rc : hpc_sync(c);
+  return rc ? rc : check_wait_error(c);
 }
 
 int hpc_precondition_m(hpc_ctx* c, int level, int dst_field, double lc) {
@@ -1605,9 +1605,9 @@ int hpc_initial_residual_u(hpc_ctx* c, int level, double small_k, double* r_norm
   m.s_out2 = S_RNORM;
   int rc = launch_mech(c, m);
   if (rc) return rc;
-  double s3[3];
-  if ((rc = read_scalars(c, 0, 3, s3))) return rc;
-  if (r_norm) *r_norm = s3[S_RNORM];
+  double rn;
+  if ((rc = read_result(c, S_RNORM, &rn))) return rc;
+  if (r_norm) *r_norm = rn;
   return HPC_OK;
 }
 
@@ -1637,9 +1637,9 @@ int hpc_initial_residual_d(hpc_ctx* c, int level, double lc, double* r_norm) {
   m.s_out2 = -1;
   int rc = launch_pf(c, m);
   if (rc) return rc;
-  double s3[3];
-  if ((rc = read_scalars(c, 0, 3, s3))) return rc;
-  if (r_norm) *r_norm = s3[S_RNORM];
+  double rn;
+  if ((rc = read_result(c, S_RNORM, &rn))) return rc;
+  if (r_norm) *r_norm = rn;
   return HPC_OK;
 }
 
@@ -1683,8 +1683,7 @@ int hpc_u_entire(hpc_ctx* c, const hpc_mg* mg, double small_k, double Ut, int t,
   int cy = 0;
   long long it = 0;
   int rc = u_entire_dev(c, *mg, small_k, Ut, t, mech_tol, &cy, &it);
-  if (rc) return rc;
-  if ((rc = hpc_sync(c))) return rc;
+  if (rc || (rc = check_wait_error(c))) return rc;  // the reaction apply follows the solve's own check
   *f_norm = c->f_norm;
   if (cycles) *cycles = cy;
   if (iters) *iters = (int)it;
@@ -1698,8 +1697,7 @@ int hpc_u_entire_fcg(hpc_ctx* c, const hpc_mg* mg, double small_k, double Ut, in
   int cy = 0;
   long long it = 0;
   int rc = u_entire_fcg_dev(c, *mg, small_k, Ut, t, mech_tol, &cy, &it, mixed != 0);
-  if (rc) return rc;
-  if ((rc = hpc_sync(c))) return rc;
+  if (rc || (rc = check_wait_error(c))) return rc;  // the reaction apply follows the solve's own check
   *f_norm = c->f_norm;
   if (cycles) *cycles = cy;
   if (iters) *iters = (int)it;
