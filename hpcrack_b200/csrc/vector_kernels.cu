@@ -141,6 +141,10 @@ __global__ void mech_update_kernel(LevelGeo g, MechUpdate<T> a, RedTarget red) {
         if (R == 2) *reinterpret_cast<V2*>(a.r_old + o) = r;
         r.x = fix[0][m] ? T(0) : fma(-wv[m].x, alpha, r.x);
         r.y = fix[1][m] ? T(0) : fma(-wv[m].y, alpha, r.y);
+        if (i + 1 >= g.nx) {  // zero there whatever alpha is: the sums and the full weighting read it
+          r.y = T(0);
+          if (i >= g.nx) r.x = T(0);
+        }
         *reinterpret_cast<V2*>(a.r + o) = r;
         if (R == 1) {
           rz = fma((double)r.x, (double)(r.x * mv[m].x), rz);
