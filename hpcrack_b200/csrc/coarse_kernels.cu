@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <map>
 #include <mutex>
 
 #include "device_common.cuh"
@@ -34,7 +35,7 @@
 namespace hpc {
 namespace {
 
-constexpr int kBlocks = 16;  // cluster size (non-portable; hpc_create asks for it)
+constexpr int kBlocks = 16;  // cluster size (non-portable)
 constexpr size_t kMaxSmem = 220 * 1024;
 
 // How a level is laid over the cluster.
@@ -43,6 +44,7 @@ struct ClusterPlan {
   int planes, n1, n2;  // extent along it; the other two axes, n1 the lower-numbered one
   int active;          // blocks that hold planes
   int lp;              // element layers a block computes at most
+  int shape;           // block shape (kShapes)
   int threads, slots;  // threads a block; own nodes and elements a thread at most
   size_t smem;
 };
@@ -51,6 +53,7 @@ struct ClusterPlan {
 // are unrolled over `slots` (the nodes' vectors live in registers): a coarsest level that needs one slot
 // does not run through the code of more, which a few iterations would mostly spend fetching.
 constexpr int kShapes[][2] = {{128, 1}, {256, 2}, {512, 2}};
+constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
 // Components of the field, and coefficients an element keeps: lam and G, or the phase field's mass and
 // gradient weights at its 8 Gauss points.
@@ -73,7 +76,8 @@ bool cluster_plan(const LevelGeo& g, ClusterPlan* p) {
   p->lp = (int)np + 1;
   constexpr int NC = FieldShape<PF>::NC, NM = FieldShape<PF>::NM;
   const size_t vals = 2 * NC * PN + NC * (np + 2) * PN + (NM + 8 * NC) * (np + 1) * EN;
-  for (const auto& sh : kShapes) {
+  for (p->shape = 0; p->shape < kNumShapes; ++p->shape) {
+    const auto& sh = kShapes[p->shape];
     p->threads = sh[0];
     p->slots = sh[1];
     p->smem = sizeof(double) * 4 * kBlocks * (sh[0] / 32) + sizeof(T) * vals + 32;
@@ -491,20 +495,25 @@ ClusterKernel<T, IO> shape_kernel(int threads) {
   return cluster_pcg_kernel<T, IO, PF, ISO, 512, 2>;
 }
 
+cudaLaunchConfig_t cluster_config(int threads, size_t smem, cudaStream_t stream, cudaLaunchAttribute* at) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kBlocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = kBlocks;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
 template <bool PF, typename T, typename IO>
 int launch_cluster(hpc_ctx* c, ClusterArgs<T, IO>& a) {
   if (!cluster_plan<T, PF>(a.g, &a.p)) return HPC_ERR_ARG;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(kBlocks);
-  cfg.blockDim = dim3(a.p.threads);
-  cfg.dynamicSmemBytes = a.p.smem;
-  cfg.stream = c->stream;
   cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = kBlocks;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  const cudaLaunchConfig_t cfg = cluster_config(a.p.threads, a.p.smem, c->stream, &at);
   const bool iso = a.g.hx == a.g.hy && a.g.hy == a.g.hz;
   HPC_CUDA(cudaLaunchKernelEx(
       &cfg, iso ? shape_kernel<T, IO, PF, true>(a.p.threads) : shape_kernel<T, IO, PF, false>(a.p.threads), a));
@@ -512,39 +521,52 @@ int launch_cluster(hpc_ctx* c, ClusterArgs<T, IO>& a) {
   return HPC_OK;
 }
 
+// Sets the kernels' attributes; clears the bits of the shapes of which no whole cluster can be resident with all the
+// shared memory a level may ask for.
 template <typename T, typename IO, bool PF>
-int prepare() {
-  for (const auto& sh : kShapes)
-    for (ClusterKernel<T, IO> k : {shape_kernel<T, IO, PF, true>(sh[0]), shape_kernel<T, IO, PF, false>(sh[0])}) {
-      HPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-      HPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+void prepare(unsigned* shapes) {
+  for (int s = 0; s < kNumShapes; ++s)
+    for (ClusterKernel<T, IO> k : {shape_kernel<T, IO, PF, true>(kShapes[s][0]), shape_kernel<T, IO, PF, false>(kShapes[s][0])}) {
+      cudaLaunchAttribute at{};
+      const cudaLaunchConfig_t cfg = cluster_config(kShapes[s][0], kMaxSmem, nullptr, &at);
+      int n = 0;
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess ||
+          cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&n, (const void*)k, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        *shapes &= ~(1u << s);
+      }
     }
-  return HPC_OK;
 }
 
 }  // namespace
 
-bool cluster_pcg_fits_geo(const LevelGeo& g) {
+// A level is smoothed in a cluster where its share fits a block and the device can hold such a cluster; a device
+// that offers fewer SMs side by side (a partitioned GPU) runs the per-iteration kernels.
+template <bool PF>
+static bool fits(const hpc_ctx* c, const LevelGeo& g) {
   ClusterPlan p;
-  return cluster_plan<double, false>(g, &p);
+  return cluster_plan<double, PF>(g, &p) && ((c->cluster_shapes >> p.shape) & 1u);
 }
-bool cluster_pcg_fits(hpc_ctx* c, int level) {
+bool cluster_pcg_fits_geo(const hpc_ctx* c, const LevelGeo& g) { return fits<false>(c, g); }
+bool cluster_pcg_fits(const hpc_ctx* c, int level) {
   if (level == c->maxlevel) return false;  // the finest level's material is nodal, not element-constant
-  return cluster_pcg_fits_geo(c->L[level]);
+  return cluster_pcg_fits_geo(c, c->L[level]);
 }
 
-// Attributes of the kernels, set once per device (called by hpc_create).
-int cluster_pcg_prepare(int device) {
+// The block shapes a cluster can be resident with on a device (a bit each); asked once per device, by hpc_create.
+unsigned cluster_pcg_shapes(int device) {
   static std::mutex mu;
-  static bool done[64] = {};
+  static std::map<int, unsigned> known;
   std::lock_guard<std::mutex> lock(mu);
-  if (device >= 0 && device < 64 && done[device]) return HPC_OK;
-  int rc;
-  if ((rc = prepare<double, double, false>()) || (rc = prepare<double, float, false>()) ||
-      (rc = prepare<float, float, false>()) || (rc = prepare<double, double, true>()))
-    return rc;
-  if (device >= 0 && device < 64) done[device] = true;
-  return HPC_OK;
+  const auto it = known.find(device);
+  if (it != known.end()) return it->second;
+  unsigned shapes = (1u << kNumShapes) - 1u;
+  prepare<double, double, false>(&shapes);
+  prepare<double, float, false>(&shapes);
+  prepare<float, float, false>(&shapes);
+  prepare<double, double, true>(&shapes);
+  return known[device] = shapes;
 }
 
 int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
@@ -574,10 +596,7 @@ int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb, bool r_given) {
   return launch_cluster<false>(c, a);
 }
 
-bool cluster_pcg_d_fits(hpc_ctx* c, int level) {
-  ClusterPlan p;
-  return cluster_plan<double, true>(c->L[level], &p);
-}
+bool cluster_pcg_d_fits(const hpc_ctx* c, int level) { return fits<true>(c, c->L[level]); }
 
 // pcg_d (phase_field_pcg.cpp:133-214) of a small level.
 int launch_cluster_pcg_d(hpc_ctx* c, int level, double lc, int nb) {

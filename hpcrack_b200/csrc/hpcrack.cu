@@ -1234,7 +1234,7 @@ static int create_ctx(hpc_ctx** out, const hpc_geometry* geo, int device, int nr
   shape_table(N);
   int rc = upload_shape_table(N);
   if (rc) return fail(rc);
-  if ((rc = cluster_pcg_prepare(device))) return fail(rc);
+  c->cluster_shapes = cluster_pcg_shapes(device);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "create sync"));
   *out = c;
   return HPC_OK;

@@ -127,6 +127,7 @@ struct hpc_ctx {
   int autotune;  // measure strip shapes on first use (hpc_set_autotune)
   int tc_apply;        // precision form: element contraction on the tensor cores (hpc_set_tensor_apply)
   int fused_coarsest;  // coarse-level pcg_u in one cluster when the level fits (hpc_set_fused_coarsest)
+  unsigned cluster_shapes;  // block shapes the device can hold a cluster of (cluster_pcg_shapes)
   int gpm_active;      // finest applies read F[maxlevel].gpm (set while a mechanical solve runs)
   int tma_stage;       // finest applies stage rows with tensor copies (hpc_set_tma_staging)
   // z-slab rank of a specimen split over ranks (hpc_create_slab); null for a whole specimen.  A
@@ -379,9 +380,9 @@ int launch_zero_count(hpc_ctx* c, int level, int ncomp, const double* v, int slo
 int upload_shape_table(const double* N64);
 // Whole pcg_u of a small coarse level in one thread-block cluster (coarse_kernels.cu): FP64, FP32 mirror
 // (homogeneous Dirichlet values), and the FP32 mirror's u and fu with FP64 arithmetic and material.
-bool cluster_pcg_fits(hpc_ctx* c, int level);
-bool cluster_pcg_fits_geo(const LevelGeo& g);
-int cluster_pcg_prepare(int device);
+bool cluster_pcg_fits(const hpc_ctx* c, int level);
+bool cluster_pcg_fits_geo(const hpc_ctx* c, const LevelGeo& g);
+unsigned cluster_pcg_shapes(int device);
 // r_given: F.ru holds the first residual.
 int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb, bool r_given);
 int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
@@ -389,7 +390,7 @@ int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double
 int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb, bool r_given);
 int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb, bool r_given);
 // The same for pcg_d, any level that fits.
-bool cluster_pcg_d_fits(hpc_ctx* c, int level);
+bool cluster_pcg_d_fits(const hpc_ctx* c, int level);
 int launch_cluster_pcg_d(hpc_ctx* c, int level, double lc, int nb);
 int tuned_shapes(int* out5, int cap);  // measured strip shapes: {nx, ny, nz, wy, cz} per entry
 

@@ -357,7 +357,7 @@ int slab_coarsest_mode(hpc_ctx* c) {
   if (!c->slab || c->slab->nr == 1) return 0;
   LevelGeo g = c->L[0];
   g.nz = c->geo.element_nb[2] + 1;
-  return c->maxlevel > 0 && cluster_pcg_fits_geo(g) ? 1 : 2;
+  return c->maxlevel > 0 && cluster_pcg_fits_geo(c, g) ? 1 : 2;
 }
 
 int slab_coarsest(hpc_ctx* c, double Ut, int nb) {
