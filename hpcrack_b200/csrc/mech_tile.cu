@@ -70,6 +70,14 @@ StripGeo tile_geo(const LevelGeo& g, int ty, long long slots, long long cap) {
   return s;
 }
 
+int tile_rows(int ny, int full, int least) {
+  const auto computed = [ny](int ty) { return (ny + ty - 2) / (ty - 1) * ty; };
+  int best = full;
+  for (int ty = full / 2; ty >= least; ty /= 2)
+    if (4 * computed(ty) <= 3 * computed(best)) best = ty;
+  return best;
+}
+
 // One chunk's blocks are a plane's tiles, however many (1025 x 865 nodes: 8556); tile_geo cuts into more chunks only
 // while the grid fits, and the persistent grids of the strip and vector kernels are smaller.
 size_t partials_doubles(int nx, int ny) {
@@ -185,9 +193,7 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
   uint64_t* bars = reinterpret_cast<uint64_t*>(base);
   T* exch = reinterpret_cast<T*>(base + S::o_exch);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & (kTX - 1);
-  // the two half-warps of a warp work 4 rows apart: with the staged row pitch that spreads an FP32
-  // warp over all 32 banks
-  const int row = (warp & 3) + 4 * (lane >> 4) + 8 * (warp >> 2);
+  const int row = tile_row<TY>(warp, lane);
   constexpr int A16 = 16 / (int)sizeof(T);  // columns per 16 bytes: a tensor copy's x start is a multiple
   const SFt<T> s = make_sf<T>(k.g);
   const T wg = ISO ? T(k.g.wg) * (s.ih[0] * s.ih[0]) : T(k.g.wg);
@@ -589,16 +595,16 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
 // FP64 7 % (703 against 656 us): a layer's arithmetic is too short to cover the copies.
 // In modes (coarse levels) FP64 needs 160 registers, so a third block fits: 65^3 FAS increments 5.67 ms against 5.75
 // with 2; in FP32 a third block spills: 97^3 precision form 98.9 ms against 98.2 with 2.
-template <typename T, bool MODES> struct TileShape;
-template <> struct TileShape<double, false> { static constexpr int TY = 8, MINB = 2, NS = 3; };
-template <> struct TileShape<float, false> { static constexpr int TY = 16, MINB = 2, NS = 3; };
-template <> struct TileShape<double, true> { static constexpr int TY = 8, MINB = 3, NS = 3; };
-template <> struct TileShape<float, true> { static constexpr int TY = 16, MINB = 2, NS = 3; };
-static_assert(TileShape<double, false>::TY >= kMinTileY && TileShape<double, true>::TY >= kMinTileY, "partials_doubles");
+// LOW: half the rows and twice the blocks an SM, for levels of few node rows (tile_rows).
+template <typename T, bool MODES, bool LOW> struct TileShape {
+  static constexpr bool F64 = sizeof(T) == 8;
+  static constexpr int FULL = F64 ? 8 : 16, TY = LOW ? FULL / 2 : FULL, MINB = (F64 && MODES ? 3 : 2) * (LOW ? 2 : 1), NS = 3;
+  static_assert(TY >= kMinTileY, "partials_doubles");
+};
 
-template <typename T, bool GPM, int EPI, bool ISO, bool TMA, bool DIR>
+template <typename T, bool GPM, int EPI, bool ISO, bool TMA, bool DIR, bool LOW>
 int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
-  using Shape = TileShape<T, !GPM && ISO>;
+  using Shape = TileShape<T, !GPM && ISO, LOW>;
   constexpr int TY = Shape::TY, NS = Shape::NS;
   constexpr bool EX = DIR || EPI == EPI_RESIDUAL;
   using S = TileSmem<T, GPM, TY, NS, EX>;
@@ -625,12 +631,18 @@ int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
   return HPC_OK;
 }
 
+template <typename T, bool GPM, int EPI, bool ISO, bool TMA, bool DIR>
+int run_tile_h(hpc_ctx* c, MechKT<T>& k, int cls) {
+  constexpr int full = TileShape<T, !GPM && ISO, false>::FULL;
+  if (tile_rows(k.g.ny, full, full / 2) < full) return run_tile<T, GPM, EPI, ISO, TMA, DIR, true>(c, k, cls);
+  return run_tile<T, GPM, EPI, ISO, TMA, DIR, false>(c, k, cls);
+}
 template <typename T, bool GPM, int EPI, bool DIR = false>
 int run_tile_e(hpc_ctx* c, MechKT<T>& k, int cls) {
   const bool iso = k.g.hx == k.g.hy && k.g.hy == k.g.hz;
   if (c->tma_stage)
-    return iso ? run_tile<T, GPM, EPI, true, true, DIR>(c, k, cls) : run_tile<T, GPM, EPI, false, true, DIR>(c, k, cls);
-  return iso ? run_tile<T, GPM, EPI, true, false, DIR>(c, k, cls) : run_tile<T, GPM, EPI, false, false, DIR>(c, k, cls);
+    return iso ? run_tile_h<T, GPM, EPI, true, true, DIR>(c, k, cls) : run_tile_h<T, GPM, EPI, false, true, DIR>(c, k, cls);
+  return iso ? run_tile_h<T, GPM, EPI, true, false, DIR>(c, k, cls) : run_tile_h<T, GPM, EPI, false, false, DIR>(c, k, cls);
 }
 
 }  // namespace

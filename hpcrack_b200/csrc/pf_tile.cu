@@ -9,7 +9,8 @@
 //
 // What bounds it: the FP64 pipe on the large levels, the layers' serial chain on the small ones.  Per
 // launch, with the strip kernel it replaced in brackets: 257^3 437 us (591), 129^3 69 (115), 65^3 19 (43),
-// 33^3 13 (21).  16 x 16 columns, two blocks of 256 threads an SM (124 registers).
+// 33^3 13 (21).  16 x 16 columns, two blocks of 256 threads an SM (124 registers); on levels of few node rows 8 or 4
+// element rows and as many threads an SM (tile_rows).
 #include <algorithm>
 
 #include "element_common.cuh"
@@ -17,10 +18,15 @@
 namespace hpc {
 namespace {
 
-constexpr int kTX = kTileX, kTY = 16, kNT = kTX * kTY, kNY = kTY + 1, kStages = 3, kBX = 18, kXP = 20;
+constexpr int kTX = kTileX, kStages = 3, kBX = 18, kXP = 20;
 constexpr unsigned kPfWaitPolls = 1u << 24;  // far above any copy's latency; then the kernel reports
-constexpr size_t kPlane = (sizeof(double) * kNY * kBX + 127) / 128 * 128;
-constexpr size_t kOExch = 128 + kStages * 2 * kPlane, kSmem = kOExch + sizeof(double) * 2 * kTY * kXP + 128;
+// A tile of TY rows: threads, staged rows, shared memory, resident blocks the registers are budgeted for.
+template <int TY> struct PfShape {
+  static constexpr int NT = kTX * TY, NY = TY + 1, MINB = 32 / TY;
+  static constexpr size_t plane = (sizeof(double) * NY * kBX + 127) / 128 * 128;
+  static constexpr size_t o_exch = 128 + kStages * 2 * plane, bytes = o_exch + sizeof(double) * 2 * TY * kXP + 128;
+  static_assert(TY >= kMinTileY, "partials_doubles");
+};
 
 struct PfTileK {
   LevelGeo g;
@@ -52,14 +58,16 @@ struct PfState {
   bool zero;  // a node of the plane's quad has gc == 0 (gauss_point_MP's zero rule)
 };
 
-template <int EPI, bool ISO, bool TMA>
-__global__ void __launch_bounds__(kNT, 2) pf_tile_kernel(const __grid_constant__ PfTileK k) {
+template <int EPI, bool ISO, bool TMA, int TY>
+__global__ void __launch_bounds__(kTX* TY, PfShape<TY>::MINB) pf_tile_kernel(const __grid_constant__ PfTileK k) {
+  using S = PfShape<TY>;
+  constexpr int NT = S::NT, NY = S::NY;
   extern __shared__ __align__(128) unsigned char pf_smem[];
   unsigned char* base = pf_smem + ((128u - (smem_u32(pf_smem) & 127u)) & 127u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(base);
-  double* exch = reinterpret_cast<double*>(base + kOExch);
+  double* exch = reinterpret_cast<double*>(base + S::o_exch);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & (kTX - 1);
-  const int row = (warp & 3) + 4 * (lane >> 4) + 8 * (warp >> 2);
+  const int row = tile_row<TY>(warp, lane);
   const SF s = make_sf(k.g);
   // ISO: only the gradient term carries 1/h^2 (see sf_forward); the mass term keeps wg
   const double wgb = (ISO ? k.g.wg * (s.ih[0] * s.ih[0]) : k.g.wg) * k.lc, wga = k.g.wg / k.lc, wgh = 2.0 * k.g.wg;
@@ -78,7 +86,7 @@ __global__ void __launch_bounds__(kNT, 2) pf_tile_kernel(const __grid_constant__
   const int tiles = k.tx * k.ty, chunks = (int)gridDim.x / tiles;
   const int tile = (int)(blockIdx.x % (unsigned)tiles), chunk = (int)(blockIdx.x / (unsigned)tiles);
   const int z0 = (int)((long long)k.g.nz * chunk / chunks), zend = (int)((long long)k.g.nz * (chunk + 1) / chunks) - 1;
-  const int x0 = (tile % k.tx) * (kTX - 1), y0 = (tile / k.tx) * (kTY - 1);
+  const int x0 = (tile % k.tx) * (kTX - 1), y0 = (tile / k.tx) * (TY - 1);
   const int x = x0 - 1 + tx, y = y0 - 1 + row;
   const int nl = zend - z0 + 2;  // element layers z0 - 1 .. zend; plane j of the stream is z0 - 1 + j
   const int xs = x0 - 1 >= 0 ? (x0 - 1) / 2 * 2 : -2, off = (x0 - 1) - xs;  // a copy starts on 16 bytes
@@ -86,7 +94,7 @@ __global__ void __launch_bounds__(kNT, 2) pf_tile_kernel(const __grid_constant__
   const bool out_node = tx >= 1 && row >= 1 && x < k.g.nx && y < k.g.ny;
 
   auto slot = [&](int j, int f) {
-    return reinterpret_cast<double*>(base + 128 + (size_t)(((unsigned)j % kStages) * 2 + f) * kPlane);
+    return reinterpret_cast<double*>(base + 128 + (size_t)(((unsigned)j % kStages) * 2 + f) * S::plane);
   };
   auto issue = [&](int j) {
     if (j <= nl) {
@@ -96,7 +104,7 @@ __global__ void __launch_bounds__(kNT, 2) pf_tile_kernel(const __grid_constant__
           const uint32_t bar = smem_u32(bars + (unsigned)j % kStages);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                       "r"((int)sizeof(double) * 2 * kNY * kBX)
+                       "r"((int)sizeof(double) * 2 * NY * kBX)
                        : "memory");
 #pragma unroll
           for (int f = 0; f < 2; ++f)
@@ -107,8 +115,8 @@ __global__ void __launch_bounds__(kNT, 2) pf_tile_kernel(const __grid_constant__
                 : "memory");
         }
       } else {
-        for (int q = tid; q < 2 * kNY * 17; q += kNT) {  // zeros outside the grid
-          const int c = q % 17, r = q / 17, ry = r % kNY, f = r / kNY;
+        for (int q = tid; q < 2 * NY * 17; q += NT) {  // zeros outside the grid
+          const int c = q % 17, r = q / 17, ry = r % NY, f = r / NY;
           const int gx = x0 - 1 + c, gy = y0 - 1 + ry;
           const bool ok = gx >= 0 && gx < k.g.nx && gy >= 0 && gy < k.g.ny && kk >= 0 && kk < k.g.nz;
           const double* src = (f ? k.gc : k.x) + (ok ? nidx(k.g, gx, gy, kk) : 0);
@@ -238,7 +246,7 @@ __global__ void __launch_bounds__(kNT, 2) pf_tile_kernel(const __grid_constant__
       f[2] = i1[0] + i1[1] - d1;
     }
     const double X0 = f[0] + __shfl_up_sync(kFull, f[1], 1, kTX);
-    double* ex_w = exch + (size_t)(li & 1) * kTY * kXP + row * kXP + tx;
+    double* ex_w = exch + (size_t)(li & 1) * TY * kXP + row * kXP + tx;
     *ex_w = f[2] + __shfl_up_sync(kFull, f[3], 1, kTX);
     bad = __syncthreads_or(bad);
     if (bad) return false;
@@ -290,31 +298,41 @@ __global__ void __launch_bounds__(kNT, 2) pf_tile_kernel(const __grid_constant__
   }
 }
 
-template <int EPI, bool ISO, bool TMA>
+template <int EPI, bool ISO, bool TMA, int TY>
 int run_pf(hpc_ctx* c, PfTileK& k, int cls) {
-  auto kern = pf_tile_kernel<EPI, ISO, TMA>;
+  using S = PfShape<TY>;
+  auto kern = pf_tile_kernel<EPI, ISO, TMA, TY>;
   int per_sm = 1, rc;
-  if ((rc = kernel_cfg((const void*)kern, kSmem, kSmem, kNT, &per_sm))) return rc;
-  const StripGeo sg = tile_geo(k.g, kTY, (long long)num_sms() * per_sm, (long long)c->partials_cap / 3);
+  if ((rc = kernel_cfg((const void*)kern, S::bytes, S::bytes, S::NT, &per_sm))) return rc;
+  const StripGeo sg = tile_geo(k.g, TY, (long long)num_sms() * per_sm, (long long)c->partials_cap / 3);
   if ((size_t)sg.nstrips * 3 > c->partials_cap) return cuda_fail(cudaErrorInvalidValue, "partials buffer");
   k.tx = sg.tx;
   k.ty = sg.ty;
   if constexpr (TMA) {
-    if ((rc = encode_tensor<double>(k.g, k.x, 1, kBX, kNY, 1, &k.xmap))) return rc;
-    if ((rc = encode_tensor<double>(k.g, k.gc, 1, kBX, kNY, 1, &k.cmap))) return rc;
+    if ((rc = encode_tensor<double>(k.g, k.x, 1, kBX, S::NY, 1, &k.xmap))) return rc;
+    if ((rc = encode_tensor<double>(k.g, k.gc, 1, kBX, S::NY, 1, &k.cmap))) return rc;
   }
   timing_begin(c, cls);
-  kern<<<(unsigned)sg.nstrips, kNT, kSmem, c->stream>>>(k);
+  kern<<<(unsigned)sg.nstrips, S::NT, S::bytes, c->stream>>>(k);
   timing_end(c, cls);
   HPC_CHECK_LAUNCH(c);
   return HPC_OK;
 }
 
+template <int EPI, bool ISO, bool TMA>
+int run_pf_h(hpc_ctx* c, PfTileK& k, int cls) {
+  switch (tile_rows(k.g.ny, 16, 4)) {
+    case 4: return run_pf<EPI, ISO, TMA, 4>(c, k, cls);
+    case 8: return run_pf<EPI, ISO, TMA, 8>(c, k, cls);
+    default: return run_pf<EPI, ISO, TMA, 16>(c, k, cls);
+  }
+}
+
 template <int EPI>
 int run_pf_e(hpc_ctx* c, PfTileK& k, int cls) {
   const bool iso = k.g.hx == k.g.hy && k.g.hy == k.g.hz;
-  if (c->tma_stage) return iso ? run_pf<EPI, true, true>(c, k, cls) : run_pf<EPI, false, true>(c, k, cls);
-  return iso ? run_pf<EPI, true, false>(c, k, cls) : run_pf<EPI, false, false>(c, k, cls);
+  if (c->tma_stage) return iso ? run_pf_h<EPI, true, true>(c, k, cls) : run_pf_h<EPI, false, true>(c, k, cls);
+  return iso ? run_pf_h<EPI, true, false>(c, k, cls) : run_pf_h<EPI, false, false>(c, k, cls);
 }
 
 }  // namespace
