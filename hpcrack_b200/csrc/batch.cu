@@ -232,23 +232,14 @@ int mech_post(hpc_ctx* c, const hpc_step_params& p, const double* sc, int* cycle
   *fin_iters = (long long)*cycles * (L == 0 ? p.mg_u.nu0 : p.mg_u.nu1 + p.mg_u.nu2);
   c->f_norm = sc[S_FNORM];
   LevelFields& F = c->F[L];
-  if (p.mech_solver == HPC_MECH_FAS && sc[S_ERR] != 0.0) {
-    launch_set_scalar(c, S_ERR, 0.0);
-    set_error("a bounded wait in a kernel (tensor copy) ran out");
-    return HPC_ERR_CUDA;
-  }
+  int rc = wait_error(c);
+  if (rc) return rc;
   if (p.mech_solver != HPC_MECH_FAS) {
-    if (sc[S_ERR] != 0.0) {
-      launch_set_scalar(c, S_ERR, 0.0);
-      set_error("a bounded wait in a kernel (tensor copy or MMA completion) ran out");
-      return HPC_ERR_CUDA;
-    }
     const size_t vbytes = sizeof(double) * 3 * (size_t)c->L[L].n;
     HPC_CUDA(cudaMemcpyAsync(F.u, c->fcg.x, vbytes, cudaMemcpyDeviceToDevice, c->stream));
     HPC_CUDA(cudaMemcpyAsync(F.fu, c->fcg.f, vbytes, cudaMemcpyDeviceToDevice, c->stream));
   }
   // externe_force_nodal (mechanical_right_hnd.cpp:18-38)
-  int rc;
   if ((rc = launch_bc(c, L, F.u, nullptr, 0, 1.0))) return rc;
   MechCall r{};
   r.level = L;

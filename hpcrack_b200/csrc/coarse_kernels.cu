@@ -572,27 +572,27 @@ unsigned cluster_pcg_shapes(int device) {
 int launch_cluster_pcg_on(hpc_ctx* c, const LevelGeo& g, double* u, const double* fu, double* ru, const double* invM,
                           const double* Ke, const double* Ge, double Ut, int nb) {
   const int r_given = 0;
-  ClusterArgs<double, double> a{g, {}, u, fu, ru, invM, Ke, Ge, Ut, nb, c->scal, r_given, S_RNORM, -1, c->scal + S_ERR};
+  ClusterArgs<double, double> a{g, {}, u, fu, ru, invM, Ke, Ge, Ut, nb, c->scal, r_given, S_RNORM, -1, c->err};
   return launch_cluster<false>(c, a);
 }
 
 int launch_cluster_pcg(hpc_ctx* c, int level, double Ut, int nb, bool r_given) {
   const LevelFields& F = c->F[level];
   ClusterArgs<double, double> a{c->L[level], {}, F.u, F.fu, F.ru, F.preMu, F.Ke, F.Ge, Ut, nb, c->scal, r_given, S_RNORM, -1,
-                                c->scal + S_ERR};
+                                c->err};
   return launch_cluster<false>(c, a);
 }
 
 int launch_cluster_pcg_f32(hpc_ctx* c, int level, int nb, bool r_given) {
   const LevelF32& F = c->F32[level];
-  ClusterArgs<float, float> a{c->L[level], {}, F.u, F.fu, F.ru, F.invM, F.Ke, F.Ge, 0.f, nb, c->scal, r_given, -1, -1, c->scal + S_ERR};
+  ClusterArgs<float, float> a{c->L[level], {}, F.u, F.fu, F.ru, F.invM, F.Ke, F.Ge, 0.f, nb, c->scal, r_given, -1, -1, c->err};
   return launch_cluster<false>(c, a);
 }
 
 int launch_cluster_pcg_mixed(hpc_ctx* c, int level, int nb, bool r_given) {
   const LevelFields& F = c->F[level];
   const LevelF32& G = c->F32[level];
-  ClusterArgs<double, float> a{c->L[level], {}, G.u, G.fu, G.ru, F.preMu, F.Ke, F.Ge, 0.0, nb, c->scal, r_given, S_RNORM, -1, c->scal + S_ERR};
+  ClusterArgs<double, float> a{c->L[level], {}, G.u, G.fu, G.ru, F.preMu, F.Ke, F.Ge, 0.0, nb, c->scal, r_given, S_RNORM, -1, c->err};
   return launch_cluster<false>(c, a);
 }
 
@@ -602,7 +602,7 @@ bool cluster_pcg_d_fits(const hpc_ctx* c, int level) { return fits<true>(c, c->L
 int launch_cluster_pcg_d(hpc_ctx* c, int level, double lc, int nb) {
   const LevelFields& F = c->F[level];
   ClusterArgs<double, double> a{c->L[level], {}, F.d, F.fd, F.R, F.preMd, F.gc, F.H, lc, nb, c->scal, 0, S_RNORM, S_FDNORM,
-                                c->scal + S_ERR};
+                                c->err};
   return launch_cluster<true>(c, a);
 }
 

@@ -958,7 +958,7 @@ int launch_mech(hpc_ctx* c, const MechCall& m) {
   k.invM = m.invM;
   k.gpm = (m.finest && c->gpm_active) ? c->F[m.level].gpm : nullptr;
   k.red = make_red(c, m.s_out0, m.s_out1, m.s_out2);
-  k.err = c->scal + S_ERR;
+  k.err = c->err;
   k.r_out = m.r_out;
   k.dir_r = m.dir_r;
   k.dir_m = m.invM;
@@ -1023,7 +1023,7 @@ int launch_mech_f32(hpc_ctx* c, const MechCall32& m) {
   k.invM = m.invM;
   k.gpm = (m.finest && c->gpm_active) ? F.gpm : nullptr;
   k.red = make_red(c, m.s_out0, m.s_out1, m.s_out2);
-  k.err = c->scal + S_ERR;
+  k.err = c->err;
   const bool fin = m.finest;
   // tensor-core contraction (hpc_set_tensor_apply): isotropic levels, Gauss-point moduli at the finest;
   // not on a slab (its epilogue sums every plane)

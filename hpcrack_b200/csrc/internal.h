@@ -67,7 +67,6 @@ enum Scalar : int {
   S_RES0 = 3,     // generic reduction results
   S_RES1 = 4,
   S_RES2 = 5,
-  S_ERR = 6,      // set to 1 by a kernel whose bounded wait ran out (tensor-core apply)
   S_LCOUNT = 7,   // device-driven solve loops (batched steps): cycles run,
   S_LREL = 8,     //   the convergence ratio the loop tests,
   S_LTRUE = 9,    //   true-residual recomputations of the flexible PCG
@@ -105,6 +104,7 @@ struct hpc_ctx {
   int device;
   double* scal;          // device scalar pool
   double* hscal;         // pinned host staging for scalar reads
+  double* err;           // pinned, set to 1 by a kernel whose bounded wait ran out; the host looks after a synchronisation
   double* stage;         // dense finest-size device buffer for uploads (first use)
   double* partials;      // per-block reduction partials
   unsigned int* counter; // last-block-done counter
@@ -417,6 +417,8 @@ int step_end(hpc_ctx* c, const hpc_step_params* p, int mcy, long long mit, int p
 int step_end_enqueue(hpc_ctx* c);
 int step_end_finish(hpc_ctx* c, const hpc_step_params* p, int mcy, long long mit, int pcy, long long pit, double* out);
 int launch_set_scalar(hpc_ctx* c, int slot, double v);
-int check_wait_error(hpc_ctx* c);
+int check_wait_error(hpc_ctx* c);  // synchronises
+int wait_error(hpc_ctx* c);        // after a synchronisation
+void set_wait_error(hpc_ctx* c);   // what such a kernel does, from the host
 
 }  // namespace hpc

@@ -348,7 +348,7 @@ int launch_pf(hpc_ctx* c, const PfCall& p) {
   k.fd = p.fd;
   k.invM = p.invM;
   k.red = make_red(c, p.s_out0, p.s_out1, p.s_out2);
-  k.err = c->scal + S_ERR;
+  k.err = c->err;
   switch (p.epi) {
     case EPI_PLAIN: return run_pf_e<EPI_PLAIN>(c, k, HPC_KC_NONE);
     case EPI_RESIDUAL: return run_pf_e<EPI_RESIDUAL>(c, k, HPC_KC_NONE);

@@ -1,7 +1,7 @@
 """Every entry point that launches kernels with bounded waits reports a wait that ran out (GPU).
 
-Such a kernel stops, sets a flag in the context's scalar pool and leaves the rest of its output unwritten.  The flag is
-set here from the host, as a kernel sets it; the call that finds it returns an error and clears it, so that the
+Such a kernel stops, sets the context's flag and leaves the rest of its output unwritten.  The flag is set here from
+the host, as a kernel sets it; the call that finds it returns an error and clears it, so that the
 next call is not blamed.
 """
 import ctypes as C
@@ -13,7 +13,6 @@ from hpcrack_b200.solver import Hierarchy, RU, U
 from cases import D, R, load_random
 
 pytestmark = pytest.mark.gpu
-S_ERR = 6  # the flag's place in the scalar pool (csrc/internal.h)
 MG = (4, 1, 1, 1, 1)
 
 CALLS = {
@@ -33,12 +32,12 @@ CALLS = {
 
 @pytest.mark.parametrize("name", CALLS)
 def test_call_reports_and_clears(name):
-    write_scalar = L.load()._ZN3hpc12write_scalarEP7hpc_ctxid  # hpc::write_scalar(hpc_ctx*, int, double)
-    write_scalar.argtypes, write_scalar.restype = [C.c_void_p, C.c_int, C.c_double], C.c_int
+    set_wait_error = L.load()._ZN3hpc14set_wait_errorEP7hpc_ctx  # hpc::set_wait_error(hpc_ctx*)
+    set_wait_error.argtypes, set_wait_error.restype = [C.c_void_p], None
     enb = (4, 3, 5)
     with Hierarchy(1, enb) as h:
         load_random([h], 1, enb, seed=2)
-        assert write_scalar(h.h, S_ERR, 1.0) == 0
+        set_wait_error(h.h)
         with pytest.raises(Exception, match="bounded wait"):
             CALLS[name](h)
         CALLS[name](h)
