@@ -115,23 +115,6 @@ def run_request(solver, w: ms.Workload, increments: int, mech_solver: int = 0, p
     return outs
 
 
-# A server that builds its own contexts runs a small increment over and over for this long before its
-# slots admit: the first increment of a process loads the library's kernels (1.9 s), the memory pool
-# and the clocks of an idle GPU need the rest.  Requests that arrive meanwhile start together.
-WARM_SECONDS = 0.1
-
-
-def warm_up(factory: Callable, mech_solver: int, precision_mg: bool):
-    w = ms.make_workload("small17")
-    end = time.perf_counter() + WARM_SECONDS
-    while time.perf_counter() < end:
-        solver = factory(w)
-        try:
-            run_request(solver, w, 1, mech_solver, precision_mg)
-        finally:
-            solver.close()
-
-
 class SolveServer:
     def __init__(self, hbm_budget: int, slots: int, solver_factory: Callable = None,
                  footprint: Callable = None, keep_fields: bool = False, mech_solver: int = 0,
@@ -139,9 +122,6 @@ class SolveServer:
         self.budget = int(hbm_budget)
         self.slots = int(slots)
         self.factory = solver_factory or default_factory()
-        self._warm = threading.Event()  # set once the slots may admit
-        if solver_factory is not None:
-            self._warm.set()
         self.footprint = footprint or default_footprint
         self.keep_fields = keep_fields
         self.mech_solver = int(mech_solver)
@@ -161,20 +141,10 @@ class SolveServer:
     # ---------------------------------------------------------------- client side
     def start(self):
         self._t0 = time.perf_counter()
-        if not self._warm.is_set():
-            threading.Thread(target=self._warm_slots, name="warm-up", daemon=True).start()
         for i in range(self.slots):
             th = threading.Thread(target=self._worker, name=f"slot{i}", daemon=True)
             th.start()
             self._workers.append(th)
-
-    def _warm_slots(self):
-        try:
-            warm_up(self.factory, self.mech_solver, self.precision_mg)
-        except BaseException:
-            pass  # a request that meets the same failure reports it
-        finally:
-            self._warm.set()
 
     def now(self) -> float:
         return time.perf_counter() - self._t0
@@ -243,7 +213,6 @@ class SolveServer:
             self._cv.notify_all()
 
     def _worker(self):
-        self._warm.wait()
         while True:
             req = self._admit()
             if req is None:

@@ -1,5 +1,6 @@
 import os
 import sys
+import time
 
 import pytest
 
@@ -28,3 +29,20 @@ def pytest_collection_modifyitems(config, items):
     for item in items:
         if "gpu" in item.keywords:
             item.add_marker(skip)
+
+
+@pytest.fixture(autouse=True)
+def runs_of_a_mix_start_together(request, monkeypatch):
+    """test_same_result_alone_and_in_mix compares requests run alone with the same ones run side by side.  They arrive
+    50 ms apart and the first takes 21 ms on a B200, so by themselves they would run one after the other: for this test
+    the slots open once all three have arrived."""
+    if request.node.name != "test_same_result_alone_and_in_mix":
+        return
+    from hpcrack_b200 import serving
+    admit = serving.SolveServer._admit
+
+    def admit_after_the_last_arrival(server):
+        time.sleep(max(0.0, 0.11 - server.now()))
+        return admit(server)
+
+    monkeypatch.setattr(serving.SolveServer, "_admit", admit_after_the_last_arrival)
