@@ -1029,7 +1029,6 @@ int launch_mech_f32(hpc_ctx* c, const MechCall32& m) {
   // not on a slab (its epilogue sums every plane)
   if (c->tc_apply && !c->slab && iso(g) && (!fin || k.gpm)) {
     switch (m.epi) {
-      case EPI_PLAIN: return fin ? run_mech_tc<true, EPI_PLAIN>(c, k) : run_mech_tc<false, EPI_PLAIN>(c, k);
       case EPI_RESIDUAL: return fin ? run_mech_tc<true, EPI_RESIDUAL>(c, k) : run_mech_tc<false, EPI_RESIDUAL>(c, k);
       case EPI_PCG: return fin ? run_mech_tc<true, EPI_PCG>(c, k) : run_mech_tc<false, EPI_PCG>(c, k);
       case EPI_FAS: return run_mech_tc<false, EPI_FAS>(c, k);

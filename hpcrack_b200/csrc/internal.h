@@ -266,7 +266,7 @@ int launch_mech_diag(hpc_ctx* c, int level, bool finest, double small_k, double*
 // Gauss-point moduli of the finest level into F[maxlevel].gpm (from bulK, G, d and the regimes)
 int launch_gp_material(hpc_ctx* c, double small_k);
 
-// Single-precision operator on the FP32 mirror of a level (EPI_PLAIN, EPI_RESIDUAL, EPI_PCG, EPI_FAS);
+// Single-precision operator on the FP32 mirror of a level (EPI_RESIDUAL, EPI_PCG, EPI_FAS);
 // the residual zeroes Dirichlet rows and sums (r, M^-1 r) into s_out1 and |r|^2 into s_out2 in FP64.
 struct MechCall32 {
   int level;

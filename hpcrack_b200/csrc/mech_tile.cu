@@ -647,17 +647,18 @@ int run_tile_e(hpc_ctx* c, MechKT<T>& k, int cls) {
 
 }  // namespace
 
+// What the drivers ask for: reactions on the finest level, the plain operator (hpc_internal_force) on coarse levels,
+// both in FP64 only.
 template <typename T>
 int launch_mech_tile(hpc_ctx* c, MechKT<T>& k, bool finest, int epi) {
-  const int pcg = sizeof(T) == 8 ? HPC_KC_MECH_PCG_FINEST : HPC_KC_MECH32_PCG_FINEST;
+  constexpr bool F64 = sizeof(T) == 8;
   if (finest) {
+    const int pcg = F64 ? HPC_KC_MECH_PCG_FINEST : HPC_KC_MECH32_PCG_FINEST;
     switch (epi) {
       case EPI_RESIDUAL: return run_tile_e<T, true, EPI_RESIDUAL>(c, k, HPC_KC_NONE);
       case EPI_PCG: return k.p_new ? run_tile_e<T, true, EPI_PCG, true>(c, k, pcg) : run_tile_e<T, true, EPI_PCG>(c, k, pcg);
       case EPI_REACTION:
-        if constexpr (sizeof(T) == 8) return run_tile_e<T, true, EPI_REACTION>(c, k, HPC_KC_NONE);
-        break;
-      case EPI_PLAIN: return run_tile_e<T, true, EPI_PLAIN>(c, k, HPC_KC_NONE);
+        if constexpr (F64) return run_tile_e<T, true, EPI_REACTION>(c, k, HPC_KC_NONE);
     }
     return HPC_ERR_ARG;
   }
@@ -666,10 +667,8 @@ int launch_mech_tile(hpc_ctx* c, MechKT<T>& k, bool finest, int epi) {
     case EPI_PCG:
       return k.p_new ? run_tile_e<T, false, EPI_PCG, true>(c, k, HPC_KC_NONE) : run_tile_e<T, false, EPI_PCG>(c, k, HPC_KC_NONE);
     case EPI_FAS: return run_tile_e<T, false, EPI_FAS>(c, k, HPC_KC_NONE);
-    case EPI_PLAIN: return run_tile_e<T, false, EPI_PLAIN>(c, k, HPC_KC_NONE);
-    case EPI_REACTION:
-      if constexpr (sizeof(T) == 8) return run_tile_e<T, false, EPI_REACTION>(c, k, HPC_KC_NONE);
-      break;
+    case EPI_PLAIN:
+      if constexpr (F64) return run_tile_e<T, false, EPI_PLAIN>(c, k, HPC_KC_NONE);
   }
   return HPC_ERR_ARG;
 }
