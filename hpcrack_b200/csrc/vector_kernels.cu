@@ -92,6 +92,8 @@ __global__ void mech_update_kernel(LevelGeo g, MechUpdate<T> a, RedTarget red) {
     const int i = 2 * (int)(q - row * half);
     const int kz = (int)(row / (unsigned)g.ny), j = (int)(row - (unsigned)kz * (unsigned)g.ny);
     const long long n = (long long)row * g.px + i;
+    if (i >= g.nx) continue;
+    const bool pad = i + 1 >= g.nx;  // the second slot is padding and stays zero in u and r
     const double rz0 = rz, rn0 = rn;
     bool fix[2][3] = {{false, false, false}, {false, false, false}};
     if (R && g.bz[kz]) {
@@ -130,10 +132,7 @@ __global__ void mech_update_kernel(LevelGeo g, MechUpdate<T> a, RedTarget red) {
         }
         x.x = fma(pv[m].x, alpha, x.x);
         x.y = fma(pv[m].y, alpha, x.y);
-        if (i + 1 >= g.nx) {  // padding slots stay zero: the applies stage them, and those of p may hold anything
-          x.y = T(0);
-          if (i >= g.nx) x.x = T(0);
-        }
+        if (pad) x.y = T(0);  // the applies stage it, and p's may hold anything
         *reinterpret_cast<V2*>(a.u + o) = x;
       }
       if (R) {
@@ -141,10 +140,7 @@ __global__ void mech_update_kernel(LevelGeo g, MechUpdate<T> a, RedTarget red) {
         if (R == 2) *reinterpret_cast<V2*>(a.r_old + o) = r;
         r.x = fix[0][m] ? T(0) : fma(-wv[m].x, alpha, r.x);
         r.y = fix[1][m] ? T(0) : fma(-wv[m].y, alpha, r.y);
-        if (i + 1 >= g.nx) {  // zero there whatever alpha is: the sums and the full weighting read it
-          r.y = T(0);
-          if (i >= g.nx) r.x = T(0);
-        }
+        if (pad) r.y = T(0);  // whatever alpha is: the sums and the full weighting read it
         *reinterpret_cast<V2*>(a.r + o) = r;
         if (R == 1) {
           rz = fma((double)r.x, (double)(r.x * mv[m].x), rz);
