@@ -129,9 +129,9 @@ constexpr int kTileX = 16;    // element columns of a tile in x
 constexpr int kMinTileY = 4;  // the fewest element rows of a tile
 // Element rows of a tile for a level of ny node rows: `full` of them, or by halves down to `least` where that computes
 // at most three quarters of the rows (a tile of ty finishes ty - 1 node rows and computes ty whatever it finishes).
-// Without it a box thin in y paid for whole tiles.  1025 x 3 x 1025 nodes: phase-field operator call 289 us, now 102;
-// two cycles of the displacement solve in FP64 12.9 ms, now 10.0, in the precision form 13.5, now 10.4.  1025 x 17 x
-// 513: 367 and 271 us, 18.7 and 18.1, 18.3 and 16.8 ms.
+// For the phase field; the displacement tiles are halved for boxes of one tile only (run_tile_h).  Boxes thin in y paid
+// for whole tiles.  1025 x 3 x 1025 nodes: phase-field operator call 289 us, now 102; two cycles of the displacement
+// solve in FP64 12.9 ms, now 10.0, in the precision form 13.5, now 10.4.  1025 x 17 x 513: operator 367 us, now 271.
 int tile_rows(int ny, int full, int least);
 // The row a thread of a tile of TY rows works on.  A warp's two half-warps work 4 rows apart (2 in the lowest tile):
 // with the staged row pitch that spreads an FP32 warp over all 32 banks.

@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
 // FP64 7 % (703 against 656 us): a layer's arithmetic is too short to cover the copies.
 // In modes (coarse levels) FP64 needs 160 registers, so a third block fits: 65^3 FAS increments 5.67 ms against 5.75
 // with 2; in FP32 a third block spills: 97^3 precision form 98.9 ms against 98.2 with 2.
-// LOW: half the rows and twice the blocks an SM, for levels of few node rows (tile_rows).
+// LOW: half the rows and twice the blocks an SM, for levels of few node rows (run_tile_h).
 template <typename T, bool MODES, bool LOW> struct TileShape {
   static constexpr bool F64 = sizeof(T) == 8;
   static constexpr int FULL = F64 ? 8 : 16, TY = LOW ? FULL / 2 : FULL, MINB = (F64 && MODES ? 3 : 2) * (LOW ? 2 : 1), NS = 3;
@@ -631,10 +631,11 @@ int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
   return HPC_OK;
 }
 
+// Half the rows where one such tile holds the whole box.  More boxes (17 rows: 24 computed instead of 32) gain 3 to 8 %
+// in single solves of 513 x 17 x 1025 nodes, but cost a batch of six small specimens 0.5 %.
 template <typename T, bool GPM, int EPI, bool ISO, bool TMA, bool DIR>
 int run_tile_h(hpc_ctx* c, MechKT<T>& k, int cls) {
-  constexpr int full = TileShape<T, !GPM && ISO, false>::FULL;
-  if (tile_rows(k.g.ny, full, full / 2) < full) return run_tile<T, GPM, EPI, ISO, TMA, DIR, true>(c, k, cls);
+  if (k.g.ny < TileShape<T, !GPM && ISO, true>::TY) return run_tile<T, GPM, EPI, ISO, TMA, DIR, true>(c, k, cls);
   return run_tile<T, GPM, EPI, ISO, TMA, DIR, false>(c, k, cls);
 }
 template <typename T, bool GPM, int EPI, bool DIR = false>

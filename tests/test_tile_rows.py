@@ -1,13 +1,10 @@
-"""The tile height a level gets never computes many more rows than the best height would (CPU)."""
+"""The height of the phase-field tiles of a level never computes many more rows than the best height would (CPU)."""
 import ctypes as C
-
-import pytest
 
 from hpcrack_b200 import lib as L
 
 
-@pytest.mark.parametrize("full,least", [(16, 4), (16, 8), (8, 4)])
-def test_no_wasted_rows(full, least):
+def test_no_wasted_rows(full=16, least=4):
     tile_rows = L.load()._ZN3hpc9tile_rowsEiii  # hpc::tile_rows(int ny, int full, int least)
     tile_rows.argtypes, tile_rows.restype = [C.c_int] * 3, C.c_int
     heights = [h for h in (4, 8, 16) if least <= h <= full]
