@@ -50,51 +50,21 @@ __device__ __forceinline__ double red_identity() {
 
 struct RedTarget {
   double* partials;      // >= NR * gridDim.x doubles
-  unsigned int* counter; // zero between kernels
+  unsigned int* counter; // zero between kernels; null: the partials are combined by launch_combine
   double* scal;          // scalar pool
   int slot[3];           // destination slots (-1 = discard)
 };
 // The reduction target of a context for the next launch; on a z-slab context the slots are also
 // recorded so that the launch check combines them over the ranks with `op` (a RedOp).
 RedTarget make_red(hpc_ctx* c, int s0, int s1, int s2, int op = RED_SUM);
+// The sums of a kernel of nb blocks that was launched without a counter, by `threads` threads as its last block would.
+void launch_combine(hpc_ctx* c, const RedTarget& red, int nb, int threads);
 
-// Block-wide reduction of NR values per thread followed by a deterministic grid-wide
-// combination: every block stores its partials; the last block to finish combines them, each of its
-// threads a fixed strided share, then a fixed tree over the threads, so the result does not depend on
-// block scheduling.  Sums whose slot is -1 are not formed.  Must be called by every thread of every
-// block (1-D grid, blockDim.x a multiple of 32, at most 1024).  It is the tail of two kernels in three on
-// the levels up to 97^3; with one warp of the last block combining, three sums each, the 65^3 precision-form
-// increments took 73.8 ms, now 68.3; 97^3 143.9 and 132.3 ms.
+// A grid's partials (nb blocks') into the scalar slots, by every thread of one block: each thread a fixed strided
+// share, then a fixed tree over the threads.
 template <int NR, int OP = RED_SUM>
-__device__ void grid_reduce(double (&v)[NR], const RedTarget& t) {
-  __shared__ double sred[NR][32];
-  __shared__ int s_last;
+__device__ void combine_partials(const RedTarget& t, int nb, double (&sred)[NR][32]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int nb = gridDim.x;
-#pragma unroll
-  for (int r = 0; r < NR; ++r) {
-    if (t.slot[r] < 0) continue;
-    const double x = warp_red<OP>(v[r]);
-    if (lane == 0) sred[r][warp] = x;
-  }
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      if (t.slot[r] < 0) continue;
-      double x = lane < nwarps ? sred[r][lane] : red_identity<OP>();
-      x = warp_red<OP>(x);
-      if (lane == 0) __stcg(t.partials + (size_t)r * nb + blockIdx.x, x);
-    }
-    if (lane == 0) {
-      __threadfence();
-      unsigned prev = atomicAdd(t.counter, 1u);
-      s_last = (prev == (unsigned)nb - 1u);
-    }
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
   double x[NR];
 #pragma unroll
   for (int r = 0; r < NR; ++r) x[r] = red_identity<OP>();
@@ -117,7 +87,48 @@ __device__ void grid_reduce(double (&v)[NR], const RedTarget& t) {
     y = warp_red<OP>(y);
     if (lane == 0) t.scal[t.slot[r]] = y;
   }
-  if (lane == 0) *t.counter = 0u;
+}
+
+// Block-wide reduction of NR values per thread followed by a deterministic grid-wide
+// combination: every block stores its partials; the last block to finish combines them, so the result does not
+// depend on block scheduling.  APART: without a counter the partials are left to a kernel of their own
+// (launch_combine).  Sums whose slot is -1 are not formed.  Must be called by every thread of every
+// block (1-D grid, blockDim.x a multiple of 32, at most 1024).  It is the tail of two kernels in three on
+// the levels up to 97^3; with one warp of the last block combining, three sums each, the 65^3 precision-form
+// increments took 73.8 ms, now 68.3; 97^3 143.9 and 132.3 ms.
+template <int NR, int OP = RED_SUM, bool APART = false>
+__device__ void grid_reduce(double (&v)[NR], const RedTarget& t) {
+  __shared__ double sred[NR][32];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int nb = gridDim.x;
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    if (t.slot[r] < 0) continue;
+    const double x = warp_red<OP>(v[r]);
+    if (lane == 0) sred[r][warp] = x;
+  }
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      if (t.slot[r] < 0) continue;
+      double x = lane < nwarps ? sred[r][lane] : red_identity<OP>();
+      x = warp_red<OP>(x);
+      if (lane == 0) __stcg(t.partials + (size_t)r * nb + blockIdx.x, x);
+    }
+    if (lane == 0 && (!APART || t.counter)) {
+      __threadfence();
+      unsigned prev = atomicAdd(t.counter, 1u);
+      s_last = (prev == (unsigned)nb - 1u);
+    }
+  }
+  if (APART && !t.counter) return;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  combine_partials<NR, OP>(t, nb, sred);
+  if (threadIdx.x == 0) *t.counter = 0u;
 }
 
 // A z plane this rank owns: reductions sum over owned nodes only (realdomain, pcg_utilities.cpp:16-58);

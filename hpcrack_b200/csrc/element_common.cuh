@@ -143,6 +143,11 @@ __device__ __forceinline__ int tile_row(int warp, int lane) {
 // Tiles of a level, `ty` element rows high, and their z chunks (tz) for `slots` resident blocks; at most cap
 // blocks where one chunk allows it.
 StripGeo tile_geo(const LevelGeo& g, int ty, long long slots, long long cap);
+// Whether a tile kernel leaves its sums to launch_combine.  A block that counts itself in holds its place on the SM
+// about 1.7 us longer, which nothing hides where blocks are many and march few planes: 1025 x 1025 x 3 nodes, four
+// iterations of pcg_d 1067 us, 1008 with a combining kernel; two cycles of the FP64 displacement solve 8.38 and 7.93 ms.
+// From nine blocks a place on; a grid that size runs for at least ten times the second launch.
+inline bool combine_apart(const StripGeo& sg, long long slots) { return sg.nstrips > 8 * slots; }
 // Tile kernels (mech_tile.cu): the mechanical operator with precomputed Gauss-point moduli (finest level,
 // k.gpm set) or element-constant moduli (coarse levels).
 template <typename T>

@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(kTX* TY, MINB) mech_tile_kernel(const __grid_c
   if (TMA && bad && tid == 0 && k.err) *k.err = 1.0;
   if (EPI == EPI_RESIDUAL || EPI == EPI_PCG || (EPI == EPI_FAS && k.red.slot[1] >= 0)) {
     double v[3] = {red0, red1, red2};
-    grid_reduce<3>(v, k.red);
+    grid_reduce<3, RED_SUM, true>(v, k.red);
   }
 }
 
@@ -624,8 +624,12 @@ int run_tile(hpc_ctx* c, MechKT<T>& k, int cls) {
       return rc;
     if (GPM && (rc = encode_tensor<T>(k.g, k.gpm, 16, S::BX, TY, 1, &k.gmap))) return rc;
   }
+  const bool apart = (k.red.slot[0] >= 0 || k.red.slot[1] >= 0 || k.red.slot[2] >= 0) &&
+                     combine_apart(k.sg, (long long)num_sms() * per_sm);
+  if (apart) k.red.counter = nullptr;
   timing_begin(c, cls);
   kern<<<(unsigned)k.sg.nstrips, kTX * TY, S::bytes, c->stream>>>(k);
+  if (apart) launch_combine(c, k.red, (int)k.sg.nstrips, kTX * TY);
   timing_end(c, cls);
   HPC_CHECK_LAUNCH(c);
   return HPC_OK;

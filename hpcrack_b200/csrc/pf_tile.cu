@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kTX* TY, PfShape<TY>::MINB) pf_tile_kernel(con
   if (TMA && bad && tid == 0 && k.err) *k.err = 1.0;
   if (EPI == EPI_RESIDUAL || EPI == EPI_PCG) {
     double v[3] = {red0, red1, red2};
-    grid_reduce<3>(v, k.red);
+    grid_reduce<3, RED_SUM, true>(v, k.red);
   }
 }
 
@@ -312,8 +312,12 @@ int run_pf(hpc_ctx* c, PfTileK& k, int cls) {
     if ((rc = encode_tensor<double>(k.g, k.x, 1, kBX, S::NY, 1, &k.xmap))) return rc;
     if ((rc = encode_tensor<double>(k.g, k.gc, 1, kBX, S::NY, 1, &k.cmap))) return rc;
   }
+  const bool apart = (k.red.slot[0] >= 0 || k.red.slot[1] >= 0 || k.red.slot[2] >= 0) &&
+                     combine_apart(sg, (long long)num_sms() * per_sm);
+  if (apart) k.red.counter = nullptr;
   timing_begin(c, cls);
   kern<<<(unsigned)sg.nstrips, S::NT, S::bytes, c->stream>>>(k);
+  if (apart) launch_combine(c, k.red, (int)sg.nstrips, S::NT);
   timing_end(c, cls);
   HPC_CHECK_LAUNCH(c);
   return HPC_OK;

@@ -383,6 +383,15 @@ int launch_dot(hpc_ctx* c, int level, int ncomp, const double* a, const double* 
   return HPC_OK;
 }
 
+__global__ void combine_kernel(RedTarget red, int nb) {
+  __shared__ double sred[3][32];
+  combine_partials<3>(red, nb, sred);
+}
+void launch_combine(hpc_ctx* c, const RedTarget& red, int nb, int threads) {
+  combine_kernel<<<1, threads, 0, c->stream>>>(red, nb);
+  c->launches++;
+}
+
 __global__ void fill_kernel(double* v, long long n, double value) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     v[i] = value;

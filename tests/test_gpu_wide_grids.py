@@ -7,7 +7,7 @@ one operator, 1e-10 for a cycle of a few smoother iterations.
 import pytest
 
 from oracle.bindings import COracle
-from hpcrack_b200.solver import Hierarchy, U
+from hpcrack_b200.solver import FD, Hierarchy, U
 from cases import D, R, load_random, rel
 
 pytestmark = pytest.mark.gpu
@@ -33,5 +33,19 @@ def test_phase_field_operator():
     for impl in (gpu, orc):
         impl.fld(1, D, R, 2.0)
     assert rel(gpu.get(R, 1), orc.get(R, 1)) < 1e-12
+    gpu.close()
+    orc.close()
+
+
+def test_sums_of_many_blocks():
+    gpu, orc = _pair((366, 364, 1), 5)  # finest 733 x 729 x 3: 2401 tiles, whose sums a kernel of its own combines
+    for impl in (gpu, orc):
+        impl.set(FD, 1, impl.get(D, 1))
+    n0 = gpu.launch_count()
+    fd = [impl.pcg_d(1, 2.0, 2, 1, 1.0)[1] for impl in (gpu, orc)]
+    assert gpu.launch_count() - n0 == 3 + 2 + 2 * 4  # the preconditioner; residual and its sums; direction, apply, sums, update
+    assert abs(fd[0] - fd[1]) <= 1e-12 * fd[1]
+    for f in (D, R):
+        assert rel(gpu.get(f, 1), orc.get(f, 1)) < 1e-10, f
     gpu.close()
     orc.close()
