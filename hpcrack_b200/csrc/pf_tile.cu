@@ -115,13 +115,14 @@ __global__ void __launch_bounds__(kTX* TY, PfShape<TY>::MINB) pf_tile_kernel(con
                 : "memory");
         }
       } else {
-        for (int q = tid; q < 2 * NY * 17; q += NT) {  // zeros outside the grid
-          const int c = q % 17, r = q / 17, ry = r % NY, f = r / NY;
-          const int gx = x0 - 1 + c, gy = y0 - 1 + ry;
-          const bool ok = gx >= 0 && gx < k.g.nx && gy >= 0 && gy < k.g.ny && kk >= 0 && kk < k.g.nz;
+        constexpr int U = kBX / 2;  // 16-byte units of a row: whole ones, padding included, zeros outside the grid
+        for (int q = tid; q < 2 * NY * U; q += NT) {
+          const int u = q % U, r = q / U, ry = r % NY, f = r / NY;
+          const int gx = xs + 2 * u, gy = y0 - 1 + ry;
+          const bool ok = gx >= 0 && gx < k.g.px && gy >= 0 && gy < k.g.ny && kk >= 0 && kk < k.g.nz;
           const double* src = (f ? k.gc : k.x) + (ok ? nidx(k.g, gx, gy, kk) : 0);
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(slot(j, f) + ry * kBX + off + c)),
-                       "l"(src), "r"(ok ? 8 : 0)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(slot(j, f) + ry * kBX + 2 * u)),
+                       "l"(src), "r"(ok ? 16 : 0)
                        : "memory");
         }
       }
