@@ -521,22 +521,23 @@ int launch_cluster(hpc_ctx* c, ClusterArgs<T, IO>& a) {
   return HPC_OK;
 }
 
-// Sets the kernels' attributes; clears the bits of the shapes of which no whole cluster can be resident with all the
-// shared memory a level may ask for.
+// Sets the kernels' attributes; false where the device refuses one.
 template <typename T, typename IO, bool PF>
-void prepare(unsigned* shapes) {
-  for (int s = 0; s < kNumShapes; ++s)
-    for (ClusterKernel<T, IO> k : {shape_kernel<T, IO, PF, true>(kShapes[s][0]), shape_kernel<T, IO, PF, false>(kShapes[s][0])}) {
-      cudaLaunchAttribute at{};
-      const cudaLaunchConfig_t cfg = cluster_config(kShapes[s][0], kMaxSmem, nullptr, &at);
-      int n = 0;
-      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess ||
-          cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-          cudaOccupancyMaxActiveClusters(&n, (const void*)k, &cfg) != cudaSuccess || n < 1) {
-        cudaGetLastError();
-        *shapes &= ~(1u << s);
-      }
-    }
+bool prepare(int shape) {
+  for (ClusterKernel<T, IO> k : {shape_kernel<T, IO, PF, true>(kShapes[shape][0]), shape_kernel<T, IO, PF, false>(kShapes[shape][0])})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+      return false;
+  return true;
+}
+// Whether a whole cluster of a shape can be resident with all the shared memory a level may ask for.  The kernels of a
+// shape have the same threads and registers for one such block an SM: one answers for all.
+bool resident(int shape) {
+  cudaLaunchAttribute at{};
+  const cudaLaunchConfig_t cfg = cluster_config(kShapes[shape][0], kMaxSmem, nullptr, &at);
+  int n = 0;
+  return cudaOccupancyMaxActiveClusters(&n, (const void*)shape_kernel<double, double, false, true>(kShapes[shape][0]),
+                                        &cfg) == cudaSuccess && n > 0;
 }
 
 }  // namespace
@@ -561,11 +562,13 @@ unsigned cluster_pcg_shapes(int device) {
   std::lock_guard<std::mutex> lock(mu);
   const auto it = known.find(device);
   if (it != known.end()) return it->second;
-  unsigned shapes = (1u << kNumShapes) - 1u;
-  prepare<double, double, false>(&shapes);
-  prepare<double, float, false>(&shapes);
-  prepare<float, float, false>(&shapes);
-  prepare<double, double, true>(&shapes);
+  unsigned shapes = 0;
+  for (int s = 0; s < kNumShapes; ++s)
+    if (prepare<double, double, false>(s) && prepare<double, float, false>(s) && prepare<float, float, false>(s) &&
+        prepare<double, double, true>(s) && resident(s))
+      shapes |= 1u << s;
+    else
+      cudaGetLastError();  // a refusal is an answer
   return known[device] = shapes;
 }
 
