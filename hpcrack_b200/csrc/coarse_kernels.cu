@@ -103,7 +103,7 @@ struct ClusterArgs {
   double* scal;
   int r_given;  // ru holds the first residual: no apply for it
   int s_rnorm, s_fnorm;  // |r|^2 of the first residual, |f|^2 (phase field); -1: not wanted
-  double* err;  // set to 1 when a bounded wait ran out
+  double* err;  // the context's: set to 1 when a bounded wait ran out
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

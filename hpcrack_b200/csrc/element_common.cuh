@@ -31,7 +31,7 @@ struct MechKT {
   const T* invM;
   const T* gpm;  // finest level, precomputed Gauss-point moduli: K - 2G/3 at [g * n + e], G at [(8 + g) * n + e]
   RedTarget red;
-  double* err;   // tensor-core kernel / TMA staging: set to 1 when a bounded wait ran out
+  double* err;   // tensor-core kernel / TMA staging: set to 1 when a bounded wait ran out (the context's, host memory)
   // PCG direction formed while the planes are staged (mech_tile.cu): p = r M^-1 + beta p_old, beta =
   // red.scal[s_rz] / red.scal[s_rz_prev] (p = r M^-1 if dir_first), written to p_new; fields[0..2] hold p_old
   const T* dir_r;

@@ -871,8 +871,8 @@ int tuned_shapes(int* out5, int cap) {
 // Isotropic spacing (hx = hy = hz) selects the kernels that fold 1/h^2 into the material.
 inline bool iso(const LevelGeo& g) { return g.hx == g.hy && g.hy == g.hz; }
 
-// The staged vector of a finest apply as a TMA tensor {px, ny, nz, 3} (x fastest; the three components
-// n apart), box {BX, 1, 2, 3}: one copy brings a row's three components on two planes.
+// encode_tensor's maps have the box {bx, by, bz, ncomp}: one copy brings a tile's rows of one plane, every
+// component.
 using EncodeTiled = PFN_cuTensorMapEncodeTiled_v12000;
 static EncodeTiled tensor_map_encoder() {
   static EncodeTiled fn = nullptr;
@@ -1045,8 +1045,8 @@ int launch_mech_f32(hpc_ctx* c, const MechCall32& m) {
 }
 
 // Gauss-point moduli of the finest level, computed once per mechanical solve (the material is
-// fixed while the solve runs): the same mech_moduli_finest as the strip kernels, so the applies that
-// read them produce the same bits as the applies that interpolate the nodal fields themselves.
+// fixed while the solve runs): the same mech_moduli_finest as the strip kernels, which interpolate the nodal
+// fields in the apply.  The tiles that read them sum in another order: equal up to rounding.
 template <typename T>
 __global__ void gp_material_kernel(LevelGeo g, const T* K, const T* G, const T* d, const int8_t* choice,
                                    double small_k, T* gpm) {

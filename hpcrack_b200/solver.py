@@ -26,10 +26,12 @@ MECH_FAS, MECH_FCG, MECH_MIXED = 0, 1, 2  # hpc_step_params.mech_solver
 # reference's V(4, 2) pays off once the cycle is a preconditioner (257^3 specimen, precision form:
 # V(4,2) 1.15 solves/s, V(4,4) 1.31)
 PRECISION_MG = (50, 4, 4, 1)
-# Coarsest iterations when the coarsest level is larger than coarsest_in_one_block's rule: there each
-# iteration costs three launches, and a 20-iteration coarse solve is the better preconditioner per
-# unit time (64-specimen mix: 50 iterations 4.2-4.8 solves/s, 20 iterations 5.9; 10 iterations 2.3).
-# With a small coarsest level (e.g. 9^3 under a 257^3 specimen) 50 stays best (1.35 vs 0.84).
+# Coarsest iterations when the coarsest level is larger than coarsest_in_one_block's rule: a 20-iteration
+# coarse solve was the better preconditioner per unit time (64-specimen mix: 50 iterations 4.2-4.8
+# solves/s, 20 iterations 5.9; 10 iterations 2.3), with a small coarsest level (e.g. 9^3 under a 257^3
+# specimen) 50 (1.35 vs 0.84).  Measured when levels above the rule ran three launches an iteration and those
+# below it in one thread block; levels up to about 17^3 run in one cluster launch now, larger ones two
+# launches an iteration, and the choice has not been measured again.
 PRECISION_NU0_LARGE_COARSEST = 20
 
 
@@ -44,7 +46,7 @@ def coarsest_in_one_block(maxlevel: int, element_nb) -> bool:
 
 def precision_mg(maxlevel: int, element_nb, ncy: int) -> tuple:
     """The flexible forms' preconditioner cycle for a hierarchy (PRECISION_MG, with fewer coarsest
-    iterations when the coarsest level does not fit one thread block)."""
+    iterations when the coarsest level is larger than coarsest_in_one_block's rule)."""
     nu0 = PRECISION_MG[0] if coarsest_in_one_block(maxlevel, element_nb) else PRECISION_NU0_LARGE_COARSEST
     return (nu0,) + tuple(PRECISION_MG[1:]) + (int(ncy),)
 
@@ -238,8 +240,8 @@ class Hierarchy:
         self._c("hpc_set_fused_coarsest", int(bool(on)))
 
     def set_tma_staging(self, on: bool = True):
-        """hpc_set_tma_staging: finest-level applies stage node rows with tensor copies (default) or
-        per-lane cp.async (False); the same bits either way."""
+        """hpc_set_tma_staging: the applies stage node planes with tensor copies (default) or per-thread
+        cp.async (False); the same bits either way."""
         self._c("hpc_set_tma_staging", int(bool(on)))
 
     def set_autotune(self, on: bool):

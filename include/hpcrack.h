@@ -145,11 +145,10 @@ int hpc_set_fused_coarsest(hpc_ctx* ctx, int on);
  * kernels.  TF32 operands approximate the FP32 operator to about 1e-3; the flexible PCG around the
  * V-cycle keeps its FP64 residual, so the solution meets the same tolerance. */
 int hpc_set_tensor_apply(hpc_ctx* ctx, int on);
-/* No counterpart in the reference: 1 stages the node rows of the finest-level operator applies
- * (FP64 and the precision form's FP32, with the Gauss-point moduli of a mechanical solve) with
- * tensor-memory-accelerator copies - one cp.async.bulk.tensor per row of three components on two
- * planes, completion on an mbarrier - instead of per-lane cp.async (the default); 0 stages with
- * per-lane cp.async.  The same values reach the same arithmetic: the same bits. */
+/* No counterpart in the reference: 1 (default) stages the node planes and moduli of the tiled operator
+ * applies (every coarse level, the phase field, and the finest level inside a mechanical solve; FP64 and
+ * the precision form's FP32) with tensor-memory-accelerator copies, completion on an mbarrier; 0 with
+ * per-thread cp.async of 16 bytes.  The same values reach the same arithmetic: the same bits. */
 int hpc_set_tma_staging(hpc_ctx* ctx, int on);
 /* Kernels launched by this context since the last reset (instrumentation for benchmarks). */
 int hpc_launch_count(hpc_ctx* ctx, long long* count, int reset);
