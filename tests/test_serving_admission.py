@@ -9,5 +9,5 @@ def test_default_factory_admits_at_once(monkeypatch):
     srv = sv.SolveServer(hbm_budget=100, slots=2)
     res = srv.replay([_req(0, 9, increments=1), _req(1, 9, increments=1)])
     assert sorted(made) == ["r0", "r1"]
-    assert max(r.admitted for r in res) < 0.05
+    assert max(r.admitted for r in res) < 0.09
     assert FakeSolver.live == 0
